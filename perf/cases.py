@@ -11,6 +11,7 @@ chunks behind a cache.  Run with the repository's root as the working folder.
     run(state)           one pass, and everything it computes
     work(case)           bytes and floating-point operations a pass cannot do without
     tolerance(case)      how far two correct implementations may be apart
+    exact(case, seed)    the results in 64 bits, by plain torch
 """
 import math
 import os
@@ -223,3 +224,67 @@ def tolerance(case):
     if case["kind"] in ("train", "packed"):
         return {"rel": 1.7e-3, "max": 6e-2}
     return {"rel": 1.2e-3, "max": 1.5e-2}
+
+
+def _attention64(q, k, v, scale, causal, d_out=None):
+    """softmax(q k^T * scale) v of one sequence in 64 bits, q [H,n,d], k and v [H_kv,m,d], the causal mask
+    aligned to the end of the keys; with d_out also the gradients.  One head at a time, in blocks of rows."""
+    group = q.shape[0] // k.shape[0]
+    n, m = q.shape[1], k.shape[1]
+    out = torch.empty(q.shape, dtype=torch.float64, device=q.device)
+    grads = None if d_out is None else [torch.zeros(x.shape, dtype=torch.float64, device=q.device) for x in (q, k, v)]
+    rows = max(1, (1 << 27) // m)
+    columns = torch.arange(m, device=q.device)
+    for h in range(q.shape[0]):
+        kh, vh = k[h // group].double(), v[h // group].double()
+        for i in range(0, n, rows):
+            qh = q[h, i:i + rows].double()
+            p = qh @ kh.T * scale
+            if causal:
+                last = torch.arange(i, i + qh.shape[0], device=q.device) + (m - n)
+                p.masked_fill_(columns[None, :] > last[:, None], -math.inf)
+            p = torch.softmax(p, dim=-1)
+            out[h, i:i + rows] = p @ vh
+            if d_out is not None:
+                g = d_out[h, i:i + rows].double()
+                ds = p * (g @ vh.T - (g * out[h, i:i + rows]).sum(-1, keepdim=True)) * scale
+                grads[0][h, i:i + rows] = ds @ kh
+                grads[1][h // group] += ds.T @ qh
+                grads[2][h // group] += p.T @ g
+    return out, grads
+
+
+def exact(case, seed):
+    """What run() returns for the inputs of this seed, in 64 bits; None where that takes too long, and in
+    the place of the caches, whose rows are copied and not computed."""
+    if work(case)["flops"] > 1e13 or work(case)["bytes"] > 2e10:
+        return None
+    s = prepare(case, seed)
+    kind, d = case["kind"], case["head_dim"]
+    scale = 1.0 / math.sqrt(d)
+    with torch.no_grad():
+        if kind in ("forward", "train"):
+            parts = [_attention64(s["q"][b], s["k"][b], s["v"][b], scale, case["causal"],
+                                  s["d_out"][b] if kind == "train" else None) for b in range(case["batch"])]
+            out = torch.stack([o for o, _ in parts])
+            return out if kind == "forward" else (out, *(torch.stack([g[i] for _, g in parts]) for i in range(3)))
+        if kind == "packed":
+            cu = s["cu"].tolist()
+            parts = []
+            for a, b in zip(cu, cu[1:]):
+                o, grads = _attention64(*(s[name][a:b].transpose(0, 1) for name in ("q", "k", "v")), scale,
+                                        case["causal"], s["d_out"][a:b].transpose(0, 1))
+                parts.append([x.transpose(0, 1) for x in (o, *grads)])
+            return tuple(torch.cat([part[i] for part in parts]) for i in range(4))
+        axis = 0 if case["layout"] == "bshd" else 1
+        outs = []
+        for b, filled in enumerate(s["lens"].tolist()):
+            kv = []
+            for name in ("k", "v"):
+                old = s[name + "_cache"][b].narrow(axis, 0, filled)
+                old = old.transpose(0, 1) if axis == 0 else old
+                kv.append(torch.cat([old, s[name][b].transpose(0, 1)], dim=1) if name in s else old)
+            o, _ = _attention64(s["q"][b].transpose(0, 1), *kv, scale, kind == "chunk")
+            outs.append(o.transpose(0, 1))
+        out = torch.stack(outs)
+        return (out, None, None) if "k" in s else out
