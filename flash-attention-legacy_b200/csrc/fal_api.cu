@@ -209,24 +209,32 @@ int decode_split_len(int batch, int capacity) {
 }
 
 // Decode scratch layout: [partial O fp32 rows*d][partial (max, sum) fp32 rows*2], rows =
-// batch*heads_q*splits.  Nothing in it needs initialising.  (Sized for the shorter split length
-// whichever is used, so the size a caller was told does not depend on the choice.)
-struct DecodeWorkspace {
-  int64_t splits;
-  int split_len;
-  size_t partial_bytes;
-  size_t total() const { return partial_bytes; }
-};
+// batch*heads_q*splits.  Nothing in it needs initialising.  (Sized for 1 024-position splits
+// whichever length is used, so the size a caller was told does not depend on the choice.)
+size_t decode_partial_bytes(int batch, int heads_q, int capacity, int head_dim, int split_len) {
+  const int64_t rows = static_cast<int64_t>(batch) * heads_q * ((capacity + split_len - 1) / split_len);
+  return static_cast<size_t>(rows) * (kernel_head_dim(head_dim) + 2) * sizeof(float);
+}
 
-DecodeWorkspace decode_workspace_layout(int batch, int heads_q, int capacity, int head_dim) {
-  head_dim = kernel_head_dim(head_dim);
-  DecodeWorkspace w;
-  w.split_len = decode_split_len(batch, capacity);
-  w.splits = (capacity + w.split_len - 1) / w.split_len;
-  const int64_t max_splits = (capacity + kDecodeSplitLen - 1) / kDecodeSplitLen;
-  const int64_t rows = static_cast<int64_t>(batch) * heads_q * max_splits;
-  w.partial_bytes = static_cast<size_t>(rows) * (head_dim + 2) * sizeof(float);
-  return w;
+// A grid that leaves SMs without a CTA is bound by the latency of one CTA's chain of slices, not by HBM:
+// splits are halved, down to 256 positions (four 16-key slices for each of the four warps), until there are
+// two CTAs per SM -- as far as the partials fit the workspace.  Only the first 4 MiB of it count, so that
+// the result does not depend on how much more a caller has.  Split-K and combine together, 1 024 positions
+// against 256: 1 entry of 1 999 (32 / 8 heads of 128) 24.4 -> 14.3 us, 8 of 2 049 (32 / 4 of 64) 18.4 -> 14.4,
+// 4 of 4 000 to 8 000 (8 / 1 of 128) 24.6 -> 16.4, 1 of 2 299 (16 / 2 of 256) 31.7 -> 18.4.  128 positions
+// measured 14.3, 16.4, 20.5 and 16.4: the partials then cost what the shorter chains save.
+constexpr int kDecodeMinSplit = 256;
+constexpr int kDecodeCtasPerSm = 2;
+constexpr size_t kDecodeFineBytes = size_t{4} << 20;
+int decode_split_len_for(int batch, int heads_q, int heads_kv, int capacity, int head_dim, size_t workspace_bytes) {
+  int len = decode_split_len(batch, capacity);
+  const int64_t units = static_cast<int64_t>(batch) * heads_kv * ((heads_q / heads_kv + 15) / 16);
+  const int64_t want = kDecodeCtasPerSm * static_cast<int64_t>(sm_count() > 0 ? sm_count() : 148);
+  const size_t room = workspace_bytes < kDecodeFineBytes ? workspace_bytes : kDecodeFineBytes;
+  while (len > kDecodeMinSplit && units * ((capacity + len - 1) / len) < want &&
+         decode_partial_bytes(batch, heads_q, capacity, head_dim, len / 2) <= room)
+    len /= 2;
+  return len;
 }
 
 // ---------------------------------------------------------------------------
@@ -766,7 +774,7 @@ int fal_scale_cast_f16(void* dst, const float* src, int batch, int heads, int ro
 
 size_t fal_decode_workspace_bytes(int batch, int heads_q, int capacity, int head_dim) {
   if (batch <= 0 || heads_q <= 0 || capacity <= 0 || head_dim <= 0) return 0;
-  return decode_workspace_layout(batch, heads_q, capacity, head_dim).total();
+  return decode_partial_bytes(batch, heads_q, capacity, head_dim, kDecodeSplitLen);
 }
 
 namespace {
@@ -802,8 +810,8 @@ int decode_with_workspace(const void* q, void* k_cache, void* v_cache, const fal
   if (rc != FAL_OK) return rc;
   if (!workspace) return FAL_ERR_INVALID_ARGUMENT;
   if ((reinterpret_cast<uintptr_t>(workspace) & 15u) != 0) return FAL_ERR_INVALID_ARGUMENT;
-  const DecodeWorkspace w = decode_workspace_layout(batch, heads_q, capacity, head_dim);
-  if (workspace_bytes < w.total()) return FAL_ERR_WORKSPACE_TOO_SMALL;
+  if (workspace_bytes < decode_partial_bytes(batch, heads_q, capacity, head_dim, kDecodeSplitLen))
+    return FAL_ERR_WORKSPACE_TOO_SMALL;
   rc = check_device();
   if (rc != FAL_OK) return rc;
 
@@ -825,8 +833,8 @@ int decode_with_workspace(const void* q, void* k_cache, void* v_cache, const fal
   p.capacity = capacity;
   p.head_dim = kernel_head_dim(head_dim);
   p.head_dim_real = head_dim;
-  p.split_len = w.split_len;
-  p.splits = static_cast<int>(w.splits);
+  p.split_len = decode_split_len_for(batch, heads_q, heads_kv, capacity, head_dim, workspace_bytes);
+  p.splits = (capacity + p.split_len - 1) / p.split_len;
   p.scale = softmax_scale;
   p.status = status;
   p.part_o = static_cast<float*>(workspace);

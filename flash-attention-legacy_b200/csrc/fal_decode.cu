@@ -123,6 +123,7 @@ fal_decode_splitk_kernel(const DecodeParams p) {
   constexpr int kLoadsPerLane = kSliceKeys * kChunks / 32;
 
   extern __shared__ __align__(128) uint8_t dec_smem[];
+  grid_dependency_launch();  // the combine kernel may take its place on the SMs; it waits for this grid's end
 
   const int group = p.heads_q / p.heads_kv;          // query heads per KV head
   const int head_chunks = (group + 15) / 16;
@@ -362,29 +363,86 @@ fal_decode_splitk_kernel(const DecodeParams p) {
 // ---------------------------------------------------------------------------
 // Combine: merge the splits a sequence actually reaches.
 // ---------------------------------------------------------------------------
-__global__ void fal_decode_combine_kernel(const DecodeParams p) {
+// One block per (batch, head).  The statistics of all splits are reduced by the whole block at once and
+// the partial rows are summed by groups of D / 4 threads (16-byte loads), a split each: with one thread
+// per column walking every split three times the kernel took 4.8 us at 2 splits, most of it exposed
+// load latency that grows with the number of splits.
+// It is launched while the split-K grid still runs and waits here for that grid's results.
+constexpr int kCombineThreads = 128;
+
+// (m, l) <- the merge with another running maximum and sum (log2 domain).
+__device__ __forceinline__ void merge_stats(float& m, float& l, float m2, float l2) {
+  const float m_new = fmaxf(m, m2);
+  const float m_use = (m_new == kNegInfD) ? 0.f : m_new;
+  l = l * fast_exp2(m - m_use) + l2 * fast_exp2(m2 - m_use);
+  m = m_new;
+}
+
+template <int D>
+__global__ void __launch_bounds__(kCombineThreads)
+fal_decode_combine_kernel(const DecodeParams p) {
+  constexpr int kLanes = D / 4;                        // threads per partial row
+  constexpr int kGroups = kCombineThreads / kLanes;    // rows in flight
+  __shared__ float2 warp_ml[kCombineThreads / 32];
+  __shared__ float4 part[kGroups][kLanes];
   const int bh = blockIdx.x;
   const int b = bh / p.heads_q;
-  const int D = p.head_dim;
+  const int tid = threadIdx.x;
   const int len = decode_range(p, b).len;
   const int n = (len + p.split_len - 1) / p.split_len;
-  const float* ml = p.part_ml + static_cast<int64_t>(bh) * p.splits * 2;
-  const float* po = p.part_o + static_cast<int64_t>(bh) * p.splits * D;
+  const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + static_cast<int64_t>(bh) * p.splits;
+  const float4* po = reinterpret_cast<const float4*>(p.part_o) + static_cast<int64_t>(bh) * p.splits * kLanes;
+  grid_dependency_wait();
 
-  float mmax = kNegInfD;
-  for (int i = 0; i < n; ++i) mmax = fmaxf(mmax, ml[2 * i]);
-  const float muse = (mmax == kNegInfD) ? 0.f : mmax;
-  float lsum = 0.f;
-  for (int i = 0; i < n; ++i) lsum += fast_exp2(ml[2 * i] - muse) * ml[2 * i + 1];
-  const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
-  for (int c = threadIdx.x; c < p.head_dim_real; c += blockDim.x) {
-    float o = 0.f;
-    for (int i = 0; i < n; ++i) o += fast_exp2(ml[2 * i] - muse) * po[static_cast<int64_t>(i) * D + c];
-    static_cast<__half*>(p.o)[static_cast<int64_t>(bh) * p.head_dim_real + c] = __float2half_rn(o * inv);
+  float m = kNegInfD, l = 0.f;
+  for (int i = tid; i < n; i += kCombineThreads) {
+    const float2 x = ml[i];
+    merge_stats(m, l, x.x, x.y);
   }
-  if (p.lse != nullptr && threadIdx.x == 0) {
-    p.lse[bh] = (lsum > 0.f) ? (mmax + log2f(lsum)) * 0.6931471805599453f : kNegInfD;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const float m2 = __shfl_xor_sync(0xffffffffu, m, off);
+    const float l2 = __shfl_xor_sync(0xffffffffu, l, off);
+    merge_stats(m, l, m2, l2);
   }
+  if ((tid & 31) == 0) warp_ml[tid >> 5] = make_float2(m, l);
+  __syncthreads();
+  m = warp_ml[0].x;
+  l = warp_ml[0].y;
+#pragma unroll
+  for (int w = 1; w < kCombineThreads / 32; ++w) merge_stats(m, l, warp_ml[w].x, warp_ml[w].y);
+  const float muse = (m == kNegInfD) ? 0.f : m;
+  const float inv = l > 0.f ? 1.f / l : 0.f;
+
+  const int lane = tid % kLanes;
+  const int grp = tid / kLanes;
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int i = grp; i < n; i += kGroups) {
+    const float w = fast_exp2(ml[i].x - muse);
+    const float4 x = po[static_cast<int64_t>(i) * kLanes + lane];
+    o.x += w * x.x;
+    o.y += w * x.y;
+    o.z += w * x.z;
+    o.w += w * x.w;
+  }
+  part[grp][lane] = o;
+  __syncthreads();
+  if (grp == 0 && lane * 4 < p.head_dim_real) {
+#pragma unroll
+    for (int g = 1; g < kGroups; ++g) {
+      const float4 x = part[g][lane];
+      o.x += x.x;
+      o.y += x.y;
+      o.z += x.z;
+      o.w += x.w;
+    }
+    uint2 out;
+    out.x = pack_half2(o.x * inv, o.y * inv);
+    out.y = pack_half2(o.z * inv, o.w * inv);
+    *reinterpret_cast<uint2*>(static_cast<__half*>(p.o) + static_cast<int64_t>(bh) * p.head_dim_real + lane * 4) = out;
+  }
+  if (p.lse != nullptr && tid == 0) p.lse[bh] = (l > 0.f) ? (m + log2f(l)) * 0.6931471805599453f : kNegInfD;
 }
 
 template <int D>
@@ -435,8 +493,11 @@ cudaError_t decode_static_scratch(float** ptr) {
 }
 
 cudaError_t launch_decode_combine(const DecodeParams& p, cudaStream_t stream) {
-  fal_decode_combine_kernel<<<p.batch * p.heads_q, p.head_dim, 0, stream>>>(p);
-  return cudaGetLastError();
+  const dim3 grid(p.batch * p.heads_q), block(kCombineThreads);
+  if (p.head_dim == 128) return launch_dependent(fal_decode_combine_kernel<128>, grid, block, 0, stream, p);
+  if (p.head_dim == 64) return launch_dependent(fal_decode_combine_kernel<64>, grid, block, 0, stream, p);
+  if (p.head_dim == 256) return launch_dependent(fal_decode_combine_kernel<256>, grid, block, 0, stream, p);
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_decode_splitk(const DecodeParams& p, cudaStream_t stream) {

@@ -35,6 +35,24 @@ class DeviceOnce {
   bool done_[kMaxDevices] = {};
 };
 
+// Launches a kernel that may start while the kernel before it in the stream still runs.  The kernel must
+// call grid_dependency_wait() before it touches anything that kernel reads or writes.
+template <class... Params, class... Args>
+cudaError_t launch_dependent(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                             const Args&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // Forward: grid = number of (p.cta_rows-row block, batch*head) units.  fwd_cta_rows gives the rows
 // a CTA takes: 256 (two query tiles) unless head_dim is 256 or the one-tile variant is asked for.
 int fwd_cta_rows(int head_dim, bool one_tile);

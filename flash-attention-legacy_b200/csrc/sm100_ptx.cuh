@@ -34,6 +34,15 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // ---------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------
+// Programmatic dependent launch: lets the next kernel of the stream start early (a kernel launched with
+// launch_dependent), and waits until the grids before this one have completed and their writes are visible.
+__device__ __forceinline__ void grid_dependency_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }

@@ -515,6 +515,7 @@ def scale_cast_f16(src, scale=1.0, out=None):
 
 
 _decode_ws = {}
+_DECODE_WS_MIN = 4 << 20  # what the library uses at most to split a small batch finer than its minimum
 
 
 def _decode_workspace(device, nbytes):
@@ -589,12 +590,12 @@ def decode(q, k_cache, v_cache, cache_seqlens, softmax_scale, k_new=None, v_new=
                                             out, None, cache_starts)
     o = torch.empty((B, Hq, d), dtype=torch.float16, device=q.device) if out is None else out
     lse = torch.empty((B, Hq), dtype=torch.float32, device=q.device) if return_lse else None
-    nbytes = _lib.fal_decode_workspace_bytes(B, Hq, S, d)
+    nbytes = max(_lib.fal_decode_workspace_bytes(B, Hq, S, d), _DECODE_WS_MIN)
     ws = _decode_workspace(q.device, nbytes)
     tail = (k_new.data_ptr() if k_new is not None else None,
             v_new.data_ptr() if v_new is not None else None,
             o.data_ptr(), lse.data_ptr() if lse is not None else None,
-            B, Hq, Hkv, S, d, float(softmax_scale), ws.data_ptr(), ws.numel(),
+            B, Hq, Hkv, S, d, float(softmax_scale), ws.data_ptr(), nbytes,
             _status_word(q.device).data_ptr(), _stream(q))
     if cache_starts is None:
         _check(_lib.fal_decode(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), ks, vs,

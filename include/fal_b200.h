@@ -242,7 +242,8 @@ FAL_API int fal_scale_cast_f16(void* dst, const float* src, int batch, int heads
 
 /*
  * Bytes of scratch fal_decode needs for its split-K partial results (no initialisation needed;
- * 16-byte aligned; calls that use the same workspace must not overlap on the GPU).
+ * 16-byte aligned; calls that use the same workspace must not overlap on the GPU).  This is the
+ * smallest workspace taken; with up to 4 MiB a small batch is split finer and finishes sooner.
  */
 FAL_API size_t fal_decode_workspace_bytes(int batch, int heads_q, int capacity, int head_dim);
 
