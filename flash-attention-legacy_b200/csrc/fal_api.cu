@@ -891,6 +891,28 @@ int fal_decode_static(const void* q, void* k_cache, void* v_cache, const fal_str
                                fal::kDecodeStaticScratchBytes, status, stream);
 }
 
+int fal_cache_append(const void* k_new, const void* v_new, void* k_cache, void* v_cache,
+                     const fal_strides* k_new_strides, const fal_strides* v_new_strides,
+                     const fal_strides* k_strides, const fal_strides* v_strides, const int32_t* cache_seqlens,
+                     int32_t* new_seqlens, uint8_t* fits, int batch, int heads_kv, int rows, int capacity,
+                     int head_dim, void* stream) {
+  if (batch <= 0 || batch > 65535 || heads_kv <= 0 || rows <= 0 || capacity <= 0 || !cache_seqlens || !new_seqlens ||
+      !fits || !vec_ok(k_new, k_new_strides, 2) || !vec_ok(v_new, v_new_strides, 2) || !vec_ok(k_cache, k_strides, 2) ||
+      !vec_ok(v_cache, v_strides, 2))
+    return FAL_ERR_INVALID_ARGUMENT;
+  if (!head_dim_ok(head_dim)) return FAL_ERR_UNSUPPORTED_HEAD_DIM;
+  int rc = check_device();
+  if (rc != FAL_OK) return rc;
+  fal::CacheAppendParams p{};
+  p.k_new = k_new; p.v_new = v_new; p.k_cache = k_cache; p.v_cache = v_cache;
+  p.k_new_strides = to_rs(k_new_strides); p.v_new_strides = to_rs(v_new_strides);
+  p.k_strides = to_rs(k_strides); p.v_strides = to_rs(v_strides);
+  p.cache_seqlens = cache_seqlens; p.new_seqlens = new_seqlens; p.fits = fits;
+  p.batch = batch; p.heads_kv = heads_kv; p.rows = rows; p.capacity = capacity; p.head_dim = head_dim;
+  cudaError_t e = fal::launch_cache_append(p, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? FAL_OK : cuda_fail(e);
+}
+
 int fal_set_fwd_variant(int variant) {
   if (variant < FAL_FWD_AUTO || variant > FAL_FWD_TWO_TILES) return FAL_ERR_INVALID_ARGUMENT;
   g_fwd_variant.store(variant, std::memory_order_relaxed);

@@ -445,6 +445,43 @@ fal_decode_combine_kernel(const DecodeParams p) {
   if (p.lse != nullptr && tid == 0) p.lse[bh] = (l > 0.f) ? (m + log2f(l)) * 0.6931471805599453f : kNegInfD;
 }
 
+// ---------------------------------------------------------------------------
+// Append of a chunk of new rows to caches filled to a different length per entry.
+// ---------------------------------------------------------------------------
+// Bound by HBM (each byte read once and written once); a thread moves 16 bytes.  One launch for K and V,
+// the new lengths and the room check: as tensor indexing it was ten launches, whose two scatter kernels
+// took 27 us each for 4 entries x 1024 rows x 8 heads x 128.
+__global__ void __launch_bounds__(256) fal_cache_append_kernel(const CacheAppendParams p) {
+  const int b = blockIdx.y;
+  const bool is_v = blockIdx.z != 0;
+  const int len = __ldg(p.cache_seqlens + b);
+  if (blockIdx.x == 0 && !is_v && threadIdx.x == 0) p.new_seqlens[b] = len + p.rows;
+  if (blockIdx.x == 0 && b == 0 && is_v) {  // every position of every entry must be inside the cache
+    bool fits = true;
+    for (int i = threadIdx.x; i < p.batch; i += 256) {
+      const int64_t l = __ldg(p.cache_seqlens + i);
+      fits = fits && l >= -static_cast<int64_t>(p.capacity) && l + p.rows <= p.capacity;
+    }
+    fits = __syncthreads_and(fits) != 0;
+    if (threadIdx.x == 0) *p.fits = fits ? 1 : 0;
+  }
+  const int chunks = p.head_dim / 8;
+  const int64_t idx = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
+  if (idx >= static_cast<int64_t>(p.rows) * p.heads_kv * chunks) return;
+  const int c = static_cast<int>(idx % chunks);
+  const int64_t rh = idx / chunks;
+  const int h = static_cast<int>(rh % p.heads_kv);
+  const int r = static_cast<int>(rh / p.heads_kv);
+  int64_t pos = static_cast<int64_t>(len) + r;
+  if (pos < 0) pos += p.capacity;  // counts from the end, as an index does
+  if (pos < 0 || pos >= p.capacity) return;
+  const RowStrides& ss = is_v ? p.v_new_strides : p.k_new_strides;
+  const RowStrides& ds = is_v ? p.v_strides : p.k_strides;
+  const __half* src = static_cast<const __half*>(is_v ? p.v_new : p.k_new) + b * ss.batch + h * ss.head + r * ss.row;
+  __half* dst = static_cast<__half*>(is_v ? p.v_cache : p.k_cache) + b * ds.batch + h * ds.head + pos * ds.row;
+  *reinterpret_cast<uint4*>(dst + c * 8) = *reinterpret_cast<const uint4*>(src + c * 8);
+}
+
 template <int D>
 cudaError_t launch_splitk_t(const DecodeParams& p, cudaStream_t stream) {
   auto kern = fal_decode_splitk_kernel<D>;
@@ -490,6 +527,13 @@ cudaError_t decode_static_scratch(float** ptr) {
   }
   *ptr = cached[dev];
   return cudaSuccess;
+}
+
+cudaError_t launch_cache_append(const CacheAppendParams& p, cudaStream_t stream) {
+  const int64_t blocks = (static_cast<int64_t>(p.rows) * p.heads_kv * (p.head_dim / 8) + 255) / 256;
+  if (blocks > 0x7fffffff || p.batch > 65535) return cudaErrorInvalidValue;
+  fal_cache_append_kernel<<<dim3(static_cast<unsigned>(blocks), p.batch, 2), 256, 0, stream>>>(p);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_decode_combine(const DecodeParams& p, cudaStream_t stream) {

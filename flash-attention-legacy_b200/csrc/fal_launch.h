@@ -162,6 +162,20 @@ struct DecodeParams {
   float scale;
   int* status;
 };
+// Rows appended to both caches at every entry's own length.
+struct CacheAppendParams {
+  const void* k_new;    // [batch, heads_kv, row] through strides, fp16
+  const void* v_new;
+  void* k_cache;
+  void* v_cache;
+  RowStrides k_new_strides, v_new_strides, k_strides, v_strides;
+  const int32_t* cache_seqlens;  // [batch]
+  int32_t* new_seqlens;          // [batch]: cache_seqlens + rows
+  uint8_t* fits;                 // 1 if every row has a place in its cache, else 0
+  int batch, heads_kv, rows, capacity, head_dim;
+};
+cudaError_t launch_cache_append(const CacheAppendParams& p, cudaStream_t stream);
+
 // Size of the library-resident scratch behind fal_decode_static, and its per-device address.
 constexpr size_t kDecodeStaticScratchBytes = 8u << 20;
 cudaError_t decode_static_scratch(float** ptr);

@@ -287,17 +287,24 @@ def flash_attn_with_kvcache(
     lens = cache_seqlens.to(torch.int32)
     if k is not None:
         assert v is not None and k.shape == v.shape and k.shape[:2] == (b, lq), "k, v must be [B, L_q, H_kv, d]"
-        # rows lens[b] ... lens[b] + Lq - 1 of every entry (an entry without room for the chunk is an error
-        # the indexing reports)
-        pos = lens.long()[:, None] + torch.arange(lq, device=q.device)[None, :]
-        rows = torch.arange(b, device=q.device)[:, None]
-        if cache_layout == "bshd":
-            k_cache[rows, pos] = k
-            v_cache[rows, pos] = v
+        # rows lens[b] ... lens[b] + Lq - 1 of every entry
+        kd, vd = (k_cache, v_cache) if cache_layout == "bshd" else (k_cache.transpose(1, 2), v_cache.transpose(1, 2))
+        tracked = torch.is_grad_enabled() and any(t.requires_grad for t in (k, v, k_cache, v_cache))
+        appended = None if tracked else flash_attn_legacy_cuda.cache_append(k, v, kd, vd, lens)
+        if appended is not None:
+            lens, fits = appended
+            torch._assert_async(fits)  # an entry without room for the chunk
+            for t in (k_cache, v_cache):
+                if not t.is_inference():
+                    torch.autograd.graph.increment_version(t)
         else:
-            k_cache.transpose(1, 2)[rows, pos] = k
-            v_cache.transpose(1, 2)[rows, pos] = v
-        lens = lens + lq
+            # tensors the append kernel does not address (broadcast heads, unaligned rows, gradients): by
+            # indexing, which reports an entry without room by itself
+            pos = lens.long()[:, None] + torch.arange(lq, device=q.device)[None, :]
+            rows = torch.arange(b, device=q.device)[:, None]
+            kd[rows, pos] = k
+            vd[rows, pos] = v
+            lens = lens + lq
     kc = k_cache.transpose(1, 2) if cache_layout == "bshd" else k_cache
     vc = v_cache.transpose(1, 2) if cache_layout == "bshd" else v_cache
     # O is written as [B,Lq,Hq,d] memory through its [B,Hq,Lq,d] view: no transpose afterwards

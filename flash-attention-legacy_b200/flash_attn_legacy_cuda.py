@@ -75,6 +75,9 @@ _lib.fal_decode_static.argtypes = [_vp, _vp, _vp, _sp, _sp, _vp, _vp, _vp, _vp, 
                                    _vp, _vp]
 DECODE_STATIC_SCRATCH_BYTES = 8 << 20
 
+_lib.fal_cache_append.restype = _i
+_lib.fal_cache_append.argtypes = [_vp] * 4 + [_sp] * 4 + [_vp] * 3 + [_i] * 5 + [_vp]
+
 _lib.fal_profile_enable.restype = _i
 _lib.fal_profile_enable.argtypes = [_i]
 _lib.fal_profile_read.restype = _i
@@ -604,6 +607,41 @@ def decode(q, k_cache, v_cache, cache_seqlens, softmax_scale, k_new=None, v_new=
         _check(_lib.fal_decode_ranged(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), ks, vs,
                                       cache_starts.data_ptr(), cache_seqlens.data_ptr(), *tail))
     return (o, lse) if return_lse else o
+
+
+def cache_append(k_new, v_new, k_cache, v_cache, cache_seqlens):
+    """Writes k_new / v_new [B,Lq,Hkv,d] behind every entry's cached rows, in one launch.
+
+    Caches are [B,S,Hkv,d] (any strides with a contiguous head_dim); row i of entry b goes to position
+    cache_seqlens[b] + i.  Returns (new lengths int32 [B], a one-element bool tensor on the device: every
+    row had a place), or None -- and nothing written -- for tensors the kernel cannot address.
+    """
+    if k_cache.dim() != 4:
+        return None
+    B, S, Hkv, d = k_cache.shape
+    caches = (k_cache.untyped_storage().data_ptr(), v_cache.untyped_storage().data_ptr())
+    if k_new.untyped_storage().data_ptr() in caches or v_new.untyped_storage().data_ptr() in caches:
+        return None  # (indexing refuses a source that overlaps the rows it writes)
+    for t in (k_new, v_new, k_cache, v_cache):
+        if (not t.is_cuda or t.device != k_cache.device or t.dtype != torch.float16 or t.dim() != 4
+                or t.stride(3) != 1 or t.data_ptr() % 16 != 0
+                or any(s % 8 != 0 or (s <= 0 and n > 1) for s, n in zip(t.stride()[:3], t.shape[:3]))):
+            return None
+    rows = k_new.shape[1]
+    shape = (B, rows, Hkv, d)
+    if (tuple(k_new.shape) != shape or tuple(v_new.shape) != shape or v_cache.shape != k_cache.shape
+            or d not in (32, 64, 96, 128, 256) or not 0 < B <= 65535 or min(shape) == 0 or S == 0
+            or cache_seqlens.dtype != torch.int32 or tuple(cache_seqlens.shape) != (B,)
+            or cache_seqlens.device != k_cache.device or not cache_seqlens.is_contiguous()
+            or k_cache.device.index != torch.cuda.current_device()):
+        return None
+    lens = torch.empty((B,), dtype=torch.int32, device=k_cache.device)
+    fits = torch.empty((1,), dtype=torch.bool, device=k_cache.device)
+    strides = [_Strides(t.stride(0), t.stride(2), t.stride(1)) for t in (k_new, v_new, k_cache, v_cache)]
+    _check(_lib.fal_cache_append(k_new.data_ptr(), v_new.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), *strides,
+                                 cache_seqlens.data_ptr(), lens.data_ptr(), fits.data_ptr(), B, Hkv, rows, S, d,
+                                 _stream(k_cache)))
+    return lens, fits
 
 
 def decode_static(q, k_cache, v_cache, cache_seqlens, softmax_scale, out, k_new=None, v_new=None,

@@ -285,6 +285,19 @@ FAL_API int fal_decode_ranged(const void* q, void* k_cache, void* v_cache,
                int* status, void* stream);
 
 /*
+ * Writes a chunk of new rows into K and V caches filled to a different length per entry: row i of entry b
+ * goes to position cache_seqlens[b] + i (a negative position counts from the end of the cache).
+ * new_seqlens[b] = cache_seqlens[b] + rows; *fits (one byte on the device) becomes 1 if every row had a place and
+ * 0 otherwise, rows without one are not stored.  Tensors are addressed as [B,Hkv,row or position,d], 16-byte
+ * aligned rows.  No counterpart in the reference (its hook's cache is written by the framework around it).
+ */
+FAL_API int fal_cache_append(const void* k_new, const void* v_new, void* k_cache, void* v_cache,
+               const fal_strides* k_new_strides, const fal_strides* v_new_strides,
+               const fal_strides* k_strides, const fal_strides* v_strides,
+               const int32_t* cache_seqlens, int32_t* new_seqlens, uint8_t* fits,
+               int batch, int heads_kv, int rows, int capacity, int head_dim, void* stream);
+
+/*
  * Decode for callers that must not allocate device memory (no counterpart in the
  * reference).  Some hosts of this library cannot call cudaMalloc at the point where
  * they decode: a serving loop that was handed a fixed memory budget at start-up, a
