@@ -164,17 +164,29 @@ int sm_count() {
 // grids that leave SMs without a two-tile CTA, or that end in a mostly empty wave.
 std::atomic<int> g_fwd_variant{FAL_FWD_AUTO};  // fal_set_fwd_variant
 
-int forward_cta_rows(int head_dim, int64_t blocks_of_256_rows, int64_t units) {
+// At head_dim 64 the TMEM and shared memory of an SM hold two CTAs of one tile and one softmax warpgroup.
+// They overlap as the two tiles of a two-tile CTA do, and each one's prologue and epilogue run under the
+// other's main loop besides, which is what short rows spend their time on; the price is that every K / V
+// tile is fetched once per 128 query rows.  us, two tiles against half-SM CTAs: 32 x 16 heads x 577 142 / 123,
+// 48 x 32 x 65 59 / 37, 20 x 8 x 257 causal 29 / 21, 8 x 16 x 512 causal 27 / 25, 4 x 16 x 2 048 133 / 129 and
+// causal 80 / 76; 2 x 16 x 4 096 232 / 236, 16 x 8 192 causal 213 / 219, 16 x 16 384 causal 757 / 796: the line
+// lies at 2 048 keys a row on average.  With no more than one CTA per SM the alternating warpgroups of the
+// one-tile CTA are faster (2 x 8 x 1 024 causal: 17 against 21).  At head_dim 128, the same shape with single
+// K and V buffers measured 89 against 93 us on 16 x 16 x 577 but 665 against 578 on 4 x 32 x 4 096 causal and
+// 116 against 112 on 2 x 32 x 1 500 (64 KB of K and V per tile and CTA); it is not built.
+constexpr int kHalfSmMaxKeys = 2048;
+
+int forward_variant(int head_dim, int64_t blocks_of_256_rows, int64_t units, int64_t mean_keys) {
   const int forced = g_fwd_variant.load(std::memory_order_relaxed);
-  bool one_tile = forced == FAL_FWD_ONE_TILE;
-  if (forced == FAL_FWD_AUTO) {
-    const int64_t sms = sm_count() > 0 ? sm_count() : 148;
-    const int64_t ctas2 = blocks_of_256_rows * units;
-    const int64_t waves2 = (ctas2 + sms - 1) / sms;
-    const int64_t waves1 = (2 * ctas2 + sms - 1) / sms;
-    one_tile = 6 * waves1 < 10 * waves2;
-  }
-  return fal::fwd_cta_rows(head_dim, one_tile);
+  if (head_dim == 256) return FAL_FWD_ONE_TILE;
+  if (forced == FAL_FWD_HALF_SM) return head_dim == 64 ? forced : FAL_FWD_TWO_TILES;
+  if (forced != FAL_FWD_AUTO) return forced;
+  const int64_t sms = sm_count() > 0 ? sm_count() : 148;
+  const int64_t ctas2 = blocks_of_256_rows * units;
+  const int64_t waves2 = (ctas2 + sms - 1) / sms;
+  const int64_t waves1 = (2 * ctas2 + sms - 1) / sms;
+  if (head_dim == 64 && 2 * ctas2 > sms && mean_keys <= kHalfSmMaxKeys) return FAL_FWD_HALF_SM;
+  return 6 * waves1 < 10 * waves2 ? FAL_FWD_ONE_TILE : FAL_FWD_TWO_TILES;
 }
 
 int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
@@ -355,9 +367,11 @@ int fwd_batched(const void* q, const void* k, const void* v, void* o, float* lse
   p.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int kdim = kernel_head_dim(head_dim);
-  const int cta_rows = forward_cta_rows(kdim, (seqlen_q + 255) / 256, static_cast<int64_t>(batch) * heads_q);
-  p.cta_rows = cta_rows;
-  p.num_qblk = (seqlen_q + cta_rows - 1) / cta_rows;
+  const int variant = forward_variant(kdim, (seqlen_q + 255) / 256, static_cast<int64_t>(batch) * heads_q,
+                                      is_causal == 1 ? seqlen_k / 2 : seqlen_k);
+  p.half_sm = variant == FAL_FWD_HALF_SM;
+  p.cta_rows = variant == FAL_FWD_TWO_TILES ? 256 : 128;
+  p.num_qblk = (seqlen_q + p.cta_rows - 1) / p.cta_rows;
   const int64_t grid = static_cast<int64_t>(p.num_qblk) * batch * heads_q;
   if (grid > 0x7fffffff) return FAL_ERR_INVALID_ARGUMENT;
   const int rec = g_timer.begin(FAL_KERNEL_FWD, st);
@@ -448,7 +462,10 @@ int fal_fwd_varlen(const void* q, const void* k, const void* v, void* o, float* 
   // The lengths stay on the device.  Every sequence rounds up to whole query blocks: at most one
   // extra block each.
   const int kdim = kernel_head_dim(head_dim);
-  p.cta_rows = forward_cta_rows(kdim, total_q / 256 + num_seqs, heads_q);
+  const int variant = forward_variant(kdim, total_q / 256 + num_seqs, heads_q,
+                                      total_k / num_seqs / (is_causal == 1 ? 2 : 1));
+  p.half_sm = variant == FAL_FWD_HALF_SM;
+  p.cta_rows = variant == FAL_FWD_TWO_TILES ? 256 : 128;
   p.num_qblk = total_q / p.cta_rows + num_seqs;
   const int64_t grid = static_cast<int64_t>(p.num_qblk) * heads_q;
   if (grid > 0x7fffffff) return FAL_ERR_INVALID_ARGUMENT;
@@ -914,7 +931,7 @@ int fal_cache_append(const void* k_new, const void* v_new, void* k_cache, void* 
 }
 
 int fal_set_fwd_variant(int variant) {
-  if (variant < FAL_FWD_AUTO || variant > FAL_FWD_TWO_TILES) return FAL_ERR_INVALID_ARGUMENT;
+  if (variant < FAL_FWD_AUTO || variant > FAL_FWD_HALF_SM) return FAL_ERR_INVALID_ARGUMENT;
   g_fwd_variant.store(variant, std::memory_order_relaxed);
   return FAL_OK;
 }

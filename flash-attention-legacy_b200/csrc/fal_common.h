@@ -35,6 +35,7 @@ struct FwdParams {
   int head_dim;   // the tensors' head_dim: 32 and 96 run on the 64 / 128 kernels (TMA fills the missing
                   // columns with zeros), output columns beyond it are not written
   int cta_rows;   // query rows per CTA: 256 (two tiles) or 128 (one tile, both softmax warpgroups on it)
+  int half_sm;    // (cta_rows 128) one softmax warpgroup per CTA and two CTAs per SM
   int num_qblk;   // batched: ceil(seqlen_q / cta_rows); packed: bound on all sequences' blocks
   int causal_shift;  // causal kernels, batched: query row i sees keys <= i + causal_shift (0: top-left aligned mask)
   int shift_per_sequence;  // causal kernels, packed: the shift of a sequence is its seqlen_k - seqlen_q

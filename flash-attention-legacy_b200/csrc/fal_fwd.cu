@@ -11,7 +11,7 @@
 // chunk of new tokens behind a cached prefix, which the reference computes
 // eagerly (flash_attn_legacy/integrations.py:77-98).
 //
-// Two CTA shapes, both 384 threads:
+// Three CTA shapes; the two that have an SM to themselves have 384 threads:
 //
 //   warps 0-3   softmax warpgroup 0 (TMEM lanes by warp % 4)
 //   warps 4-7   softmax warpgroup 1
@@ -35,7 +35,10 @@
 // P has columns of its own here, so a score buffer is free again as soon as its warpgroup has read it.
 // (head_dim 256 has no columns left for this: one warpgroup takes every key tile, as in a two-tile CTA.)
 //
-// P (fp16) feeds the PV MMA straight from TMEM; in the two-tile CTA it overwrites the first 64
+// Half an SM (128 query rows, head_dim 64, 256 threads): one softmax warpgroup and its tile, two CTAs per SM.
+// TMEM columns: S [0,128) O [128,192).
+//
+// P (fp16) feeds the PV MMA straight from TMEM; except in the one-tile CTA it overwrites the first 64
 // columns of its S block.
 #define FAL_WAIT_SLOW_PATH_INLINE  // this kernel uses setmaxnreg, which rules out calls
 #include "fal_common.h"
@@ -46,10 +49,7 @@ namespace fal {
 
 namespace {
 
-// Kernel variants (ONE_TILE):
-//   false  two query tiles per CTA, one softmax warpgroup per tile
-//   true   one query tile per CTA, the softmax warpgroups take alternate key tiles of it
-// A thread owns one 128-column score row either way.
+// A thread owns one 128-column score row in every CTA shape (FwdShape).
 // Built, measured on B4 Hq32 Hkv8 N4096 d128 causal and not kept:
 //  - two tiles with two softmax warpgroups EACH (640 threads, 104 registers per softmax thread): 583
 //    against 515 us; ncu: tensor pipe 45.7 % against 54.3 %, long-scoreboard stalls per issue 4.9
@@ -58,8 +58,11 @@ namespace {
 //  - one tile with both warpgroups on the SAME key tile, 64 score columns per thread and the row
 //    maxima exchanged every step: 600 us even with two score buffers; the two warps of a scheduler
 //    then run in lockstep (both load, both exponentiate) instead of filling each other's gaps.
-constexpr int kFwdThreads = 384;
-constexpr int kSmWarps = 8;  // softmax warps; then producer, issuer, 2 idle
+enum FwdShape : int {
+  kTwoTiles = 0,   // 256 query rows, one CTA per SM
+  kOneTile = 1,    // 128 query rows, one CTA per SM: the warpgroups take alternate key tiles
+  kHalfSm = 2,     // 128 query rows, one softmax warpgroup, two CTAs per SM (head_dim 64)
+};
 constexpr int kTileM = 128;   // query rows per softmax warpgroup
 constexpr int kTileN = 128;   // keys per step
 constexpr float kNegInf = -INFINITY;
@@ -93,10 +96,6 @@ __device__ __forceinline__ uint64_t tile_exp2_pair(int i, uint64_t x) {
 #ifndef FAL_FWD_REGS_OTHER
 #define FAL_FWD_REGS_OTHER 72
 #endif
-constexpr int kRegsSoftmax = FAL_FWD_REGS_SOFTMAX;
-constexpr int kRegsOther = FAL_FWD_REGS_OTHER;
-static_assert(2 * 128 * kRegsSoftmax + 128 * kRegsOther <= 168 * 384,
-              "setmaxnreg split exceeds the registers the CTA was launched with");
 // Barrier ids (only used to label a wait that gave up).
 enum FwdBarrier : int {
   kBarQFull = 0,
@@ -109,18 +108,33 @@ enum FwdBarrier : int {
   kBarODone = 70,
 };
 
-template <int D, bool ONE_TILE>
+template <int D, int SHAPE>
 struct FwdSmem {
+  static constexpr bool ONE_TILE = SHAPE != kTwoTiles;
+  static constexpr int kSmWarps = SHAPE == kHalfSm ? 4 : 8;  // softmax warps; then K producer, issuer, V producer, idle
+  static constexpr int kThreads = kSmWarps * 32 + 128;
+  static constexpr int kCtasPerSm = SHAPE == kHalfSm ? 2 : 1;
+  // registers per thread at launch, and how setmaxnreg splits them
+  static constexpr int kRegsLaunch = SHAPE == kHalfSm ? 128 : 168;
+  static constexpr int kRegsSoftmax = SHAPE == kHalfSm ? 200 : FAL_FWD_REGS_SOFTMAX;
+  static constexpr int kRegsOther = SHAPE == kHalfSm ? 56 : FAL_FWD_REGS_OTHER;
+  static_assert(kSmWarps * 32 * kRegsSoftmax + 128 * kRegsOther <= kRegsLaunch * kThreads,
+                "setmaxnreg split exceeds the registers the CTA was launched with");
+  // TMEM columns: score buffer w at 128 w, the output accumulator(s) at kOCol
+  static constexpr int kTmemCols = SHAPE == kHalfSm ? 256 : 512;
+  static constexpr int kOCol = SHAPE == kHalfSm ? 128 : 256;
+
   // One 128-row query tile per CTA: always at head_dim 256 (its O accumulator alone takes 256 of the
   // 512 TMEM columns; single K and V buffers, a 128 x 256 tile is 64 KB), and at head_dim 64 / 128
   // when two-tile CTAs would leave SMs without work.
   static_assert(ONE_TILE || D != 256, "head_dim 256 runs one query tile per CTA");
+  static_assert(SHAPE != kHalfSm || D == 64, "two CTAs per SM are built for head_dim 64");
   static constexpr int kQTiles = ONE_TILE ? 1 : 2;
   // One tile at head_dim 64 / 128: the softmax warpgroups take alternate key tiles (kAlt).  At 256 there
   // is no TMEM left for that (P needs columns of its own), one warpgroup takes every key tile.
-  static constexpr bool kAlt = ONE_TILE && D != 256;
+  static constexpr bool kAlt = SHAPE == kOneTile && D != 256;
   static constexpr int kCtaRows = kQTiles * kTileM;
-  static constexpr int kStages = (D == 256) ? 1 : (D == 128) ? 2 : 4;
+  static constexpr int kStages = SHAPE == kHalfSm ? 2 : (D == 256) ? 1 : (D == 128) ? 2 : 4;
   static constexpr int kBoxes = D / 64;                 // 64-element (128-byte) column boxes
   static constexpr int kBoxBytes = kTileM * 128;        // one box of a 128-row tile
   static constexpr int kTileBytes = kBoxes * kBoxBytes;  // Q, K and V tiles are all 128 x D
@@ -137,6 +151,7 @@ struct FwdSmem {
   static constexpr int kXchBytes = kAlt ? 3 * kTileM * 4 : 0;
   static constexpr int kBytes = kXchOff + kXchBytes;
   static constexpr int kAllocBytes = kBytes + 1024;  // room to align the base to 1024
+  static_assert(kCtasPerSm * (kAllocBytes + 1024) <= 228 * 1024, "exceeds the shared memory of an SM");
 };
 
 struct FwdWork {
@@ -230,13 +245,14 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t sr
 
 // SHIFTED (causal only): the mask's diagonal is moved by seqlen_k - seqlen_q keys (bottom-right
 // alignment); the kernels of the reference's own top-left mask are compiled without it.
-template <int D, bool CAUSAL, bool SHIFTED, bool ONE_TILE>
-__global__ void __launch_bounds__(kFwdThreads, 1)
+template <int D, bool CAUSAL, bool SHIFTED, int SHAPE>
+__global__ void __launch_bounds__(FwdSmem<D, SHAPE>::kThreads, FwdSmem<D, SHAPE>::kCtasPerSm)
 fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
                const FwdParams p) {
-  using L = FwdSmem<D, ONE_TILE>;
+  using L = FwdSmem<D, SHAPE>;
   constexpr int NS = L::kStages;
+  constexpr int kSmWarps = L::kSmWarps;
 
   FwdWork wk;
   constexpr int kCtaRows = L::kCtaRows;
@@ -338,7 +354,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     }
   }
   if (warp == kSmWarps + 1) {
-    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), L::kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -349,7 +365,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   // Register rebalancing between warpgroups (first statement of every role): the softmax warps
   // keep a whole 128-wide score row in registers, the producer / issuer warpgroup needs few.
   if (warp >= kSmWarps) {
-    setmaxnreg_dec<kRegsOther>();
+    setmaxnreg_dec<L::kRegsOther>();
     if (warp == kSmWarps || warp == kSmWarps + 2) {
     // ===================== TMA producers ====================================
     // K tiles from warp 8, V tiles from warp 10: each ring refills as soon as its own stage is free
@@ -418,7 +434,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       // sb = buffer that holds P, ot = output accumulator.
       auto issue_pv = [&](int sb, int ot, int j, int half) {
         const uint32_t v_lo = smem_desc_lo(sbase + L::kVOff + (j % NS) * L::kTileBytes, L::kBoxBytes);
-        const uint32_t t_o = L::kAlt ? tmem_base + 384 : tmem_base + 256 + ot * D;
+        const uint32_t t_o = L::kAlt ? tmem_base + 384 : tmem_base + L::kOCol + ot * D;
         const uint32_t t_p = L::kAlt ? tmem_base + 256 + sb * 64 : tmem_base + sb * kTileN;
 #pragma unroll
         for (int kk = 0; kk < kTileN / 32; ++kk) {
@@ -518,7 +534,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   }
   } else {
     // ===================== softmax + output =================================
-    setmaxnreg_inc<kRegsSoftmax>();
+    setmaxnreg_inc<L::kRegsSoftmax>();
     {
     // kAlt (one query tile): warpgroup wg takes key tiles wg, wg + 2, ... of the one tile, from score
     // buffer wg.  Otherwise warpgroup wg owns query tile wg and takes every key tile of it.
@@ -530,7 +546,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const int q_local = q_tile0 + row;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t tS = tmem_base + lane_addr + wg * kTileN;
-    const uint32_t tO = tmem_base + lane_addr + (kAlt ? 384 : 256 + wg * D);
+    const uint32_t tO = tmem_base + lane_addr + (kAlt ? 384 : L::kOCol + wg * D);
     const uint32_t tP = kAlt ? tmem_base + lane_addr + 256 + wg * 64 : tS;  // packed fp16 P
     const int nt = kAlt ? ntile[0] : ntile[wg];
     const float c2 = p.scale_log2;
@@ -783,49 +799,48 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   __syncthreads();
   if (warp == kSmWarps + 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, L::kTmemCols);
   }
 }
 
-template <int D, bool CAUSAL, bool SHIFTED, bool ONE_TILE>
+template <int D, bool CAUSAL, bool SHIFTED, int SHAPE>
 cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const CUtensorMap& to, const FwdParams& p, int grid, cudaStream_t stream) {
-  auto kern = fal_fwd_kernel<D, CAUSAL, SHIFTED, ONE_TILE>;
+  using L = FwdSmem<D, SHAPE>;
+  auto kern = fal_fwd_kernel<D, CAUSAL, SHIFTED, SHAPE>;
   static DeviceOnce configured;  // one per template instance
   cudaError_t e = configured.run([&] {
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                FwdSmem<D, ONE_TILE>::kAllocBytes);
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAllocBytes);
   });
   if (e != cudaSuccess) return e;
-  kern<<<grid, kFwdThreads, FwdSmem<D, ONE_TILE>::kAllocBytes, stream>>>(tq, tk, tv, to, p);
+  kern<<<grid, L::kThreads, L::kAllocBytes, stream>>>(tq, tk, tv, to, p);
   return cudaGetLastError();
 }
 
-template <int D, bool ONE_TILE>
+template <int D, int SHAPE>
 cudaError_t launch_fwd_d(bool causal, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const CUtensorMap& to, const FwdParams& p, int grid, cudaStream_t stream) {
   if (causal && (p.causal_shift != 0 || p.shift_per_sequence != 0))
-    return launch_fwd_t<D, true, true, ONE_TILE>(tq, tk, tv, to, p, grid, stream);
-  return causal ? launch_fwd_t<D, true, false, ONE_TILE>(tq, tk, tv, to, p, grid, stream)
-                : launch_fwd_t<D, false, false, ONE_TILE>(tq, tk, tv, to, p, grid, stream);
+    return launch_fwd_t<D, true, true, SHAPE>(tq, tk, tv, to, p, grid, stream);
+  return causal ? launch_fwd_t<D, true, false, SHAPE>(tq, tk, tv, to, p, grid, stream)
+                : launch_fwd_t<D, false, false, SHAPE>(tq, tk, tv, to, p, grid, stream);
 }
 
 }  // namespace
-
-int fwd_cta_rows(int head_dim, bool one_tile) { return (head_dim == 256 || one_tile) ? 128 : 256; }
 
 cudaError_t launch_fwd(int head_dim, bool causal, const CUtensorMap& tq, const CUtensorMap& tk,
                        const CUtensorMap& tv, const CUtensorMap& to, const FwdParams& p, int grid,
                        cudaStream_t stream) {
   const bool one_tile = p.cta_rows == 128;
-  if (head_dim == 256) return one_tile ? launch_fwd_d<256, true>(causal, tq, tk, tv, to, p, grid, stream) : cudaErrorInvalidValue;
+  if (head_dim == 256) return one_tile ? launch_fwd_d<256, kOneTile>(causal, tq, tk, tv, to, p, grid, stream) : cudaErrorInvalidValue;
   if (head_dim == 128) {
-    return one_tile ? launch_fwd_d<128, true>(causal, tq, tk, tv, to, p, grid, stream)
-                    : launch_fwd_d<128, false>(causal, tq, tk, tv, to, p, grid, stream);
+    return one_tile ? launch_fwd_d<128, kOneTile>(causal, tq, tk, tv, to, p, grid, stream)
+                    : launch_fwd_d<128, kTwoTiles>(causal, tq, tk, tv, to, p, grid, stream);
   }
   if (head_dim == 64) {
-    return one_tile ? launch_fwd_d<64, true>(causal, tq, tk, tv, to, p, grid, stream)
-                    : launch_fwd_d<64, false>(causal, tq, tk, tv, to, p, grid, stream);
+    if (p.half_sm) return launch_fwd_d<64, kHalfSm>(causal, tq, tk, tv, to, p, grid, stream);
+    return one_tile ? launch_fwd_d<64, kOneTile>(causal, tq, tk, tv, to, p, grid, stream)
+                    : launch_fwd_d<64, kTwoTiles>(causal, tq, tk, tv, to, p, grid, stream);
   }
   return cudaErrorInvalidValue;
 }

@@ -53,9 +53,7 @@ cudaError_t launch_dependent(void (*kern)(Params...), dim3 grid, dim3 block, siz
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-// Forward: grid = number of (p.cta_rows-row block, batch*head) units.  fwd_cta_rows gives the rows
-// a CTA takes: 256 (two query tiles) unless head_dim is 256 or the one-tile variant is asked for.
-int fwd_cta_rows(int head_dim, bool one_tile);
+// Forward: grid = number of (p.cta_rows-row block, batch*head) units.
 cudaError_t launch_fwd(int head_dim, bool causal, const CUtensorMap& tq, const CUtensorMap& tk,
                        const CUtensorMap& tv, const CUtensorMap& to, const FwdParams& p, int grid,
                        cudaStream_t stream);

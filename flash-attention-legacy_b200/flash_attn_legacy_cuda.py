@@ -104,7 +104,7 @@ __version__ = _lib.fal_version().decode()
 KERNEL_FWD, KERNEL_BWD, KERNEL_DECODE_SPLITK = 0, 1, 2
 
 
-FWD_AUTO, FWD_ONE_TILE, FWD_TWO_TILES = 0, 1, 2
+FWD_AUTO, FWD_ONE_TILE, FWD_TWO_TILES, FWD_HALF_SM = 0, 1, 2, 3
 
 
 def set_forward_variant(variant=FWD_AUTO):
