@@ -908,6 +908,32 @@ int fal_decode_static(const void* q, void* k_cache, void* v_cache, const fal_str
                                fal::kDecodeStaticScratchBytes, status, stream);
 }
 
+static_assert(sizeof(fal_fwd_args) == 192 && sizeof(fal_bwd_args) == 328 && sizeof(fal_decode_args) == 176,
+              "the Python binding packs these blocks");
+
+int fal_fwd_args_run(const fal_fwd_args* a) {
+  if (!a) return FAL_ERR_INVALID_ARGUMENT;
+  return fwd_batched(a->q, a->k, a->v, a->o, a->lse, a->cache_seqlens, a->batch, a->heads_q, a->heads_kv, a->seqlen_q,
+                     a->seqlen_k, a->head_dim, &a->q_strides, &a->k_strides, &a->v_strides, &a->o_strides,
+                     a->softmax_scale, a->is_causal, a->status, a->stream);
+}
+
+int fal_bwd_args_run(const fal_bwd_args* a) {
+  if (!a) return FAL_ERR_INVALID_ARGUMENT;
+  return fal_bwd(a->d_out, a->q, a->k, a->v, a->o, a->lse, a->dq, a->dk, a->dv, a->batch, a->heads_q, a->heads_kv,
+                 a->seqlen_q, a->seqlen_k, a->head_dim, &a->do_strides, &a->q_strides, &a->k_strides, &a->v_strides,
+                 &a->o_strides, &a->dq_strides, &a->dk_strides, &a->dv_strides, a->softmax_scale, a->is_causal,
+                 a->workspace, a->workspace_bytes, a->status, a->stream);
+}
+
+int fal_decode_args_run(const fal_decode_args* a) {
+  if (!a) return FAL_ERR_INVALID_ARGUMENT;
+  return decode_with_workspace(a->q, a->k_cache, a->v_cache, &a->k_strides, &a->v_strides, a->cache_starts,
+                               a->cache_seqlens, a->k_new, a->v_new, a->o, a->lse, a->batch, a->heads_q, a->heads_kv,
+                               a->capacity, a->head_dim, a->softmax_scale, a->workspace, a->workspace_bytes,
+                               a->status, a->stream);
+}
+
 int fal_cache_append(const void* k_new, const void* v_new, void* k_cache, void* v_cache,
                      const fal_strides* k_new_strides, const fal_strides* v_new_strides,
                      const fal_strides* k_strides, const fal_strides* v_strides, const int32_t* cache_seqlens,

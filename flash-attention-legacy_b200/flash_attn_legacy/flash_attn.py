@@ -40,6 +40,8 @@ def _kernel_ready(t: torch.Tensor) -> torch.Tensor:
     a real (positive) stride on every dimension longer than one -- an `expand`ed tensor (stride 0:
     K/V broadcast over heads, or the gradient of a `sum`) is copied.
     """
+    if t.is_contiguous():  # (what the general test accepts; a copy would be `t` again)
+        return t
     if (t.stride(-1) == 1 and t.data_ptr() % 16 == 0
             and all(s % 8 == 0 and (s > 0 or n == 1) for s, n in zip(t.stride()[:-1], t.shape[:-1]))):
         return t

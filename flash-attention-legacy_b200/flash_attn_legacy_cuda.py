@@ -13,6 +13,7 @@ device pointers and the current stream.
 """
 import ctypes
 import os
+import struct
 
 import torch
 
@@ -77,6 +78,18 @@ DECODE_STATIC_SCRATCH_BYTES = 8 << 20
 
 _lib.fal_cache_append.restype = _i
 _lib.fal_cache_append.argtypes = [_vp] * 4 + [_sp] * 4 + [_vp] * 3 + [_i] * 5 + [_vp]
+
+# The calls of every model step take one packed argument block (fal_fwd_args and so on in fal_b200.h): one
+# struct.pack and one pointer instead of up to 30 converted arguments, which took longer than the launch.
+_FWD_ARGS = struct.Struct("@6Q6i12qfi2Q")
+_BWD_ARGS = struct.Struct("@9Q6i24qfi4Q")
+_DECODE_ARGS = struct.Struct("@9Q5if6q4Q")
+assert (_FWD_ARGS.size, _BWD_ARGS.size, _DECODE_ARGS.size) == (192, 328, 176)
+for _name in ("fal_fwd_args_run", "fal_bwd_args_run", "fal_decode_args_run"):
+    _fn = getattr(_lib, _name)
+    _fn.restype = _i
+    _fn.argtypes = [ctypes.c_char_p]
+_fwd_run, _bwd_run, _decode_run = _lib.fal_fwd_args_run, _lib.fal_bwd_args_run, _lib.fal_decode_args_run
 
 _lib.fal_profile_enable.restype = _i
 _lib.fal_profile_enable.argtypes = [_i]
@@ -145,6 +158,12 @@ def profile_read(kind):
 _status = {}
 
 
+def _status_ptr(idx):
+    """Device address of the status word of CUDA device `idx`."""
+    t = _status.get(idx)
+    return (t if t is not None else _status_word(torch.device("cuda", idx))).data_ptr()
+
+
 def _status_word(device):
     idx = device.index if device.index is not None else torch.cuda.current_device()
     t = _status.get(idx)
@@ -190,7 +209,7 @@ def _packed_strides(t):
 
 
 def _stream(t):
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    return _raw_stream(t.get_device())
 
 
 def _require_cuda_half(name, t, ndim):
@@ -204,13 +223,19 @@ def _require_cuda_half(name, t, ndim):
         raise RuntimeError(f"{name} must have a contiguous last dimension")
 
 
+_raw_stream = torch._C._cuda_getCurrentRawStream
+_current_device = torch._C._cuda_getDevice
+
+
 def _same_device(*ts):
-    dev = ts[0].device
+    """Index of the device that all tensors (the first is a CUDA tensor) live on; it must be the current one."""
+    dev = ts[0].get_device()
     for t in ts:
-        if t is not None and t.device != dev:
+        if t is not None and t.get_device() != dev:
             raise RuntimeError("all tensors must be on the same device")
-    if dev.index != torch.cuda.current_device():
+    if dev != _current_device():
         raise RuntimeError("tensors must live on the current CUDA device")
+    return dev
 
 
 def forward(Q, K, V, softmax_scale, is_causal=False, out=None, lse=None):
@@ -223,7 +248,7 @@ def forward(Q, K, V, softmax_scale, is_causal=False, out=None, lse=None):
     _require_cuda_half("Q", Q, 4)
     _require_cuda_half("K", K, 4)
     _require_cuda_half("V", V, 4)
-    _same_device(Q, K, V)
+    dev = _same_device(Q, K, V)
     B, Hq, N, d = Q.shape
     Hkv = K.shape[1]
     if K.shape != (B, Hkv, N, d) or V.shape != K.shape:
@@ -232,11 +257,10 @@ def forward(Q, K, V, softmax_scale, is_causal=False, out=None, lse=None):
         raise RuntimeError("H_q must be divisible by H_kv")
     O = torch.empty((B, Hq, N, d), dtype=torch.float16, device=Q.device) if out is None else out
     L = torch.empty((B, Hq, N), dtype=torch.float32, device=Q.device) if lse is None else lse
-    _check(_lib.fal_fwd(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), L.data_ptr(),
-                        B, Hq, Hkv, N, N, d,
-                        _bhn_strides(Q), _bhn_strides(K), _bhn_strides(V), _bhn_strides(O),
-                        float(softmax_scale), int(bool(is_causal)),
-                        _status_word(Q.device).data_ptr(), _stream(Q)))
+    _check(_fwd_run(_FWD_ARGS.pack(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), L.data_ptr(), 0,
+                                   B, Hq, Hkv, N, N, d,
+                                   *Q.stride()[:3], *K.stride()[:3], *V.stride()[:3], *O.stride()[:3],
+                                   softmax_scale, 1 if is_causal else 0, _status_ptr(dev), _raw_stream(dev))))
     return [O, L]
 
 
@@ -287,7 +311,7 @@ def forward_kvcache(Q, K_cache, V_cache, cache_seqlens, softmax_scale, is_causal
     _require_cuda_half("Q", Q, 4)
     _require_cuda_half("K_cache", K_cache, 4)
     _require_cuda_half("V_cache", V_cache, 4)
-    _same_device(Q, K_cache, V_cache, cache_seqlens)
+    dev = _same_device(Q, K_cache, V_cache, cache_seqlens)
     B, Hq, Nq, d = Q.shape
     Hkv, S = K_cache.shape[1], K_cache.shape[2]
     if K_cache.shape[0] != B or tuple(V_cache.shape) != tuple(K_cache.shape) or K_cache.shape[3] != d:
@@ -300,11 +324,10 @@ def forward_kvcache(Q, K_cache, V_cache, cache_seqlens, softmax_scale, is_causal
             raise RuntimeError("out must be [B, H_q, N_q, d]")
     O = out if out is not None else torch.empty((B, Hq, Nq, d), dtype=torch.float16, device=Q.device)
     L = torch.empty((B, Hq, Nq), dtype=torch.float32, device=Q.device)
-    _check(_lib.fal_fwd_kvcache(Q.data_ptr(), K_cache.data_ptr(), V_cache.data_ptr(), O.data_ptr(), L.data_ptr(),
-                                cache_seqlens.data_ptr(), B, Hq, Hkv, Nq, S, d,
-                                _bhn_strides(Q), _bhn_strides(K_cache), _bhn_strides(V_cache), _bhn_strides(O),
-                                float(softmax_scale), 2 if is_causal else 0,
-                                _status_word(Q.device).data_ptr(), _stream(Q)))
+    _check(_fwd_run(_FWD_ARGS.pack(Q.data_ptr(), K_cache.data_ptr(), V_cache.data_ptr(), O.data_ptr(), L.data_ptr(),
+                                   cache_seqlens.data_ptr(), B, Hq, Hkv, Nq, S, d,
+                                   *Q.stride()[:3], *K_cache.stride()[:3], *V_cache.stride()[:3], *O.stride()[:3],
+                                   softmax_scale, 2 if is_causal else 0, _status_ptr(dev), _raw_stream(dev))))
     return [O, L]
 
 
@@ -360,7 +383,7 @@ def backward(dO, Q, K, V, O, L, softmax_scale, is_causal=False, out=None, worksp
     """
     for name, t in (("dO", dO), ("Q", Q), ("K", K), ("V", V), ("O", O)):
         _require_cuda_half(name, t, 4)
-    _same_device(dO, Q, K, V, O, L)
+    dev = _same_device(dO, Q, K, V, O, L)
     B, Hq, Nq, d = Q.shape
     Hkv, Nk = K.shape[1], K.shape[2]
     if dO.shape != Q.shape or O.shape != Q.shape:
@@ -377,13 +400,13 @@ def backward(dO, Q, K, V, O, L, softmax_scale, is_causal=False, out=None, worksp
     ws = torch.empty(nbytes, dtype=torch.uint8, device=Q.device) if workspace is None else workspace
     if ws.numel() < nbytes:
         raise RuntimeError("workspace too small")
-    _check(_lib.fal_bwd(dO.data_ptr(), Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(),
-                        L.data_ptr(), dQ.data_ptr(), dK.data_ptr(), dV.data_ptr(),
-                        B, Hq, Hkv, Nq, Nk, d,
-                        _bhn_strides(dO), _bhn_strides(Q), _bhn_strides(K), _bhn_strides(V),
-                        _bhn_strides(O), _bhn_strides(dQ), _bhn_strides(dK), _bhn_strides(dV),
-                        float(softmax_scale), _causal_code(is_causal, bottom_right),
-                        ws.data_ptr(), nbytes, _status_word(Q.device).data_ptr(), _stream(Q)))
+    _check(_bwd_run(_BWD_ARGS.pack(dO.data_ptr(), Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(),
+                                   L.data_ptr(), dQ.data_ptr(), dK.data_ptr(), dV.data_ptr(),
+                                   B, Hq, Hkv, Nq, Nk, d,
+                                   *dO.stride()[:3], *Q.stride()[:3], *K.stride()[:3], *V.stride()[:3],
+                                   *O.stride()[:3], *dQ.stride()[:3], *dK.stride()[:3], *dV.stride()[:3],
+                                   softmax_scale, _causal_code(is_causal, bottom_right),
+                                   ws.data_ptr(), nbytes, _status_ptr(dev), _raw_stream(dev))))
     return [dQ, dK, dV]
 
 
@@ -527,7 +550,7 @@ def _decode_workspace(device, nbytes):
     One workspace per (device, stream): calls on different streams may overlap on the GPU and must
     not share partial results.  A workspace is replaced when a call needs more room.
     """
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    key = (device.index, _raw_stream(device.index))
     ws = _decode_ws.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
@@ -548,12 +571,11 @@ def _decode_args(q, k_cache, v_cache, cache_seqlens, k_new, v_new, cache_layout,
         raise RuntimeError("k_cache and v_cache must have the same shape")
     if cache_layout == "bshd":
         S, Hkv = k_cache.shape[1], k_cache.shape[2]
-        ks = _Strides(k_cache.stride(0), k_cache.stride(2), k_cache.stride(1))
-        vs = _Strides(v_cache.stride(0), v_cache.stride(2), v_cache.stride(1))
+        (kb, kr, kh, _), (vb, vr, vh, _) = k_cache.stride(), v_cache.stride()
+        ks, vs = (kb, kh, kr), (vb, vh, vr)
     elif cache_layout == "bhsd":
         Hkv, S = k_cache.shape[1], k_cache.shape[2]
-        ks = _Strides(k_cache.stride(0), k_cache.stride(1), k_cache.stride(2))
-        vs = _Strides(v_cache.stride(0), v_cache.stride(1), v_cache.stride(2))
+        ks, vs = k_cache.stride()[:3], v_cache.stride()[:3]
     else:
         raise ValueError("cache_layout must be 'bshd' or 'bhsd'")
     if k_cache.shape[0] != B or k_cache.shape[3] != d:
@@ -595,17 +617,15 @@ def decode(q, k_cache, v_cache, cache_seqlens, softmax_scale, k_new=None, v_new=
     lse = torch.empty((B, Hq), dtype=torch.float32, device=q.device) if return_lse else None
     nbytes = max(_lib.fal_decode_workspace_bytes(B, Hq, S, d), _DECODE_WS_MIN)
     ws = _decode_workspace(q.device, nbytes)
-    tail = (k_new.data_ptr() if k_new is not None else None,
-            v_new.data_ptr() if v_new is not None else None,
-            o.data_ptr(), lse.data_ptr() if lse is not None else None,
-            B, Hq, Hkv, S, d, float(softmax_scale), ws.data_ptr(), nbytes,
-            _status_word(q.device).data_ptr(), _stream(q))
-    if cache_starts is None:
-        _check(_lib.fal_decode(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), ks, vs,
-                               cache_seqlens.data_ptr(), *tail))
-    else:
-        _check(_lib.fal_decode_ranged(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), ks, vs,
-                                      cache_starts.data_ptr(), cache_seqlens.data_ptr(), *tail))
+    dev = q.get_device()
+    _check(_decode_run(_DECODE_ARGS.pack(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
+                                         cache_starts.data_ptr() if cache_starts is not None else 0,
+                                         cache_seqlens.data_ptr(),
+                                         k_new.data_ptr() if k_new is not None else 0,
+                                         v_new.data_ptr() if v_new is not None else 0,
+                                         o.data_ptr(), lse.data_ptr() if lse is not None else 0,
+                                         B, Hq, Hkv, S, d, softmax_scale, *ks, *vs,
+                                         ws.data_ptr(), nbytes, _status_ptr(dev), _raw_stream(dev))))
     return (o, lse) if return_lse else o
 
 
@@ -663,7 +683,7 @@ def decode_static(q, k_cache, v_cache, cache_seqlens, softmax_scale, out, k_new=
     """
     B, Hq, Hkv, S, d, ks, vs = _decode_args(q, k_cache, v_cache, cache_seqlens, k_new, v_new, cache_layout,
                                             out, lse)
-    _check(_lib.fal_decode_static(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), ks, vs,
+    _check(_lib.fal_decode_static(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), _Strides(*ks), _Strides(*vs),
                                   cache_seqlens.data_ptr(),
                                   k_new.data_ptr() if k_new is not None else None,
                                   v_new.data_ptr() if v_new is not None else None,

@@ -289,6 +289,57 @@ FAL_API int fal_decode_ranged(const void* q, void* k_cache, void* v_cache,
                int* status, void* stream);
 
 /*
+ * fal_fwd / fal_fwd_kvcache (cache_seqlens set), fal_bwd and fal_decode / fal_decode_ranged (cache_starts set)
+ * with their arguments in one block, for hosts where converting each argument costs more than the launch.
+ */
+typedef struct fal_fwd_args {
+  const void *q, *k, *v;
+  void* o;
+  float* lse;
+  const int32_t* cache_seqlens; /* optional: keys in use per batch entry, seqlen_k is then the capacity */
+  int batch, heads_q, heads_kv, seqlen_q, seqlen_k, head_dim;
+  fal_strides q_strides, k_strides, v_strides, o_strides;
+  float softmax_scale;
+  int is_causal;
+  int* status;
+  void* stream;
+} fal_fwd_args;
+FAL_API int fal_fwd_args_run(const fal_fwd_args* args);
+
+typedef struct fal_bwd_args {
+  const void *d_out, *q, *k, *v, *o;
+  const float* lse;
+  void *dq, *dk, *dv;
+  int batch, heads_q, heads_kv, seqlen_q, seqlen_k, head_dim;
+  fal_strides do_strides, q_strides, k_strides, v_strides, o_strides, dq_strides, dk_strides, dv_strides;
+  float softmax_scale;
+  int is_causal;
+  void* workspace;
+  size_t workspace_bytes;
+  int* status;
+  void* stream;
+} fal_bwd_args;
+FAL_API int fal_bwd_args_run(const fal_bwd_args* args);
+
+typedef struct fal_decode_args {
+  const void* q;
+  void *k_cache, *v_cache;
+  const int32_t *cache_starts; /* optional */
+  const int32_t *cache_seqlens;
+  const void *k_new, *v_new;   /* optional */
+  void* o;
+  float* lse;                  /* optional */
+  int batch, heads_q, heads_kv, capacity, head_dim;
+  float softmax_scale;
+  fal_strides k_strides, v_strides;
+  void* workspace;
+  size_t workspace_bytes;
+  int* status;
+  void* stream;
+} fal_decode_args;
+FAL_API int fal_decode_args_run(const fal_decode_args* args);
+
+/*
  * Writes a chunk of new rows into K and V caches filled to a different length per entry: row i of entry b
  * goes to position cache_seqlens[b] + i (a negative position counts from the end of the cache).
  * new_seqlens[b] = cache_seqlens[b] + rows; *fits (one byte on the device) becomes 1 if every row had a place and
