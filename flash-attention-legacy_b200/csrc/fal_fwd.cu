@@ -167,6 +167,48 @@ struct FwdWork {
   int64_t lse_base;  // float offset of the same
 };
 
+// The slot-th heaviest (entry, query block) of a chunk of queries behind caches of different lengths, by key
+// tiles: entry b's block q sees about lens[b] + q * cta_rows keys.  Every warp finds it for itself: a binary
+// search over the tile count (how many blocks have at least v tiles: a closed form per entry, entries on the
+// lanes), then the rank among the blocks of exactly that count, of which an entry has at most one.
+__device__ __forceinline__ void fwd_heaviest_block(const FwdParams& p, int slot, int& entry, int& qblk) {
+  const int lane = threadIdx.x & 31;
+  auto blocks_from = [&](int b, int v) -> int {  // blocks of entry b with at least v tiles
+    const int len = max(min(__ldg(p.seqused_k + b), p.seqlen_k), 0);
+    const int short_by = v * kTileN - len;
+    return p.num_qblk - min(max((short_by + p.cta_rows - 1) / p.cta_rows, 0), p.num_qblk);
+  };
+  auto count = [&](int v) -> int {
+    int n = 0;
+    for (int b = lane; b < p.batch; b += 32) n += blocks_from(b, v);
+    return __reduce_add_sync(0xffffffffu, n);
+  };
+  int lo = 0;  // count(lo) > slot
+  int hi = (p.seqlen_k + p.num_qblk * p.cta_rows) / kTileN + 1;  // count(hi) == 0
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (count(mid) > slot) lo = mid;
+    else hi = mid;
+  }
+  int rank = slot - count(lo + 1);
+  entry = 0;
+  qblk = 0;
+  for (int base = 0; base < p.batch; base += 32) {
+    const int b = base + lane;
+    const int n = b < p.batch ? blocks_from(b, lo) : 0;
+    const bool has = b < p.batch && n > blocks_from(b, lo + 1);
+    const unsigned mask = __ballot_sync(0xffffffffu, has);
+    if (rank < __popc(mask)) {
+      const unsigned hit = __ballot_sync(0xffffffffu, has && __popc(mask & ((1u << lane) - 1u)) == rank);
+      const int src = __ffs(hit) - 1;
+      entry = base + src;
+      qblk = p.num_qblk - __shfl_sync(0xffffffffu, n, src);
+      return;
+    }
+    rank -= __popc(mask);
+  }
+}
+
 // Maps blockIdx.x to a unit of work.  Returns false when the block has none
 // (packed mode launches an upper bound of blocks).
 __device__ __forceinline__ bool fwd_decode_work(const FwdParams& p, int cta_rows, FwdWork& w) {
@@ -178,6 +220,13 @@ __device__ __forceinline__ bool fwd_decode_work(const FwdParams& p, int cta_rows
     const int bh = idx % bh_count;
     w.batch = bh / p.heads_q;
     w.head = bh % p.heads_q;
+    if (p.seqused_k != nullptr && p.shift_per_sequence != 0 && p.batch > 1) {
+      // Entries of 1 500 and of 8 000 keys in one grid: in the order above the longest entry's last blocks
+      // start late and the SMs wait for them.  Heaviest first, 4 entries x 1 024 queries (32 / 8 heads of 128)
+      // behind 512 to 7 000 keys: 329 -> 310 us a call; the search costs a CTA well under a microsecond.
+      w.head = idx % p.heads_q;
+      fwd_heaviest_block(p, idx / p.heads_q, w.batch, w.qblk);
+    }
     w.q_row0 = 0;
     w.k_row0 = 0;
     w.seqlen_q = p.seqlen_q;
@@ -222,7 +271,8 @@ __device__ __forceinline__ bool fwd_decode_work(const FwdParams& p, int cta_rows
       }
     }
     if (seq < 0) return false;
-    w.qblk = slot - first;
+    // a sequence's last block first: under a causal mask it is the heaviest
+    w.qblk = (w.seqlen_q + cta_rows - 1) / cta_rows - 1 - (slot - first);
     w.q_row0 = q_start;
     w.k_row0 = __ldg(p.cu_k + seq);
     w.seqlen_k = __ldg(p.cu_k + seq + 1) - w.k_row0;
