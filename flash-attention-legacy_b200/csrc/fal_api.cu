@@ -189,6 +189,22 @@ int forward_variant(int head_dim, int64_t blocks_of_256_rows, int64_t units, int
   return 6 * waves1 < 10 * waves2 ? FAL_FWD_ONE_TILE : FAL_FWD_TWO_TILES;
 }
 
+// CTAs that share the keys of each query block of a chunk behind a cache.  A chunk with fewer than half as many
+// 128-row blocks as there are SMs is bound by one CTA's walk over the cache; its keys are then dealt to as many
+// CTAs as the SMs hold, two key tiles or more each.  us a call, one CTA per block against this: 1 entry (32 / 8 heads of 128)
+// behind 4 000 keys, 16 queries 83 / 32, 128 queries 85 / 38, 512 queries 95 / 64; 1 entry (8 / 1 of 64) behind
+// 8 000, 40 queries 101 / 30; 2 entries (16 of 256) behind 1 500 and 3 000, 60 queries 99 / 48.
+int chunk_kv_splits(int64_t blocks, int capacity) {
+  const int64_t sms = sm_count() > 0 ? sm_count() : 148;
+  const int64_t most = (capacity + 255) / 256;
+  int64_t s = blocks > 0 ? sms / blocks : 1;
+  if (s > most) s = most;
+  return s < 2 ? 1 : static_cast<int>(s < 32 ? s : 32);  // (the merge takes a split per lane)
+}
+size_t chunk_split_bytes(int splits, int batch, int heads_q, int seqlen_q, int head_dim) {
+  return splits < 2 ? 0 : static_cast<size_t>(splits) * batch * heads_q * seqlen_q * (head_dim + 1) * sizeof(float);
+}
+
 int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 
 // Backward scratch layout: [dq_accum fp32 batch*heads*padded_rows*d][delta fp32 batch*heads*padded_rows]
@@ -313,7 +329,7 @@ int fwd_batched(const void* q, const void* k, const void* v, void* o, float* lse
                 int seqlen_k, int head_dim, const fal_strides* q_strides,
                 const fal_strides* k_strides, const fal_strides* v_strides,
                 const fal_strides* o_strides, float softmax_scale, int is_causal, int* status,
-                void* stream) {
+                void* stream, void* workspace = nullptr, size_t workspace_bytes = 0) {
   if (!q || !k || !v || !o || !lse || !q_strides || !k_strides || !v_strides || !o_strides)
     return FAL_ERR_INVALID_ARGUMENT;
   if (batch <= 0 || heads_q <= 0 || heads_kv <= 0 || seqlen_q <= 0 || seqlen_k < 0)
@@ -367,8 +383,19 @@ int fwd_batched(const void* q, const void* k, const void* v, void* o, float* lse
   p.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int kdim = kernel_head_dim(head_dim);
-  const int variant = forward_variant(kdim, (seqlen_q + 255) / 256, static_cast<int64_t>(batch) * heads_q,
-                                      is_causal == 1 ? seqlen_k / 2 : seqlen_k);
+  int variant = forward_variant(kdim, (seqlen_q + 255) / 256, static_cast<int64_t>(batch) * heads_q,
+                                is_causal == 1 ? seqlen_k / 2 : seqlen_k);
+  p.kv_splits = 1;
+  if (seqused_k != nullptr && workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) {
+    const int64_t blocks = static_cast<int64_t>((seqlen_q + 127) / 128) * batch * heads_q;
+    const int splits = chunk_kv_splits(blocks, seqlen_k);
+    if (splits > 1 && workspace_bytes >= chunk_split_bytes(splits, batch, heads_q, seqlen_q, head_dim)) {
+      p.kv_splits = splits;
+      p.part_o = static_cast<float*>(workspace);
+      p.part_lse = p.part_o + static_cast<int64_t>(splits) * batch * heads_q * seqlen_q * head_dim;
+      variant = FAL_FWD_ONE_TILE;
+    }
+  }
   p.half_sm = variant == FAL_FWD_HALF_SM;
   p.cta_rows = variant == FAL_FWD_TWO_TILES ? 256 : 128;
   p.num_qblk = (seqlen_q + p.cta_rows - 1) / p.cta_rows;
@@ -377,6 +404,7 @@ int fwd_batched(const void* q, const void* k, const void* v, void* o, float* lse
   const int rec = g_timer.begin(FAL_KERNEL_FWD, st);
   cudaError_t e = fal::launch_fwd(kdim, is_causal != 0, tq, tk, tv, to, p, static_cast<int>(grid), st);
   g_timer.end(FAL_KERNEL_FWD, rec, st);
+  if (e == cudaSuccess && p.kv_splits > 1) e = fal::launch_fwd_combine(p, st);
   return e == cudaSuccess ? FAL_OK : cuda_fail(e);
 }
 
@@ -916,6 +944,19 @@ int fal_fwd_args_run(const fal_fwd_args* a) {
   return fwd_batched(a->q, a->k, a->v, a->o, a->lse, a->cache_seqlens, a->batch, a->heads_q, a->heads_kv, a->seqlen_q,
                      a->seqlen_k, a->head_dim, &a->q_strides, &a->k_strides, &a->v_strides, &a->o_strides,
                      a->softmax_scale, a->is_causal, a->status, a->stream);
+}
+
+size_t fal_fwd_kvcache_workspace_bytes(int batch, int heads_q, int seqlen_q, int cache_capacity, int head_dim) {
+  if (batch <= 0 || heads_q <= 0 || seqlen_q <= 0 || cache_capacity <= 0 || !head_dim_ok(head_dim)) return 0;
+  const int64_t blocks = static_cast<int64_t>((seqlen_q + 127) / 128) * batch * heads_q;
+  return chunk_split_bytes(chunk_kv_splits(blocks, cache_capacity), batch, heads_q, seqlen_q, head_dim);
+}
+
+int fal_fwd_kvcache_split_run(const fal_fwd_args* a, void* workspace, size_t workspace_bytes) {
+  if (!a || !a->cache_seqlens) return FAL_ERR_INVALID_ARGUMENT;
+  return fwd_batched(a->q, a->k, a->v, a->o, a->lse, a->cache_seqlens, a->batch, a->heads_q, a->heads_kv, a->seqlen_q,
+                     a->seqlen_k, a->head_dim, &a->q_strides, &a->k_strides, &a->v_strides, &a->o_strides,
+                     a->softmax_scale, a->is_causal, a->status, a->stream, workspace, workspace_bytes);
 }
 
 int fal_bwd_args_run(const fal_bwd_args* a) {

@@ -42,6 +42,9 @@ struct FwdParams {
   int store_by_tma;  // O tiles leave through shared memory and TMA stores (the output's tensor map is valid)
   const int32_t* seqused_k;  // batched mode, optional: keys in use per batch entry (a cache filled to different
                              // lengths); seqlen_k is then the capacity, and shift_per_sequence applies per entry
+  int kv_splits;     // (seqused_k) CTAs that share a query block's keys, each a range of key tiles; 1: none
+  float* part_o;     // kv_splits > 1: [split, batch, heads_q, seqlen_q, head_dim] fp32, normalised per split
+  float* part_lse;   // [split, batch, heads_q, seqlen_q]
   float scale;       // softmax scale
   float scale_log2;  // softmax scale * log2(e)
   int* status;       // device status word, may be nullptr

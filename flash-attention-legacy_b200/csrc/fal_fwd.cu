@@ -326,9 +326,19 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 
   // SHIFTED: keys the causal diagonal is moved by (batched: one value; packed, or a cache with its
   // own length per entry: each sequence's seqlen_k - seqlen_q).
-  const int cshift = SHIFTED ? ((p.cu_q != nullptr || p.seqused_k != nullptr) ? wk.seqlen_k - wk.seqlen_q
+  int cshift = SHIFTED ? ((p.cu_q != nullptr || p.seqused_k != nullptr) ? wk.seqlen_k - wk.seqlen_q
                                                                               : p.causal_shift)
                              : 0;
+  // Several CTAs share this block's keys: this one takes its range of the entry's key tiles, as a shorter key
+  // sequence with the diagonal moved along.
+  if (p.kv_splits > 1) {
+    const int tiles = (wk.seqlen_k + kTileN - 1) / kTileN;
+    const int per = (tiles + p.kv_splits - 1) / p.kv_splits;
+    const int key0 = min(static_cast<int>(blockIdx.y) * per, tiles) * kTileN;
+    wk.seqlen_k = max(min(wk.seqlen_k - key0, per * kTileN), 0);
+    wk.k_row0 += key0;
+    if (SHIFTED) cshift -= key0;
+  }
   // Number of key tiles each 128-row query tile visits.
   const int nk_tiles = (wk.seqlen_k + kTileN - 1) / kTileN;
   int ntile[2];
@@ -786,8 +796,10 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const bool tile_used = (kAlt || wg < L::kQTiles) && q_tile0 < wk.seqlen_q;
     // (Not at head_dim 256: measured 5 - 10 % slower there -- the CTA then waits for the TMA unit to read
     // 64 KB of staging before it can exit, where plain stores drain behind its back.)
-    const bool by_tma = D != 256 && p.store_by_tma != 0 && tile_used &&
+    const bool by_tma = D != 256 && p.store_by_tma != 0 && p.kv_splits <= 1 && tile_used &&
                         (p.cu_q == nullptr || q_tile0 + kTileM <= wk.seqlen_q);
+    const int64_t part_row =
+        ((static_cast<int64_t>(blockIdx.y) * p.batch + wk.batch) * p.heads_q + wk.head) * p.seqlen_q + q_local;
     uint8_t* stage_row = sgen + L::kQOff + (kAlt ? 0 : wg * L::kTileBytes) + row * 128;
 #pragma unroll
     for (int c = 0; c < D / 32; ++c) {
@@ -811,6 +823,15 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           // box c / 2, 16-byte chunk (c % 2) * 4 + v of the row, 128-byte XOR swizzle
           *reinterpret_cast<uint4*>(stage_row + (c >> 1) * L::kBoxBytes + ((((c & 1) * 4 + v) ^ (row & 7)) << 4)) = out;
         }
+      } else if (row_ok && p.kv_splits > 1) {
+        float* part = p.part_o + part_row * p.head_dim + c * 32;
+        if (c * 32 < p.head_dim) {
+#pragma unroll
+          for (int v = 0; v < 8; ++v)
+            *reinterpret_cast<float4*>(part + v * 4) =
+                make_float4(__uint_as_float(r[v * 4 + 0]) * inv, __uint_as_float(r[v * 4 + 1]) * inv,
+                            __uint_as_float(r[v * 4 + 2]) * inv, __uint_as_float(r[v * 4 + 3]) * inv);
+        }
       } else if (row_ok) {
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -827,7 +848,8 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     if (row_ok && (!kAlt || wg == 0)) {
       const float lse = (nt > 0 && m_ref != kNegInf) ? m_ref * p.scale + logf(fmaxf(l, 1e-20f))
                                                       : kNegInf;
-      p.lse[wk.lse_base + static_cast<int64_t>(q_local) * p.lse_strides.row] = lse;
+      if (p.kv_splits > 1) p.part_lse[part_row] = lse;
+      else p.lse[wk.lse_base + static_cast<int64_t>(q_local) * p.lse_strides.row] = lse;
     }
     if (by_tma) {  // the same for every thread that wrote into the tile's staging buffer
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -853,6 +875,52 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   }
 }
 
+// Merges the splits of a query block's keys: a warp per (batch, head, row), split s on lane s for the weights,
+// 16 bytes of every split's row per lane for the sum.  Bound by the partials' traffic, at most 128 rows per SM.
+__global__ void __launch_bounds__(128) fal_fwd_combine_kernel(const FwdParams p) {
+  const int lane = threadIdx.x & 31;
+  const int64_t rows = static_cast<int64_t>(p.batch) * p.heads_q * p.seqlen_q;
+  const int64_t id = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
+  if (id >= rows) return;
+  const float l = lane < p.kv_splits ? p.part_lse[lane * rows + id] : kNegInf;
+  float m = l;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+  const float m_use = m == kNegInf ? 0.f : m;
+  float w = fast_exp2((l - m_use) * 1.4426950408889634f);
+  float sum = w;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  w *= sum > 0.f ? 1.f / sum : 0.f;
+  const int row = static_cast<int>(id % p.seqlen_q);
+  const int64_t bh = id / p.seqlen_q;
+  const int head = static_cast<int>(bh % p.heads_q);
+  const int64_t b = bh / p.heads_q;
+  __half* o = static_cast<__half*>(p.o) + b * p.o_strides.batch + head * p.o_strides.head +
+              static_cast<int64_t>(row) * p.o_strides.row;
+  for (int base = 0; base < p.head_dim; base += 128) {
+    const int c = base + lane * 4;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < p.kv_splits; ++s) {
+      const float ws = __shfl_sync(0xffffffffu, w, s);
+      if (c < p.head_dim) {
+        const float4 x = *reinterpret_cast<const float4*>(p.part_o + (s * rows + id) * p.head_dim + c);
+        acc.x += ws * x.x;
+        acc.y += ws * x.y;
+        acc.z += ws * x.z;
+        acc.w += ws * x.w;
+      }
+    }
+    if (c < p.head_dim) {
+      uint2 out;
+      out.x = pack_half2(acc.x, acc.y);
+      out.y = pack_half2(acc.z, acc.w);
+      *reinterpret_cast<uint2*>(o + c) = out;
+    }
+  }
+  if (lane == 0) p.lse[b * p.lse_strides.batch + head * p.lse_strides.head + row] = sum > 0.f ? m + logf(sum) : kNegInf;
+}
+
 template <int D, bool CAUSAL, bool SHIFTED, int SHAPE>
 cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const CUtensorMap& to, const FwdParams& p, int grid, cudaStream_t stream) {
@@ -863,7 +931,7 @@ cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAllocBytes);
   });
   if (e != cudaSuccess) return e;
-  kern<<<grid, L::kThreads, L::kAllocBytes, stream>>>(tq, tk, tv, to, p);
+  kern<<<dim3(grid, p.kv_splits > 1 ? p.kv_splits : 1), L::kThreads, L::kAllocBytes, stream>>>(tq, tk, tv, to, p);
   return cudaGetLastError();
 }
 
@@ -877,6 +945,12 @@ cudaError_t launch_fwd_d(bool causal, const CUtensorMap& tq, const CUtensorMap& 
 }
 
 }  // namespace
+
+cudaError_t launch_fwd_combine(const FwdParams& p, cudaStream_t stream) {
+  const int64_t rows = static_cast<int64_t>(p.batch) * p.heads_q * p.seqlen_q;
+  fal_fwd_combine_kernel<<<static_cast<unsigned>((rows + 3) / 4), 128, 0, stream>>>(p);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_fwd(int head_dim, bool causal, const CUtensorMap& tq, const CUtensorMap& tk,
                        const CUtensorMap& tv, const CUtensorMap& to, const FwdParams& p, int grid,

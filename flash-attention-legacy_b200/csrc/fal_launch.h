@@ -58,6 +58,9 @@ cudaError_t launch_fwd(int head_dim, bool causal, const CUtensorMap& tq, const C
                        const CUtensorMap& tv, const CUtensorMap& to, const FwdParams& p, int grid,
                        cudaStream_t stream);
 
+// Merges the partial results of a forward with p.kv_splits > 1 into p.o and p.lse.
+cudaError_t launch_fwd_combine(const FwdParams& p, cudaStream_t stream);
+
 // Backward pre-pass: delta = rowsum(dO * O) and zero of the fp32 dQ accumulator.
 struct BwdPrepParams {
   const void* o;

@@ -89,6 +89,10 @@ for _name in ("fal_fwd_args_run", "fal_bwd_args_run", "fal_decode_args_run"):
     _fn = getattr(_lib, _name)
     _fn.restype = _i
     _fn.argtypes = [ctypes.c_char_p]
+_lib.fal_fwd_kvcache_workspace_bytes.restype = ctypes.c_size_t
+_lib.fal_fwd_kvcache_workspace_bytes.argtypes = [_i] * 5
+_lib.fal_fwd_kvcache_split_run.restype = _i
+_lib.fal_fwd_kvcache_split_run.argtypes = [ctypes.c_char_p, _vp, ctypes.c_size_t]
 _fwd_run, _bwd_run, _decode_run = _lib.fal_fwd_args_run, _lib.fal_bwd_args_run, _lib.fal_decode_args_run
 
 _lib.fal_profile_enable.restype = _i
@@ -324,10 +328,16 @@ def forward_kvcache(Q, K_cache, V_cache, cache_seqlens, softmax_scale, is_causal
             raise RuntimeError("out must be [B, H_q, N_q, d]")
     O = out if out is not None else torch.empty((B, Hq, Nq, d), dtype=torch.float16, device=Q.device)
     L = torch.empty((B, Hq, Nq), dtype=torch.float32, device=Q.device)
-    _check(_fwd_run(_FWD_ARGS.pack(Q.data_ptr(), K_cache.data_ptr(), V_cache.data_ptr(), O.data_ptr(), L.data_ptr(),
-                                   cache_seqlens.data_ptr(), B, Hq, Hkv, Nq, S, d,
-                                   *Q.stride()[:3], *K_cache.stride()[:3], *V_cache.stride()[:3], *O.stride()[:3],
-                                   softmax_scale, 2 if is_causal else 0, _status_ptr(dev), _raw_stream(dev))))
+    args = _FWD_ARGS.pack(Q.data_ptr(), K_cache.data_ptr(), V_cache.data_ptr(), O.data_ptr(), L.data_ptr(),
+                          cache_seqlens.data_ptr(), B, Hq, Hkv, Nq, S, d,
+                          *Q.stride()[:3], *K_cache.stride()[:3], *V_cache.stride()[:3], *O.stride()[:3],
+                          softmax_scale, 2 if is_causal else 0, _status_ptr(dev), _raw_stream(dev))
+    nbytes = _lib.fal_fwd_kvcache_workspace_bytes(B, Hq, Nq, S, d)
+    if nbytes:
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=Q.device)
+        _check(_lib.fal_fwd_kvcache_split_run(args, ws.data_ptr(), nbytes))
+    else:
+        _check(_fwd_run(args))
     return [O, L]
 
 

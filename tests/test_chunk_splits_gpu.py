@@ -1,0 +1,42 @@
+"""A chunk of new tokens too small to fill the GPU: several thread blocks share each query block's keys."""
+import math
+
+import pytest
+import torch
+
+from oracle import attention_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture()
+def ext():
+    import flash_attn_legacy_cuda as m
+    return m
+
+
+# One and two query blocks; entries whose keys end inside the first split, at a tile's edge, in the last split; an
+# entry shorter than the chunk (its first queries see no key) and an empty one; every head_dim; up to 32 splits.
+@pytest.mark.parametrize("hq,hkv,d,nq,lens,capacity", [
+    (4, 1, 128, 2, [1999], 2100), (8, 2, 64, 130, [130, 512, 3000], 3001), (2, 2, 256, 128, [640, 100], 700),
+    (6, 3, 96, 37, [5, 0, 1300, 129], 1300), (1, 1, 32, 300, [9000], 9001)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_split_chunk_against_the_oracle(ext, hq, hkv, d, nq, lens, capacity, causal):
+    gen = torch.Generator().manual_seed(d + nq)
+    b, scale = len(lens), 1 / math.sqrt(d)
+    assert ext._lib.fal_fwd_kvcache_workspace_bytes(b, hq, nq, capacity, d) > 0
+    q = torch.randn(b, hq, nq, d, generator=gen).half()
+    kc, vc = (torch.randn(b, hkv, capacity, d, generator=gen).half() for _ in range(2))
+    for i, n in enumerate(lens):   # what lies behind a length does not matter
+        kc[i, :, n:] = float("nan")
+        vc[i, :, n:] = float("inf")
+    lens = torch.tensor(lens, dtype=torch.int32)
+    wide = torch.full((b, hq, nq, d + 8), 7.0, dtype=torch.float16, device="cuda")   # guard columns
+    o, lse = ext.forward_kvcache(q.cuda(), kc.cuda(), vc.cuda(), lens.cuda(), scale, causal, out=wide[..., :d])
+    o_ref, lse_ref = orc.kvcache_chunk_fwd(q, kc, vc, lens, scale, causal)
+    assert orc.rel_max_err(o, o_ref) <= orc.TOL_O
+    seen = torch.isfinite(lse_ref)
+    assert orc.abs_max_err(lse.cpu()[seen], lse_ref[seen]) <= orc.TOL_LSE
+    assert torch.isneginf(lse.cpu()[~seen]).all() and not o.cpu()[~seen].any()
+    assert (wide[..., d:] == 7.0).all()
+    assert ext.device_status() == 0
