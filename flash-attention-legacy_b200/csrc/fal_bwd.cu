@@ -37,13 +37,16 @@
 //               that step's consumed dP^T), dV [256,256+D), dK [256+D,256+2D).
 // Shared memory at head_dim 128: K 32K, V 32K, Q 2 x 32K, dO 32K, dS^T 32K, dQ staging 2 x 16K.
 //
-// head_dim 256 (SPLIT = true) runs the head_dim-128 layout on column halves: two CTAs share a key
-// tile, each owning 128 of the 256 columns of dV, dK and dQ.  The two score GEMMs contract over all
-// 256 columns, so every step first loads the OTHER half of K, Q, V and dO into the (single) tile
-// buffers and starts S^T and dP^T on it, then loads its own half over them and accumulates; from
-// there the step is the head_dim-128 step.  K and V are therefore reloaded every step (they come
-// from L2) and a step's loads and GEMMs run one after the other: it is the reference's head_dim
-// 256 backward made available, not a tuned kernel.
+// head_dim 256 (SPLIT = true): two CTAs share a key tile, each owning 128 of the 256 columns of dV, dK and
+// dQ.  The two score GEMMs contract over all 256 columns, so a CTA needs both halves of K, Q, V and dO:
+// K and V stay in shared memory for the whole key tile (128 KB); of Q and dO the own half has a buffer and
+// the other half passes through one more, X, which then takes dS^T.  A step: S^T = K Q^T (other half from X,
+// own half), dP^T = V dO^T (the same), dV, dQ, dK.  128 KB a step come from L2.  Bound by the latency of a
+// step's chain of loads, GEMMs and softmax, of which only the own dO's load overlaps the step before.
+// 2 x 16 heads x 2 048 causal: 327 us; with K and V reloaded every step (256 KB, all eight half tiles through
+// four buffers) 395.
+#include <type_traits>
+
 #include "fal_common.h"
 #include "fal_launch.h"
 #include "sm100_ptx.cuh"
@@ -61,6 +64,7 @@ enum BwdBarrier : int {
   kBbKFull = 100, kBbVFull = 101, kBbQFull = 110, kBbDoFull = 120, kBbStatFull = 130,
   kBbQEmpty = 140, kBbDoEmpty = 145, kBbSReady = 150, kBbDpReady = 160, kBbPReady = 161,
   kBbDsReady = 162, kBbDqReady = 164, kBbDqFree = 165, kBbAllDone = 166, kBbAFull = 170, kBbADone = 171,
+  kBbBFull = 172,
 };
 
 template <int D>
@@ -81,13 +85,34 @@ struct BwdSmem {
   static constexpr int kStatBytes = kQStages * 2 * kQTile * 4;
   static constexpr int kBarOff = kStatOff + kStatBytes;
   // k_full v_full q_full[2] q_empty[2] stat_full[2] do_full do_empty
-  // s_ready dp_ready dq_ready dq_free p_ready ds_ready all_done ds_free a_full a_done
-  static constexpr int kNumBars = 2 + 6 + 2 + 8 + 2;
+  // s_ready dp_ready dq_ready dq_free p_ready ds_ready all_done ds_free a_full a_done b_full
+  static constexpr int kNumBars = 2 + 6 + 2 + 8 + 3;
   static constexpr int kMiscOff = kBarOff + kNumBars * 8;
   static constexpr int kBytes = kMiscOff + 16;
   // No slack for re-aligning the base: at head_dim 128 the layout fills the 227 KB limit, so the
   // kernel requires the dynamic shared memory window itself to be 1024-byte aligned and reports
   // an error otherwise.
+  static constexpr int kAllocBytes = kBytes;
+  static_assert(kAllocBytes <= 232448, "exceeds the per-CTA shared memory limit");
+};
+
+// The layout of the head_dim 256 kernel: K and V in full (own columns, then the other CTA's), one Q and one
+// dO buffer (own columns), and X = kDsOff: Q's other columns, then dO's, then dS^T.
+struct BwdSplitSmem {
+  static constexpr int kQStages = 1;
+  static constexpr int kBoxes = 2;
+  static constexpr int kBoxBytes = 128 * 128;
+  static constexpr int kTileBytes = kBoxes * kBoxBytes;
+  static constexpr int kKOff = 0;
+  static constexpr int kVOff = 2 * kTileBytes;
+  static constexpr int kQOff = 4 * kTileBytes;
+  static constexpr int kDoOff = 5 * kTileBytes;
+  static constexpr int kDsOff = 6 * kTileBytes;
+  static constexpr int kStatOff = 7 * kTileBytes;
+  static constexpr int kBarOff = kStatOff + 2 * kQTile * 4;
+  static constexpr int kNumBars = 21;
+  static constexpr int kMiscOff = kBarOff + kNumBars * 8;
+  static constexpr int kBytes = kMiscOff + 16;
   static constexpr int kAllocBytes = kBytes;
   static_assert(kAllocBytes <= 232448, "exceeds the per-CTA shared memory limit");
 };
@@ -199,6 +224,45 @@ __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* map, uint32
       : "memory");
 }
 
+__device__ __forceinline__ void red_add_v4(float* dst, const uint32_t (&v)[4]) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(__uint_as_float(v[0])),
+               "f"(__uint_as_float(v[1])), "f"(__uint_as_float(v[2])), "f"(__uint_as_float(v[3]))
+               : "memory");
+}
+
+// Adds 16 rows of a dQ tile to the accumulator rows at `rows` (row_floats apart; the first `valid` of them).
+// r[c][4 k + 0, 1]: columns 64 c + 8 k + 2 (lane % 4) + {0, 1} of row lane / 4; r[c][4 k + 2, 3]: of row
+// lane / 4 + 8.  Lanes trade registers until an instruction covers RED_SHAPE
+template <int D>
+__device__ __forceinline__ void dq_reduce(float* rows, int row_floats, const uint32_t (&r)[D / 64][32], int valid) {
+  const int lane = threadIdx.x & 31;
+  const bool odd = (lane & 1) != 0;
+  // four columns of one row per lane: lane pairs trade halves of two neighbouring 8-column blocks
+  auto four_columns = [&](int c, int k, int h, uint32_t (&v)[4]) {
+    const uint32_t a0 = r[c][4 * k + 2 * h], a1 = r[c][4 * k + 2 * h + 1];
+    const uint32_t b0 = r[c][4 * k + 4 + 2 * h], b1 = r[c][4 * k + 4 + 2 * h + 1];
+    const uint32_t x0 = __shfl_xor_sync(0xffffffffu, odd ? a0 : b0, 1);
+    const uint32_t x1 = __shfl_xor_sync(0xffffffffu, odd ? a1 : b1, 1);
+    v[0] = odd ? x0 : a0;
+    v[1] = odd ? x1 : a1;
+    v[2] = odd ? b0 : x0;
+    v[3] = odd ? b1 : x1;
+  };
+  const int col = (odd ? 8 : 0) + ((lane & 2) << 1);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int row = h * 8 + (lane >> 2);
+#pragma unroll
+    for (int c = 0; c < D / 64; ++c)
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        uint32_t v[4];
+        four_columns(c, k, h, v);
+        if (row < valid) red_add_v4(rows + row * row_floats + c * 64 + k * 8 + col, v);
+      }
+  }
+}
+
 // One swizzled shared-memory box into a 4-D tensor (TMA store; rows and columns past the tensor's
 // extent are dropped).
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src_smem, int c0, int c1, int c2,
@@ -219,8 +283,8 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_dk,
                const __grid_constant__ CUtensorMap tm_dv, const BwdParams p) {
-  using L = BwdSmem<D>;
-  constexpr int NS = SPLIT ? 1 : L::kQStages;
+  using L = std::conditional_t<SPLIT, BwdSplitSmem, BwdSmem<D>>;
+  constexpr int NS = L::kQStages;
   // SPLIT: head_dim is 2 * D; CTAs 2n and 2n+1 share key tile n and own columns [0, D) and [D, 2D).
   const int col_own = SPLIT ? static_cast<int>(blockIdx.x & 1) * D : 0;
   const int col_other = SPLIT ? D - col_own : 0;
@@ -239,7 +303,8 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   auto bar = [&](int i) { return bar0 + 8u * i; };
   constexpr int iKFull = 0, iVFull = 1, iQFull = 2, iQEmpty = 4, iStatFull = 6, iDoFull = 8, iDoEmpty = 9,
                 iSReady = 10, iDpReady = 11, iDqReady = 12, iDqFree = 13, iPReady = 14, iDsReady = 15,
-                iAllDone = 16, iDsFree = 17, iAFull = 18, iADone = 19;
+                iAllDone = 16, iDsFree = 17, iAFull = 18, iADone = 19,
+                iBFull = 20;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sgen + L::kMiscOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sgen + L::kMiscOff + 4);
   const WaitCtx wctx{abort_flag, p.status};
@@ -279,6 +344,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     mbar_init(bar(iDsFree), 1);
     mbar_init(bar(iAFull), 1);
     mbar_init(bar(iADone), 1);
+    mbar_init(bar(iBFull), 1);
     fence_mbar_init();
   }
   if (warp == 9) {
@@ -300,36 +366,43 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         tma_prefetch_desc(&tm_v);
         tma_prefetch_desc(&tm_do);
         tma_prefetch_desc(&tm_dq);
-        const uint32_t k_s = sbase + L::kKOff, v_s = sbase + L::kVOff, q_s = sbase + L::kQOff,
-                       do_s = sbase + L::kDoOff;
+        auto load_half = [&](uint32_t dst, const CUtensorMap* map, int b, int col, int row, int head) {
+          for (int bx = 0; bx < L::kBoxes; ++bx)
+            tma_load_4d(dst + bx * L::kBoxBytes, map, bar(b), col + bx * 64, row, head, wk.batch);
+        };
+        const int krow = wk.k_row0 + kv0;
+        const uint32_t x_s = sbase + L::kDsOff;
         for (int i = 0; i < n_iter; ++i) {
           const int head = wk.kv_head * group + i / nq;
           const int row = wk.q_row0 + (qt0 + i % nq) * kQTile;
-          const int krow = wk.k_row0 + kv0;
-          // every GEMM of the previous step has completed: all four tile buffers are free
+          // own dO: free once dV of the previous step has read it
+          if (i >= 1) mbar_wait(bar(iDoEmpty), (i - 1) & 1, wctx, kBbDoEmpty);
+          if (i >= 1) {
+            mbar_arrive_expect_tx(bar(iDoFull), L::kTileBytes);
+            load_half(sbase + L::kDoOff, &tm_do, iDoFull, col_own, row, head);
+          }
+          // X and own Q: free once the dQ tile of the previous step has left them
           if (i >= 1) mbar_wait(bar(iQEmpty), (i - 1) & 1, wctx, kBbQEmpty);
-          mbar_arrive_expect_tx(bar(iAFull), 4 * L::kTileBytes);
-          for (int bx = 0; bx < L::kBoxes; ++bx) {
-            const int x = col_other + bx * 64;
-            tma_load_4d(k_s + bx * L::kBoxBytes, &tm_k, bar(iAFull), x, krow, wk.kv_head, wk.batch);
-            tma_load_4d(q_s + bx * L::kBoxBytes, &tm_q, bar(iAFull), x, row, head, wk.batch);
-            tma_load_4d(v_s + bx * L::kBoxBytes, &tm_v, bar(iAFull), x, krow, wk.kv_head, wk.batch);
-            tma_load_4d(do_s + bx * L::kBoxBytes, &tm_do, bar(iAFull), x, row, head, wk.batch);
+          mbar_arrive_expect_tx(bar(iAFull), L::kTileBytes);
+          load_half(x_s, &tm_q, iAFull, col_other, row, head);
+          if (i == 0) {
+            mbar_arrive_expect_tx(bar(iKFull), 2 * L::kTileBytes);
+            load_half(sbase + L::kKOff + L::kTileBytes, &tm_k, iKFull, col_other, krow, wk.kv_head);
+            load_half(sbase + L::kKOff, &tm_k, iKFull, col_own, krow, wk.kv_head);
           }
-          // the partial S^T and dP^T have read them: this CTA's own columns go over them
+          mbar_arrive_expect_tx(bar(iQFull), L::kTileBytes);
+          load_half(sbase + L::kQOff, &tm_q, iQFull, col_own, row, head);
+          if (i == 0) {
+            mbar_arrive_expect_tx(bar(iVFull), 2 * L::kTileBytes);
+            load_half(sbase + L::kVOff + L::kTileBytes, &tm_v, iVFull, col_other, krow, wk.kv_head);
+            load_half(sbase + L::kVOff, &tm_v, iVFull, col_own, krow, wk.kv_head);
+            mbar_arrive_expect_tx(bar(iDoFull), L::kTileBytes);
+            load_half(sbase + L::kDoOff, &tm_do, iDoFull, col_own, row, head);
+          }
+          // the other half of dO follows Q's through X as soon as S^T has read that
           mbar_wait(bar(iADone), i & 1, wctx, kBbADone);
-          mbar_arrive_expect_tx(bar(iQFull), 2 * L::kTileBytes);
-          for (int bx = 0; bx < L::kBoxes; ++bx) {
-            const int x = col_own + bx * 64;
-            tma_load_4d(k_s + bx * L::kBoxBytes, &tm_k, bar(iQFull), x, krow, wk.kv_head, wk.batch);
-            tma_load_4d(q_s + bx * L::kBoxBytes, &tm_q, bar(iQFull), x, row, head, wk.batch);
-          }
-          mbar_arrive_expect_tx(bar(iDoFull), 2 * L::kTileBytes);
-          for (int bx = 0; bx < L::kBoxes; ++bx) {
-            const int x = col_own + bx * 64;
-            tma_load_4d(v_s + bx * L::kBoxBytes, &tm_v, bar(iDoFull), x, krow, wk.kv_head, wk.batch);
-            tma_load_4d(do_s + bx * L::kBoxBytes, &tm_do, bar(iDoFull), x, row, head, wk.batch);
-          }
+          mbar_arrive_expect_tx(bar(iBFull), L::kTileBytes);
+          load_half(x_s, &tm_do, iBFull, col_other, row, head);
         }
       }
       __syncwarp();
@@ -443,23 +516,25 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const int st1 = (i + 1) % NS;
         const uint32_t q_lo_mn = smem_desc_lo(sbase + L::kQOff + st * L::kTileBytes, L::kBoxBytes);
         if constexpr (SPLIT) {
-          // S^T(i) and dP^T(i) in two parts: the other column half first, then this CTA's own, which
-          // stays in the tile buffers for dV, dK and dQ.  S^T goes over P^T(i-1), which dV(i-1)
-          // -- issued before -- has read; dP^T goes over dQ(i-1), which the write-back warps must
-          // have read out.
+          // S^T(i) and dP^T(i) in two parts, the other column half (from X) first.  S^T goes over P^T(i-1),
+          // which dV(i-1) -- issued before -- has read; dP^T goes over dQ(i-1), which the write-back warps
+          // must have read out.
+          const uint32_t k_lo_other = smem_desc_lo(k_s + L::kTileBytes, 16);
+          const uint32_t v_lo_other = smem_desc_lo(v_s + L::kTileBytes, 16);
+          if (i == 0) mbar_wait(bar(iKFull), 0, wctx, kBbKFull);
           mbar_wait(bar(iAFull), i & 1, wctx, kBbAFull);
           tc_fence_after_sync();
-          issue_xyT(kColS, k_lo_k, sbase + L::kQOff);
-          if (i >= 1) {
-            mbar_wait(bar(iDqFree), (i - 1) & 1, wctx, kBbDqFree);
-            tc_fence_after_sync();
-          }
-          issue_xyT(kColDpq, v_lo_k, sbase + L::kDoOff);
+          issue_xyT(kColS, k_lo_other, sbase + L::kDsOff);
           tc_commit(bar(iADone));
           mbar_wait(bar(iQFull), i & 1, wctx, kBbQFull);
           tc_fence_after_sync();
           issue_xyT(kColS, k_lo_k, sbase + L::kQOff, true);
           tc_commit(bar(iSReady));
+          if (i == 0) mbar_wait(bar(iVFull), 0, wctx, kBbVFull);
+          else mbar_wait(bar(iDqFree), (i - 1) & 1, wctx, kBbDqFree);
+          mbar_wait(bar(iBFull), i & 1, wctx, kBbBFull);
+          tc_fence_after_sync();
+          issue_xyT(kColDpq, v_lo_other, sbase + L::kDsOff);
           mbar_wait(bar(iDoFull), i & 1, wctx, kBbDoFull);
           tc_fence_after_sync();
           issue_xyT(kColDpq, v_lo_k, sbase + L::kDoOff, true);
@@ -494,7 +569,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     smem_desc_join(q_lo_mn + ((ks * 2048) >> 4), kHi), idesc_dkv,
                     (i > 0 || ks > 0) ? 1u : 0u);
           }
-          tc_commit(bar(iQEmpty + st));  // Q(i) has no reader left once dK(i) is done
+          tc_commit(bar(iQEmpty + st));  // Q(i) (SPLIT: and X) has no reader left once dK(i) is done
         };
         // dQ(i) = dS(i) K: the dS^T buffer read as an M-contiguous A operand; the result (queries on
         // the lanes, head_dim on the columns) goes into the columns of the consumed dP^T(i)
@@ -720,46 +795,76 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // that add the boxes to the fp32 accumulator.  The second half is pulled into registers (and the
     // TMEM columns handed back to the issuer) before waiting for the first half's reductions.
     const int quarter = warp & 3;
-    const int qrow = quarter * 32 + lane;
-    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    const bool issuer = warp == 10 && lane == 0;
-    uint8_t* box_row = sgen + L::kStageOff + qrow * 128;
-    for (int i = 0; i < n_iter; ++i) {
-      const int head = wk.kv_head * group + i / nq;
-      const int qt = qt0 + i % nq;
-      mbar_wait(bar(iDqReady), i & 1, wctx, kBbDqReady);
-      tc_fence_after_sync();
-      const int grow = wk.q_row0 + qt * kQTile;  // accumulator row of the tile's first query
+    if constexpr (SPLIT) {
+      // At head_dim 256 there is no room for staging boxes.  The tile is read in the 16-lane x 8-column shape, in
+      // which four lanes hold 8 columns of a row, and added to the accumulator from registers.  (Where the
+      // boxes fit, TMA reductions from shared memory are faster: 1 410 against 1 518 us at head_dim 128 on
+      // 4 x 32 / 8 x 4 096 causal.)  Staging through X and the Q buffer instead, which then wait for the
+      // reductions to read them, took 360 us against 327.
+      for (int i = 0; i < n_iter; ++i) {
+        const int head = wk.kv_head * group + i / nq;
+        const int qt = qt0 + i % nq;
+        mbar_wait(bar(iDqReady), i & 1, wctx, kBbDqReady);
+        tc_fence_after_sync();
+        float* tile = p.dq_accum + wk.batch * p.dq_accum_batch_stride + head * p.dq_accum_head_stride +
+                      (static_cast<int64_t>(wk.q_row0) + qt * kQTile) * (2 * D) + col_own;
+        const int rows_here = wk.seqlen_q - qt * kQTile;  // rows behind the sequence are another's, or nobody's
 #pragma unroll
-      for (int hf = 0; hf < D / 64; ++hf) {
-        uint32_t r[2][32];
-        tmem_ld_32x32b_x32(tmem_base + lane_addr + kColDpq + hf * 64, r[0]);
-        tmem_ld_32x32b_x32(tmem_base + lane_addr + kColDpq + hf * 64 + 32, r[1]);
-        tmem_wait_ld();
-        if (hf == D / 64 - 1) {  // everything is in registers: the issuer may overwrite the columns
-          tc_fence_before_sync();
-          mbar_arrive(bar(iDqFree));
-        }
-        // Earlier reductions must be done reading the staging boxes.
-        if (issuer) bulk_wait_group_read<0>();
-        named_barrier_sync(1, 128);
+        for (int hr = 0; hr < 2; ++hr) {
+          uint32_t r[D / 64][32];
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int v = 0; v < 8; ++v)
-            *reinterpret_cast<uint4*>(box_row + c * L::kBoxBytes + ((v ^ (qrow & 7)) << 4)) =
-                make_uint4(r[c][4 * v + 0], r[c][4 * v + 1], r[c][4 * v + 2], r[c][4 * v + 3]);
-        fence_proxy_async_smem();
-        named_barrier_sync(1, 128);
-        if (issuer) {
-          tma_reduce_add_4d(&tm_dq, sbase + L::kStageOff, col_own + hf * 64, grow, head, wk.batch);
-          tma_reduce_add_4d(&tm_dq, sbase + L::kStageOff + L::kBoxBytes, col_own + hf * 64 + 32, grow, head,
-                            wk.batch);
-          bulk_commit_group();
+          for (int c = 0; c < D / 64; ++c)
+            tmem_ld_16x256b_x8(tmem_base + (static_cast<uint32_t>(quarter * 32 + hr * 16) << 16) + kColDpq + c * 64, r[c]);
+          tmem_wait_ld();
+          if (hr == 1) {  // everything is in registers: the issuer may overwrite the columns
+            tc_fence_before_sync();
+            mbar_arrive(bar(iDqFree));
+          }
+          const int row = quarter * 32 + hr * 16;
+          dq_reduce<D>(tile + static_cast<int64_t>(row) * (2 * D), 2 * D, r, rows_here - row);
         }
       }
+    } else {
+      const int qrow = quarter * 32 + lane;
+      const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+      const bool issuer = warp == 10 && lane == 0;
+      uint8_t* box_row = sgen + L::kStageOff + qrow * 128;
+      for (int i = 0; i < n_iter; ++i) {
+        const int head = wk.kv_head * group + i / nq;
+        const int qt = qt0 + i % nq;
+        mbar_wait(bar(iDqReady), i & 1, wctx, kBbDqReady);
+        tc_fence_after_sync();
+        const int grow = wk.q_row0 + qt * kQTile;  // accumulator row of the tile's first query
+#pragma unroll
+        for (int hf = 0; hf < D / 64; ++hf) {
+          uint32_t r[2][32];
+          tmem_ld_32x32b_x32(tmem_base + lane_addr + kColDpq + hf * 64, r[0]);
+          tmem_ld_32x32b_x32(tmem_base + lane_addr + kColDpq + hf * 64 + 32, r[1]);
+          tmem_wait_ld();
+          if (hf == D / 64 - 1) {  // everything is in registers: the issuer may overwrite the columns
+            tc_fence_before_sync();
+            mbar_arrive(bar(iDqFree));
+          }
+          // Earlier reductions must be done reading the staging boxes.
+          if (issuer) bulk_wait_group_read<0>();
+          named_barrier_sync(1, 128);
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int v = 0; v < 8; ++v)
+              *reinterpret_cast<uint4*>(box_row + c * L::kBoxBytes + ((v ^ (qrow & 7)) << 4)) =
+                  make_uint4(r[c][4 * v + 0], r[c][4 * v + 1], r[c][4 * v + 2], r[c][4 * v + 3]);
+          fence_proxy_async_smem();
+          named_barrier_sync(1, 128);
+          if (issuer) {
+            tma_reduce_add_4d(&tm_dq, sbase + L::kStageOff, hf * 64, grow, head, wk.batch);
+            tma_reduce_add_4d(&tm_dq, sbase + L::kStageOff + L::kBoxBytes, hf * 64 + 32, grow, head, wk.batch);
+            bulk_commit_group();
+          }
+        }
+      }
+      if (issuer) bulk_wait_group0();
     }
-    if (issuer) bulk_wait_group0();
   }
 
   tc_fence_before_sync();
@@ -855,14 +960,13 @@ cudaError_t launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
                          const CUtensorMap& tdo, const CUtensorMap& tdq, const CUtensorMap& tdk,
                          const CUtensorMap& tdv, const BwdParams& p, int grid, cudaStream_t stream) {
   auto kern = fal_bwd_kernel<D, CAUSAL, SPLIT>;
+  constexpr int kSmem = SPLIT ? BwdSplitSmem::kAllocBytes : BwdSmem<D>::kAllocBytes;
   static DeviceOnce configured;
-  cudaError_t e = configured.run([&] {
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                BwdSmem<D>::kAllocBytes);
-  });
+  cudaError_t e = configured.run(
+      [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem); });
   if (e != cudaSuccess) return e;
   if (SPLIT && grid > 0x3fffffff) return cudaErrorInvalidValue;
-  kern<<<SPLIT ? 2 * grid : grid, kBwdThreads, BwdSmem<D>::kAllocBytes, stream>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
+  kern<<<SPLIT ? 2 * grid : grid, kBwdThreads, kSmem, stream>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
   return cudaGetLastError();
 }
 
