@@ -82,10 +82,10 @@ int make_tensor_map(CUtensorMap* map, const void* base, int head_dim, int64_t ro
 }
 
 // fp32 dQ accumulator addressed as [batch, head, row, head_dim] through strides in floats (rows of
-// head_dim contiguous floats); box = 32 floats x 128 rows, 128-byte swizzle: the shape of one dQ
+// head_dim contiguous floats); box = 32 floats x box_rows, 128-byte swizzle: the shape of one dQ
 // staging box of the backward kernel.  `rows` is the extent reductions are clipped to.
 int make_accum_tensor_map(CUtensorMap* map, const float* base, int head_dim, int64_t rows, int64_t heads,
-                          int64_t batch, const fal::RowStrides& st) {
+                          int64_t batch, const fal::RowStrides& st, int box_rows) {
   EncodeTiledFn enc = get_encode_fn();
   if (enc == nullptr) return FAL_ERR_TENSOR_MAP;
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0) return FAL_ERR_INVALID_ARGUMENT;
@@ -97,7 +97,7 @@ int make_accum_tensor_map(CUtensorMap* map, const float* base, int head_dim, int
   const cuuint64_t strides[3] = {fix(st.row), fix(st.head), fix(st.batch)};
   for (int i = 0; i < 3; ++i)
     if (strides[i] % 16u != 0) return FAL_ERR_INVALID_ARGUMENT;
-  const cuuint32_t box[4] = {32u, 128u, 1u, 1u};
+  const cuuint32_t box[4] = {32u, static_cast<cuuint32_t>(box_rows), 1u, 1u};
   const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dims, strides, box,
                    estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -577,7 +577,7 @@ int run_bwd(const BwdCall& c) {
   if ((rc = make_tensor_map(&tdo, c.d_out, c.head_dim, c.rows_q, c.heads_q, c.batch, c.s_do, 128)))
     return rc;
   if ((rc = make_accum_tensor_map(&tdq, dq_accum, kdim, acc_rows, c.heads_q, c.batch,
-                                  fal::RowStrides{acc_batch, acc_head, kdim})))
+                                  fal::RowStrides{acc_batch, acc_head, kdim}, fal::bwd_dq_box_rows(kdim))))
     return rc;
   if ((rc = make_tensor_map(&tk, c.k, c.head_dim, c.rows_k, c.heads_kv, c.batch, c.s_k, 128))) return rc;
   if ((rc = make_tensor_map(&tv, c.v, c.head_dim, c.rows_k, c.heads_kv, c.batch, c.s_v, 128))) return rc;

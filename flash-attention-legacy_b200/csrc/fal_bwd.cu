@@ -59,6 +59,7 @@ constexpr int kBwdThreads = 512;
 constexpr int kKvTile = 128;
 constexpr int kQTile = 128;
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr int kDqBoxBytes = 32 * 128;  // one dQ staging box: 32 rows of 32 fp32 columns
 
 enum BwdBarrier : int {
   kBbKFull = 100, kBbVFull = 101, kBbQFull = 110, kBbDoFull = 120, kBbStatFull = 130,
@@ -79,8 +80,10 @@ struct BwdSmem {
   static constexpr int kDoOff = kQOff + kQStages * kTileBytes;  // single stage
   static constexpr int kDsOff = kDoOff + kTileBytes;            // [2 boxes][128 keys][64 queries] fp16
   static constexpr int kDsBytes = 2 * kBoxBytes;
-  static constexpr int kStageOff = kDsOff + kDsBytes;           // dQ staging: 2 x [128 rows][32 fp32]
+  static constexpr int kStageOff = kDsOff + kDsBytes;           // dQ staging: 2 x [128 rows][32 fp32], or per warp 2 x [32][32]
+  static constexpr bool kWarpDq = D == 128;                     // the write-back warps work independently
   static constexpr int kStageBytes = 2 * kBoxBytes;
+  static_assert(kStageBytes == 4 * 2 * kDqBoxBytes, "staging");
   static constexpr int kStatOff = kStageOff + kStageBytes;      // per Q stage: lse2[128], delta[128]
   static constexpr int kStatBytes = kQStages * 2 * kQTile * 4;
   static constexpr int kBarOff = kStatOff + kStatBytes;
@@ -789,11 +792,6 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     }
   } else if (warp < 14) {
     // ===================== dQ write-back ======================================
-    // dQ tile: TMEM lane = query row, column = head_dim.  It leaves in 64-column halves.  For each
-    // half a thread reads its row's 64 values, writes them as two 32-float slices into the two
-    // swizzled [128 rows][128 bytes] staging boxes, and one thread issues two TMA tensor reductions
-    // that add the boxes to the fp32 accumulator.  The second half is pulled into registers (and the
-    // TMEM columns handed back to the issuer) before waiting for the first half's reductions.
     const int quarter = warp & 3;
     if constexpr (SPLIT) {
       // At head_dim 256 there is no room for staging boxes.  The tile is read in the 16-lane x 8-column shape, in
@@ -824,7 +822,64 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           dq_reduce<D>(tile + static_cast<int64_t>(row) * (2 * D), 2 * D, r, rows_here - row);
         }
       }
+    } else if constexpr (L::kWarpDq) {
+      // dQ tile: TMEM lane = query row, column = head_dim.  Every warp takes its 32 rows by itself, 32 columns at a
+      // time: a row per thread into one of its two swizzled [32 rows][128 bytes] boxes, which its first lane
+      // hands to the TMA unit as an fp32 reduction while the other box fills.  Three column groups are in
+      // registers before the first is staged, so that the TMEM columns go back to the issuer as soon as that
+      // one has left its registers to the fourth.  The four warps in step instead, 64 columns at a time through two
+      // boxes of 128 rows, wrote for 4 490 of a step's 5 170 cycles, 2 290 of them waiting for the boxes to be
+      // read (an SM sends out 25 bytes of reductions a clock), and the next dP^T waited 1 120 for the columns:
+      // 4 x 32 / 8 x 4 096 causal 1 438 -> 1 293 us, 4 x 16 x 2 048 374 -> 317, 1 x 32 / 8 x 2 987 causal 297 -> 240.
+      const uint32_t t_dq = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + kColDpq;
+      const uint32_t box_off = L::kStageOff + quarter * 2 * kDqBoxBytes;
+      uint8_t* box_row = sgen + box_off + lane * 128;
+      for (int i = 0; i < n_iter; ++i) {
+        const int head = wk.kv_head * group + i / nq;
+        const int q_row = (qt0 + i % nq) * kQTile + quarter * 32;  // local index of the warp's first query
+        const int grow = wk.q_row0 + q_row;                        // its accumulator row
+        mbar_wait(bar(iDqReady), i & 1, wctx, kBbDqReady);
+        tc_fence_after_sync();
+        if (q_row >= wk.seqlen_q) {  // no query of the sequence among the warp's rows
+          mbar_arrive(bar(iDqFree));
+          continue;
+        }
+        constexpr int kGroups = D / 32, kAhead = 3;
+        static_assert(kGroups == kAhead + 1, "one column group is fetched late");
+        uint32_t r[kAhead][32];
+#pragma unroll
+        for (int c = 0; c < kAhead; ++c) tmem_ld_32x32b_x32(t_dq + c * 32, r[c]);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < kGroups; ++c) {
+          const uint32_t box = (c & 1) * kDqBoxBytes;
+          if (lane == 0) bulk_wait_group_read<1>();  // the box's last reduction has read it
+          __syncwarp();
+#pragma unroll
+          for (int v = 0; v < 8; ++v)
+            *reinterpret_cast<uint4*>(box_row + box + ((v ^ (lane & 7)) << 4)) =
+                make_uint4(r[c % kAhead][4 * v + 0], r[c % kAhead][4 * v + 1], r[c % kAhead][4 * v + 2],
+                           r[c % kAhead][4 * v + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_reduce_add_4d(&tm_dq, sbase + box_off + box, c * 32, grow, head, wk.batch);
+            bulk_commit_group();
+          }
+          if (c == 0) {  // everything is in registers then: the issuer may overwrite the columns
+            tmem_ld_32x32b_x32(t_dq + kAhead * 32, r[0]);
+            tmem_wait_ld();
+            tc_fence_before_sync();
+            mbar_arrive(bar(iDqFree));
+          }
+        }
+      }
+      if (lane == 0) bulk_wait_group0();
     } else {
+      // head_dim 64: the tile is 64 columns wide and leaves at once, a row per thread into the two swizzled
+      // [128 rows][32 floats] boxes, by two reductions.  (By warps as above 235 -> 254 us on 4 x 16 x 2 048: here
+      // the write-back warps are not what a step waits for, and eight small reductions take more of the TMA
+      // unit's and the issue slots' time than two.)
       const int qrow = quarter * 32 + lane;
       const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
       const bool issuer = warp == 10 && lane == 0;

@@ -83,7 +83,9 @@ struct BwdPrepParams {
 cudaError_t launch_bwd_prep(const BwdPrepParams& p, cudaStream_t stream);
 
 // Backward main kernel: grid = number of (128-key block, batch*kv_head) units.
-// tdq: fp32 tensor map of the dQ accumulator (head_dim, padded rows, heads, batch), 32 x 128 boxes.
+// tdq: fp32 tensor map of the dQ accumulator (head_dim, padded rows, heads, batch), boxes of 32 floats x
+// bwd_dq_box_rows.
+constexpr int bwd_dq_box_rows(int kernel_head_dim) { return kernel_head_dim == 128 ? 32 : 128; }
 cudaError_t launch_bwd(int head_dim, bool causal, const CUtensorMap& tq, const CUtensorMap& tk,
                        const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq,
                        const CUtensorMap& tdk, const CUtensorMap& tdv, const BwdParams& p, int grid,
