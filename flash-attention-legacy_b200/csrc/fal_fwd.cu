@@ -211,6 +211,7 @@ __device__ __forceinline__ void fwd_heaviest_block(const FwdParams& p, int slot,
 
 // Maps blockIdx.x to a unit of work.  Returns false when the block has none
 // (packed mode launches an upper bound of blocks).
+template <bool SHIFTED>
 __device__ __forceinline__ bool fwd_decode_work(const FwdParams& p, int cta_rows, FwdWork& w) {
   const int idx = blockIdx.x;
   if (p.cu_q == nullptr) {
@@ -220,7 +221,7 @@ __device__ __forceinline__ bool fwd_decode_work(const FwdParams& p, int cta_rows
     const int bh = idx % bh_count;
     w.batch = bh / p.heads_q;
     w.head = bh % p.heads_q;
-    if (p.seqused_k != nullptr && p.shift_per_sequence != 0 && p.batch > 1) {
+    if (SHIFTED && p.seqused_k != nullptr && p.shift_per_sequence != 0 && p.batch > 1) {
       // Entries of 1 500 and of 8 000 keys in one grid: in the order above the longest entry's last blocks
       // start late and the SMs wait for them.  Heaviest first, 4 entries x 1 024 queries (32 / 8 heads of 128)
       // behind 512 to 7 000 keys: 329 -> 310 us a call; the search costs a CTA well under a microsecond.
@@ -303,10 +304,13 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   using L = FwdSmem<D, SHAPE>;
   constexpr int NS = L::kStages;
   constexpr int kSmWarps = L::kSmWarps;
+  // Instances that a chunk behind a cache does not run carry no code for it: with it the two-tile kernel at
+  // head_dim 64 spilled more in its main loop (16 heads x 16 384 causal 755 -> 791 us).
+  constexpr bool kMaySplit = SHAPE == kOneTile && (SHIFTED || !CAUSAL);
 
   FwdWork wk;
   constexpr int kCtaRows = L::kCtaRows;
-  if (!fwd_decode_work(p, kCtaRows, wk)) return;
+  if (!fwd_decode_work<SHIFTED>(p, kCtaRows, wk)) return;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -331,7 +335,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                              : 0;
   // Several CTAs share this block's keys: this one takes its range of the entry's key tiles, as a shorter key
   // sequence with the diagonal moved along.
-  if (p.kv_splits > 1) {
+  if (kMaySplit && p.kv_splits > 1) {
     const int tiles = (wk.seqlen_k + kTileN - 1) / kTileN;
     const int per = (tiles + p.kv_splits - 1) / p.kv_splits;
     const int key0 = min(static_cast<int>(blockIdx.y) * per, tiles) * kTileN;
@@ -796,7 +800,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const bool tile_used = (kAlt || wg < L::kQTiles) && q_tile0 < wk.seqlen_q;
     // (Not at head_dim 256: measured 5 - 10 % slower there -- the CTA then waits for the TMA unit to read
     // 64 KB of staging before it can exit, where plain stores drain behind its back.)
-    const bool by_tma = D != 256 && p.store_by_tma != 0 && p.kv_splits <= 1 && tile_used &&
+    const bool by_tma = D != 256 && p.store_by_tma != 0 && !(kMaySplit && p.kv_splits > 1) && tile_used &&
                         (p.cu_q == nullptr || q_tile0 + kTileM <= wk.seqlen_q);
     const int64_t part_row =
         ((static_cast<int64_t>(blockIdx.y) * p.batch + wk.batch) * p.heads_q + wk.head) * p.seqlen_q + q_local;
@@ -823,7 +827,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           // box c / 2, 16-byte chunk (c % 2) * 4 + v of the row, 128-byte XOR swizzle
           *reinterpret_cast<uint4*>(stage_row + (c >> 1) * L::kBoxBytes + ((((c & 1) * 4 + v) ^ (row & 7)) << 4)) = out;
         }
-      } else if (row_ok && p.kv_splits > 1) {
+      } else if (kMaySplit && row_ok && p.kv_splits > 1) {
         float* part = p.part_o + part_row * p.head_dim + c * 32;
         if (c * 32 < p.head_dim) {
 #pragma unroll
@@ -848,7 +852,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     if (row_ok && (!kAlt || wg == 0)) {
       const float lse = (nt > 0 && m_ref != kNegInf) ? m_ref * p.scale + logf(fmaxf(l, 1e-20f))
                                                       : kNegInf;
-      if (p.kv_splits > 1) p.part_lse[part_row] = lse;
+      if (kMaySplit && p.kv_splits > 1) p.part_lse[part_row] = lse;
       else p.lse[wk.lse_base + static_cast<int64_t>(q_local) * p.lse_strides.row] = lse;
     }
     if (by_tma) {  // the same for every thread that wrote into the tile's staging buffer
