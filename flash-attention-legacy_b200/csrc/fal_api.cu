@@ -386,7 +386,9 @@ int fwd_batched(const void* q, const void* k, const void* v, void* o, float* lse
   int variant = forward_variant(kdim, (seqlen_q + 255) / 256, static_cast<int64_t>(batch) * heads_q,
                                 is_causal == 1 ? seqlen_k / 2 : seqlen_k);
   p.kv_splits = 1;
-  if (seqused_k != nullptr && workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) {
+  // (the kernel instances of the top-left mask carry no code for a share of the keys)
+  if (seqused_k != nullptr && is_causal != FAL_CAUSAL_TOP_LEFT && workspace != nullptr &&
+      (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) {
     const int64_t blocks = static_cast<int64_t>((seqlen_q + 127) / 128) * batch * heads_q;
     const int splits = chunk_kv_splits(blocks, seqlen_k);
     if (splits > 1 && workspace_bytes >= chunk_split_bytes(splits, batch, heads_q, seqlen_q, head_dim)) {

@@ -310,7 +310,7 @@ FAL_API int fal_fwd_args_run(const fal_fwd_args* args);
  * fal_fwd_kvcache for a chunk too small to fill the GPU: with a workspace of at least
  * fal_fwd_kvcache_workspace_bytes (0: nothing to gain; 16-byte aligned, not shared by calls that overlap on the GPU)
  * the keys of a query block are dealt to several thread blocks and their results merged by a second kernel.
- * A smaller or null workspace gives fal_fwd_kvcache.
+ * A smaller or null workspace, and the top-left mask (is_causal 1), give fal_fwd_kvcache.
  */
 FAL_API size_t fal_fwd_kvcache_workspace_bytes(int batch, int heads_q, int seqlen_q, int cache_capacity, int head_dim);
 FAL_API int fal_fwd_kvcache_split_run(const fal_fwd_args* args, void* workspace, size_t workspace_bytes);

@@ -40,3 +40,39 @@ def test_split_chunk_against_the_oracle(ext, hq, hkv, d, nq, lens, capacity, cau
     assert torch.isneginf(lse.cpu()[~seen]).all() and not o.cpu()[~seen].any()
     assert (wide[..., d:] == 7.0).all()
     assert ext.device_status() == 0
+
+
+def _call(ext, q, kc, vc, lens, mask, workspace=None):
+    """fal_fwd_kvcache, or the split call with a workspace; returns (O, LSE)."""
+    (b, hq, nq, d), (hkv, capacity) = q.shape, kc.shape[1:3]
+    o, lse = torch.full_like(q, 5.0), torch.full((b, hq, nq), 5.0, device="cuda")
+    args = ext._FWD_ARGS.pack(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), o.data_ptr(), lse.data_ptr(), lens.data_ptr(),
+                              b, hq, hkv, nq, capacity, d, *q.stride()[:3], *kc.stride()[:3], *vc.stride()[:3],
+                              *o.stride()[:3], 1 / math.sqrt(d), mask, ext._status_ptr(0), ext._raw_stream(0))
+    if workspace is None:
+        ext._check(ext._fwd_run(args))
+    else:
+        ext._check(ext._lib.fal_fwd_kvcache_split_run(args, workspace.data_ptr(), workspace.numel() * 4))
+    assert ext.device_status() == 0
+    return o.cpu(), lse.cpu()
+
+
+def _inputs(ext, hq, hkv, d, nq, lens, capacity):
+    """Inputs of a chunk that is split, and a workspace full of NaN."""
+    gen = torch.Generator().manual_seed(d + nq)
+    b = len(lens)
+    q = torch.randn(b, hq, nq, d, generator=gen).half().cuda()
+    kc, vc = (torch.randn(b, hkv, capacity, d, generator=gen).half().cuda() for _ in range(2))
+    nbytes = ext._lib.fal_fwd_kvcache_workspace_bytes(b, hq, nq, capacity, d)
+    assert nbytes > 0
+    return q, kc, vc, torch.tensor(lens, dtype=torch.int32).cuda(), torch.full((nbytes // 4,), math.nan, device="cuda")
+
+
+@pytest.mark.parametrize("mask", [0, 1, 2])
+@pytest.mark.parametrize("d", [64, 96, 128, 256])
+def test_the_split_call_takes_every_mask(ext, mask, d):
+    q, kc, vc, lens, ws = _inputs(ext, 4, 2, d, 200, [1500, 333], 1500)
+    o, lse = _call(ext, q, kc, vc, lens, mask, ws)
+    o_whole, lse_whole = _call(ext, q, kc, vc, lens, mask)
+    assert orc.rel_max_err(o, o_whole) <= orc.TOL_O
+    assert orc.abs_max_err(lse, lse_whole) <= orc.TOL_LSE
