@@ -209,6 +209,11 @@ __device__ __forceinline__ void fwd_heaviest_block(const FwdParams& p, int slot,
   }
 }
 
+// Key tiles of a sequence of `keys` keys that one of `splits` CTAs takes.
+__device__ __forceinline__ int fwd_split_tiles(int keys, int splits) {
+  return ((keys + kTileN - 1) / kTileN + splits - 1) / splits;
+}
+
 // Maps blockIdx.x to a unit of work.  Returns false when the block has none
 // (packed mode launches an upper bound of blocks).
 template <bool SHIFTED>
@@ -334,12 +339,15 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                                                                               : p.causal_shift)
                              : 0;
   // Several CTAs share this block's keys: this one takes its range of the entry's key tiles, as a shorter key
-  // sequence with the diagonal moved along.
+  // sequence with the diagonal moved along.  A range that no row of the block sees is left alone: the merge knows
+  // that it has no part in them.  (Visited for its hidden scores, an infinity among its values would reach rows
+  // that cannot see it.)
   if (kMaySplit && p.kv_splits > 1) {
-    const int tiles = (wk.seqlen_k + kTileN - 1) / kTileN;
-    const int per = (tiles + p.kv_splits - 1) / p.kv_splits;
-    const int key0 = min(static_cast<int>(blockIdx.y) * per, tiles) * kTileN;
-    wk.seqlen_k = max(min(wk.seqlen_k - key0, per * kTileN), 0);
+    const int per = fwd_split_tiles(wk.seqlen_k, p.kv_splits);
+    const int key0 = static_cast<int>(blockIdx.y) * per * kTileN;
+    const int seen = SHIFTED ? min(wk.seqlen_k, (wk.qblk + 1) * kTileM + cshift) : wk.seqlen_k;
+    if (key0 >= seen) return;
+    wk.seqlen_k = min(wk.seqlen_k - key0, per * kTileN);
     wk.k_row0 += key0;
     if (SHIFTED) cshift -= key0;
   }
@@ -880,13 +888,22 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 }
 
 // Merges the splits of a query block's keys: a warp per (batch, head, row), split s on lane s for the weights,
-// 16 bytes of every split's row per lane for the sum.  Bound by the partials' traffic, at most 128 rows per SM.
+// 16 bytes of every split's row per lane for the sum.  Only the splits with keys that the row sees are read: the
+// others have nothing to add, and what they hold may be another row's infinity (or memory nobody wrote).
+// Bound by the partials' traffic, at most 128 rows per SM.
 __global__ void __launch_bounds__(128) fal_fwd_combine_kernel(const FwdParams p) {
   const int lane = threadIdx.x & 31;
+  const int row = static_cast<int>(blockIdx.x) * 4 + (threadIdx.x >> 5);
+  if (row >= p.seqlen_q) return;
+  const int head = blockIdx.y;
+  const int64_t b = blockIdx.z;
   const int64_t rows = static_cast<int64_t>(p.batch) * p.heads_q * p.seqlen_q;
-  const int64_t id = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
-  if (id >= rows) return;
-  const float l = lane < p.kv_splits ? p.part_lse[lane * rows + id] : kNegInf;
+  const int64_t id = (b * p.heads_q + head) * p.seqlen_q + row;
+  const int keys = max(min(__ldg(p.seqused_k + b), p.seqlen_k), 0);
+  const int seen = p.shift_per_sequence != 0 ? row + 1 + keys - p.seqlen_q : keys;
+  const int split_keys = fwd_split_tiles(keys, p.kv_splits) * kTileN;
+  const int splits = seen > 0 ? (seen + split_keys - 1) / split_keys : 0;
+  const float l = lane < splits ? p.part_lse[lane * rows + id] : kNegInf;
   float m = l;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
@@ -896,16 +913,12 @@ __global__ void __launch_bounds__(128) fal_fwd_combine_kernel(const FwdParams p)
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
   w *= sum > 0.f ? 1.f / sum : 0.f;
-  const int row = static_cast<int>(id % p.seqlen_q);
-  const int64_t bh = id / p.seqlen_q;
-  const int head = static_cast<int>(bh % p.heads_q);
-  const int64_t b = bh / p.heads_q;
   __half* o = static_cast<__half*>(p.o) + b * p.o_strides.batch + head * p.o_strides.head +
               static_cast<int64_t>(row) * p.o_strides.row;
   for (int base = 0; base < p.head_dim; base += 128) {
     const int c = base + lane * 4;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < p.kv_splits; ++s) {
+    for (int s = 0; s < splits; ++s) {
       const float ws = __shfl_sync(0xffffffffu, w, s);
       if (c < p.head_dim) {
         const float4 x = *reinterpret_cast<const float4*>(p.part_o + (s * rows + id) * p.head_dim + c);
@@ -922,7 +935,8 @@ __global__ void __launch_bounds__(128) fal_fwd_combine_kernel(const FwdParams p)
       *reinterpret_cast<uint2*>(o + c) = out;
     }
   }
-  if (lane == 0) p.lse[b * p.lse_strides.batch + head * p.lse_strides.head + row] = sum > 0.f ? m + logf(sum) : kNegInf;
+  if (lane == 0)
+    p.lse[b * p.lse_strides.batch + head * p.lse_strides.head + row] = m == kNegInf ? kNegInf : m + logf(fmaxf(sum, 1e-20f));
 }
 
 template <int D, bool CAUSAL, bool SHIFTED, int SHAPE>
@@ -951,8 +965,8 @@ cudaError_t launch_fwd_d(bool causal, const CUtensorMap& tq, const CUtensorMap& 
 }  // namespace
 
 cudaError_t launch_fwd_combine(const FwdParams& p, cudaStream_t stream) {
-  const int64_t rows = static_cast<int64_t>(p.batch) * p.heads_q * p.seqlen_q;
-  fal_fwd_combine_kernel<<<static_cast<unsigned>((rows + 3) / 4), 128, 0, stream>>>(p);
+  // (heads and entries fit the grid's y and z: a chunk of more than half as many blocks as SMs is not split)
+  fal_fwd_combine_kernel<<<dim3((p.seqlen_q + 3) / 4, p.heads_q, p.batch), 128, 0, stream>>>(p);
   return cudaGetLastError();
 }
 

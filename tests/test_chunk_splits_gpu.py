@@ -76,3 +76,25 @@ def test_the_split_call_takes_every_mask(ext, mask, d):
     o_whole, lse_whole = _call(ext, q, kc, vc, lens, mask)
     assert orc.rel_max_err(o, o_whole) <= orc.TOL_O
     assert orc.abs_max_err(lse, lse_whole) <= orc.TOL_LSE
+
+
+@pytest.mark.parametrize("where,value", [("v", math.inf), ("v", math.nan), ("k", math.inf), ("k", math.nan)])
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("hq,nq,keys,at", [(8, 512, 600, 300), (8, 512, 600, 599), (2, 130, 3000, 2990), (4, 300, 200, 150)])
+def test_what_a_row_cannot_see_does_not_reach_it(ext, where, value, d, hq, nq, keys, at):
+    """An infinity or NaN in one key or value row: in the split chunk it reaches every row that sees the key and no
+    row that it does not reach in the unsplit one (whose blocks read whole key tiles)."""
+    q, kc, vc, lens, ws = _inputs(ext, hq, hq, d, nq, [keys], 700 if keys < 700 else keys)
+    (kc if where == "k" else vc)[0, :, at] = value
+    o, lse = _call(ext, q, kc, vc, lens, 2, ws)
+    o_whole, lse_whole = _call(ext, q, kc, vc, lens, 2)
+    sees = torch.arange(nq) + keys - nq >= at
+    reached, reached_whole = ~torch.isfinite(o).all(-1), ~torch.isfinite(o_whole).all(-1)
+    assert torch.equal(reached[..., sees], reached_whole[..., sees]) and not (reached & ~reached_whole).any()
+    clean = ~reached_whole
+    seen = clean & torch.isfinite(lse_whole)
+    if seen.any():
+        assert orc.rel_max_err(o[clean], o_whole[clean]) <= orc.TOL_O
+        assert orc.abs_max_err(lse[seen], lse_whole[seen]) <= orc.TOL_LSE
+    if where == "v":   # scores and their sums are as without it
+        assert torch.equal(torch.isfinite(lse), torch.isfinite(lse_whole))
