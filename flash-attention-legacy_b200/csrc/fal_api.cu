@@ -386,8 +386,10 @@ int fwd_batched(const void* q, const void* k, const void* v, void* o, float* lse
   int variant = forward_variant(kdim, (seqlen_q + 255) / 256, static_cast<int64_t>(batch) * heads_q,
                                 is_causal == 1 ? seqlen_k / 2 : seqlen_k);
   p.kv_splits = 1;
-  // (the kernel instances of the top-left mask carry no code for a share of the keys)
+  // (the kernel instances of the top-left mask carry no code for a share of the keys; a variant forced by
+  // fal_set_fwd_variant runs as it was asked for)
   if (seqused_k != nullptr && is_causal != FAL_CAUSAL_TOP_LEFT && workspace != nullptr &&
+      g_fwd_variant.load(std::memory_order_relaxed) == FAL_FWD_AUTO &&
       (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) {
     const int64_t blocks = static_cast<int64_t>((seqlen_q + 127) / 128) * batch * heads_q;
     const int splits = chunk_kv_splits(blocks, seqlen_k);

@@ -310,7 +310,8 @@ FAL_API int fal_fwd_args_run(const fal_fwd_args* args);
  * fal_fwd_kvcache for a chunk too small to fill the GPU: with a workspace of at least
  * fal_fwd_kvcache_workspace_bytes (0: nothing to gain; 16-byte aligned, not shared by calls that overlap on the GPU)
  * the keys of a query block are dealt to several thread blocks and their results merged by a second kernel.
- * A smaller or null workspace, and the top-left mask (is_causal 1), give fal_fwd_kvcache.
+ * A smaller or null workspace, the top-left mask (is_causal 1) and a variant forced by fal_set_fwd_variant give
+ * fal_fwd_kvcache.
  */
 FAL_API size_t fal_fwd_kvcache_workspace_bytes(int batch, int heads_q, int seqlen_q, int cache_capacity, int head_dim);
 FAL_API int fal_fwd_kvcache_split_run(const fal_fwd_args* args, void* workspace, size_t workspace_bytes);
@@ -415,7 +416,7 @@ FAL_API int fal_selftest_wait_timeout(int barrier_id, int* status, int* waits_gi
  * its benchmarks time whole operator calls (benchmarks/benchmark.py:36-49).
  */
 enum fal_kernel_kind {
-  FAL_KERNEL_FWD = 0,          /* forward main kernel */
+  FAL_KERNEL_FWD = 0,          /* forward main kernel (without the merge of a split chunk) */
   FAL_KERNEL_BWD = 1,          /* backward dK/dV/dQ kernel (without pre/post passes) */
   FAL_KERNEL_DECODE_SPLITK = 2 /* decode streaming pass incl. the append (without the combine) */
 };

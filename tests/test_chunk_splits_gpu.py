@@ -98,3 +98,16 @@ def test_what_a_row_cannot_see_does_not_reach_it(ext, where, value, d, hq, nq, k
         assert orc.abs_max_err(lse[seen], lse_whole[seen]) <= orc.TOL_LSE
     if where == "v":   # scores and their sums are as without it
         assert torch.equal(torch.isfinite(lse), torch.isfinite(lse_whole))
+
+
+@pytest.mark.parametrize("variant", ["FWD_ONE_TILE", "FWD_TWO_TILES", "FWD_HALF_SM"])
+def test_a_forced_variant_is_not_split(ext, variant):
+    q, kc, vc, lens, ws = _inputs(ext, 4, 2, 64, 200, [1500, 333], 1500)
+    ext.set_forward_variant(getattr(ext, variant))
+    try:
+        o, lse = _call(ext, q, kc, vc, lens, 2, ws)
+        o_whole, lse_whole = _call(ext, q, kc, vc, lens, 2)
+    finally:
+        ext.set_forward_variant(ext.FWD_AUTO)
+    assert torch.equal(o, o_whole) and torch.equal(lse, lse_whole)
+    assert torch.isnan(ws).all()   # nobody wrote a partial result
