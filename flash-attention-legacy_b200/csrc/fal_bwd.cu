@@ -208,11 +208,6 @@ __device__ __forceinline__ float bwd_exp2(int j, float x) {
   return (((j + K) & 7) < FAL_BWD_EXP_EMU_PER8) ? exp2_fma(x) : fast_exp2(x);
 }
 
-// dQ(i) issued before dK(i) (1): the write-back warps drain dQ out of TMEM -- which the next
-// step's dP^T needs gone -- while dK still runs.  0: dK first.
-#ifndef FAL_BWD_DQ_FIRST
-#define FAL_BWD_DQ_FIRST 1
-#endif
 // One elected lane per compute warp arrives on p_ready / ds_ready (1) or every thread (0).
 #ifndef FAL_BWD_ELECT_ARRIVE
 #define FAL_BWD_ELECT_ARRIVE 1
@@ -572,7 +567,9 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     smem_desc_join(q_lo_mn + ((ks * 2048) >> 4), kHi), idesc_dkv,
                     (i > 0 || ks > 0) ? 1u : 0u);
           }
-          tc_commit(bar(iQEmpty + st));  // Q(i) (SPLIT: and X) has no reader left once dK(i) is done
+          // Q(i) has no reader left once dK(i) is done.  (SPLIT: nor has X, which holds dS^T(i): a commit
+          // covers everything issued before it, so dQ(i), its other reader, must have been.)
+          tc_commit(bar(iQEmpty + st));
         };
         // dQ(i) = dS(i) K: the dS^T buffer read as an M-contiguous A operand; the result (queries on
         // the lanes, head_dim on the columns) goes into the columns of the consumed dP^T(i)
@@ -584,13 +581,10 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           }
           tc_commit(bar(iDqReady));
         };
-#if FAL_BWD_DQ_FIRST
+        // dQ first: the write-back warps drain it out of TMEM -- which the next step's dP^T needs gone --
+        // while dK still runs; and see the commit in issue_dk.
         issue_dq();
         issue_dk();
-#else
-        issue_dk();
-        issue_dq();
-#endif
         tc_commit(bar(iDsFree));  // both readers of the dS^T buffer are done
         // dP^T(i+1) goes where dQ(i) is: the write-back warps must have read it out first.
         if (!SPLIT && i + 1 < n_iter) {
