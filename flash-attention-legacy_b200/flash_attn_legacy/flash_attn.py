@@ -291,8 +291,11 @@ def flash_attn_with_kvcache(
         assert v is not None and k.shape == v.shape and k.shape[:2] == (b, lq), "k, v must be [B, L_q, H_kv, d]"
         # rows lens[b] ... lens[b] + Lq - 1 of every entry
         kd, vd = (k_cache, v_cache) if cache_layout == "bshd" else (k_cache.transpose(1, 2), v_cache.transpose(1, 2))
+        # what autograd has a say in (gradients; a cache made in inference mode, which it refuses to have written
+        # outside of it) goes through indexing
         tracked = torch.is_grad_enabled() and any(t.requires_grad for t in (k, v, k_cache, v_cache))
-        appended = None if tracked else flash_attn_legacy_cuda.cache_append(k, v, kd, vd, lens)
+        frozen = not torch.is_inference_mode_enabled() and (k_cache.is_inference() or v_cache.is_inference())
+        appended = None if tracked or frozen else flash_attn_legacy_cuda.cache_append(k, v, kd, vd, lens)
         if appended is not None:
             lens, fits = appended
             torch._assert_async(fits)  # an entry without room for the chunk

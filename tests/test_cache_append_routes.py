@@ -1,0 +1,40 @@
+"""Which chunks of new tokens may be written by the append kernel, and which autograd has a say in."""
+import pytest
+import torch
+
+import flash_attn_legacy_cuda as ext
+from flash_attn_legacy import flash_attn_with_kvcache
+
+
+@pytest.fixture()
+def appended(monkeypatch):
+    """Stands in for the append kernel and lists its calls (the attention behind it then refuses CPU tensors)."""
+    calls = []
+
+    def fake(k, v, k_cache, v_cache, lens):
+        calls.append((k, v))
+        return lens + k.shape[1], torch.ones(1, dtype=torch.bool)
+
+    monkeypatch.setattr(ext, "cache_append", fake)
+    return calls
+
+
+def _tensors():
+    gen = torch.Generator().manual_seed(1)
+    q, k, v = (torch.randn(2, 3, 4, 64, generator=gen).half() for _ in range(3))
+    kc, vc = (torch.zeros(2, 16, 4, 64, dtype=torch.float16) for _ in range(2))
+    return q, kc, vc, k, v, torch.tensor([2, 5], dtype=torch.int32)
+
+
+@pytest.mark.parametrize("which", [0, 1])
+def test_a_cache_made_in_inference_mode_is_not_written_outside_of_it(appended, which):
+    q, kc, vc, k, v, lens = _tensors()
+    caches = [kc, vc]
+    with torch.inference_mode():
+        caches[which] = caches[which].clone()
+    with pytest.raises(RuntimeError, match="[Ii]nference"):
+        flash_attn_with_kvcache(q, *caches, k=k, v=v, cache_seqlens=lens)
+    assert not appended
+    with torch.inference_mode(), pytest.raises(RuntimeError, match="CUDA"):
+        flash_attn_with_kvcache(q, *caches, k=k, v=v, cache_seqlens=lens)
+    assert len(appended) == 1
