@@ -15,6 +15,7 @@ from typing import Optional
 import torch
 import torch.nn as nn
 from torch.autograd import Function
+from torch.autograd.forward_ad import unpack_dual
 
 try:
     import flash_attn_legacy_cuda
@@ -291,9 +292,10 @@ def flash_attn_with_kvcache(
         assert v is not None and k.shape == v.shape and k.shape[:2] == (b, lq), "k, v must be [B, L_q, H_kv, d]"
         # rows lens[b] ... lens[b] + Lq - 1 of every entry
         kd, vd = (k_cache, v_cache) if cache_layout == "bshd" else (k_cache.transpose(1, 2), v_cache.transpose(1, 2))
-        # what autograd has a say in (gradients; a cache made in inference mode, which it refuses to have written
-        # outside of it) goes through indexing
-        tracked = torch.is_grad_enabled() and any(t.requires_grad for t in (k, v, k_cache, v_cache))
+        # what autograd has a say in (gradients and forward-mode tangents, which the caches take over; a cache made
+        # in inference mode, which it refuses to have written outside of it) goes through indexing
+        tracked = ((torch.is_grad_enabled() and any(t.requires_grad for t in (k, v, k_cache, v_cache)))
+                   or any(unpack_dual(t).tangent is not None for t in (k, v, k_cache, v_cache)))
         frozen = not torch.is_inference_mode_enabled() and (k_cache.is_inference() or v_cache.is_inference())
         appended = None if tracked or frozen else flash_attn_legacy_cuda.cache_append(k, v, kd, vd, lens)
         if appended is not None:

@@ -38,3 +38,15 @@ def test_a_cache_made_in_inference_mode_is_not_written_outside_of_it(appended, w
     with torch.inference_mode(), pytest.raises(RuntimeError, match="CUDA"):
         flash_attn_with_kvcache(q, *caches, k=k, v=v, cache_seqlens=lens)
     assert len(appended) == 1
+
+
+def test_forward_mode_tangents_go_into_the_caches(appended):
+    from torch.autograd import forward_ad
+    q, kc, vc, k, v, lens = _tensors()
+    with forward_ad.dual_level():
+        tangent = torch.ones_like(v)
+        with pytest.raises(RuntimeError, match="CUDA"):
+            flash_attn_with_kvcache(q, kc, vc, k=k, v=forward_ad.make_dual(v, tangent), cache_seqlens=lens)
+        assert not appended
+        got = forward_ad.unpack_dual(vc).tangent
+        assert got is not None and torch.equal(got[1, 5:8], tangent[1]) and not got[1, :5].any()
