@@ -639,6 +639,27 @@ def decode(q, k_cache, v_cache, cache_seqlens, softmax_scale, k_new=None, v_new=
     return (o, lse) if return_lse else o
 
 
+def _rows_apart(k_cache, v_cache):
+    """Whether no element of one cache (same shapes) is one of the other's.
+
+    The append kernel writes both at once, where indexing writes K and then V.  Caches of one allocation are
+    recognised as apart when their strides nest: halves of one tensor, in whatever dimension, or separate pieces.
+    """
+    if k_cache.untyped_storage().data_ptr() != v_cache.untyped_storage().data_ptr():
+        return True
+    gap = abs(v_cache.storage_offset() - k_cache.storage_offset())
+    dims = [(s, n) for s, n in zip(k_cache.stride(), k_cache.shape) if n > 1]
+    if k_cache.stride() != v_cache.stride():   # apart only if one ends before the other begins
+        first, second = sorted((k_cache, v_cache), key=lambda t: t.storage_offset())
+        return gap > sum(s * (n - 1) for s, n in zip(first.stride(), first.shape))
+    reach = 0
+    for stride, n in sorted(dims + [(gap, 2)]):
+        if stride <= reach:
+            return False
+        reach += stride * (n - 1)
+    return True
+
+
 def cache_append(k_new, v_new, k_cache, v_cache, cache_seqlens):
     """Writes k_new / v_new [B,Lq,Hkv,d] behind every entry's cached rows, in one launch.
 
@@ -663,7 +684,7 @@ def cache_append(k_new, v_new, k_cache, v_cache, cache_seqlens):
             or d not in (32, 64, 96, 128, 256) or not 0 < B <= 65535 or min(shape) == 0 or S == 0
             or cache_seqlens.dtype != torch.int32 or tuple(cache_seqlens.shape) != (B,)
             or cache_seqlens.device != k_cache.device or not cache_seqlens.is_contiguous()
-            or k_cache.device.index != torch.cuda.current_device()):
+            or k_cache.device.index != torch.cuda.current_device() or not _rows_apart(k_cache, v_cache)):
         return None
     lens = torch.empty((B,), dtype=torch.int32, device=k_cache.device)
     fits = torch.empty((1,), dtype=torch.bool, device=k_cache.device)

@@ -61,3 +61,13 @@ def test_tensors_the_kernel_cannot_address_are_left_to_indexing(ext):
         assert ext.cache_append(*bad, lens) is None
     assert ext.cache_append(k, v, kc, vc, lens.long()) is None
     assert torch.equal(kc, before)
+
+
+def test_one_tensor_for_both_caches_ends_up_with_the_values(ext):
+    gen = torch.Generator().manual_seed(5)
+    kc, _, k, v = _case(gen, 2, 64, 4, 64, 8, "bshd", False)
+    lens = torch.tensor([0, 30], dtype=torch.int32).cuda()
+    assert ext.cache_append(k, v, kc, kc, lens) is None       # (the kernel writes both at once)
+    kv = torch.zeros(2, 64, 2, 4, 64, dtype=torch.float16, device="cuda")   # K and V of a position side by side
+    assert ext.cache_append(k, v, kv[:, :, 0], kv[:, :, 1], lens) is not None
+    assert torch.equal(kv[1, 30:38, 0], k[1]) and torch.equal(kv[1, 30:38, 1], v[1])

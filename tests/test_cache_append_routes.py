@@ -50,3 +50,19 @@ def test_forward_mode_tangents_go_into_the_caches(appended):
         assert not appended
         got = forward_ad.unpack_dual(vc).tangent
         assert got is not None and torch.equal(got[1, 5:8], tangent[1]) and not got[1, :5].any()
+
+
+@pytest.mark.parametrize("make,apart", [
+    (lambda t: (t[0], t[1]), True),                                          # halves of one allocation
+    (lambda t: (t.view(2, 10, 2, 3, 32)[:, :, 0], t.view(2, 10, 2, 3, 32)[:, :, 1]), True),   # K and V of a position side by side
+    (lambda t: (t.view(2, 10, 3, 64)[..., :32], t.view(2, 10, 3, 64)[..., 32:]), True),       # of a head
+    (lambda t: (t.clone()[0], t[0]), True),
+    (lambda t: (t[0], t[0]), False),                                         # one tensor for both
+    (lambda t: (t[0, :, :9], t[0, :, 1:]), False),
+    (lambda t: (t[0, 0], t[1, 0]), True),
+    (lambda t: (t[0, 0], t[0].transpose(1, 2)[1].transpose(0, 1)), True),    # other strides, behind the first
+    (lambda t: (t.flatten()[:960].view(1, 10, 3, 32), t.flatten()[512:1472].view(1, 10, 3, 32)), False),
+])
+def test_caches_that_share_rows_are_told_from_those_that_share_an_allocation(make, apart):
+    k_cache, v_cache = make(torch.zeros(2, 2, 10, 3, 32, dtype=torch.float16))
+    assert ext._rows_apart(k_cache, v_cache) is apart and ext._rows_apart(v_cache, k_cache) is apart
