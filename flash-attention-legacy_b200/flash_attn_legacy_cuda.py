@@ -242,6 +242,11 @@ def _same_device(*ts):
     return dev
 
 
+def _scale(softmax_scale):
+    """The scale as the C calls take it: anything float() takes, rounded to 32 bits (too large: infinity)."""
+    return ctypes.c_float(float(softmax_scale)).value
+
+
 def forward(Q, K, V, softmax_scale, is_causal=False, out=None, lse=None):
     """Batched forward.  Q [B,Hq,N,d], K/V [B,Hkv,N,d] fp16 -> [O [B,Hq,N,d] fp16, L [B,Hq,N] fp32].
 
@@ -264,7 +269,7 @@ def forward(Q, K, V, softmax_scale, is_causal=False, out=None, lse=None):
     _check(_fwd_run(_FWD_ARGS.pack(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), L.data_ptr(), 0,
                                    B, Hq, Hkv, N, N, d,
                                    *Q.stride()[:3], *K.stride()[:3], *V.stride()[:3], *O.stride()[:3],
-                                   softmax_scale, 1 if is_causal else 0, _status_ptr(dev), _raw_stream(dev))))
+                                   _scale(softmax_scale), 1 if is_causal else 0, _status_ptr(dev), _raw_stream(dev))))
     return [O, L]
 
 
@@ -331,7 +336,7 @@ def forward_kvcache(Q, K_cache, V_cache, cache_seqlens, softmax_scale, is_causal
     args = _FWD_ARGS.pack(Q.data_ptr(), K_cache.data_ptr(), V_cache.data_ptr(), O.data_ptr(), L.data_ptr(),
                           cache_seqlens.data_ptr(), B, Hq, Hkv, Nq, S, d,
                           *Q.stride()[:3], *K_cache.stride()[:3], *V_cache.stride()[:3], *O.stride()[:3],
-                          softmax_scale, 2 if is_causal else 0, _status_ptr(dev), _raw_stream(dev))
+                          _scale(softmax_scale), 2 if is_causal else 0, _status_ptr(dev), _raw_stream(dev))
     nbytes = _lib.fal_fwd_kvcache_workspace_bytes(B, Hq, Nq, S, d)
     if nbytes:
         ws = torch.empty(nbytes, dtype=torch.uint8, device=Q.device)
@@ -415,7 +420,7 @@ def backward(dO, Q, K, V, O, L, softmax_scale, is_causal=False, out=None, worksp
                                    B, Hq, Hkv, Nq, Nk, d,
                                    *dO.stride()[:3], *Q.stride()[:3], *K.stride()[:3], *V.stride()[:3],
                                    *O.stride()[:3], *dQ.stride()[:3], *dK.stride()[:3], *dV.stride()[:3],
-                                   softmax_scale, _causal_code(is_causal, bottom_right),
+                                   _scale(softmax_scale), _causal_code(is_causal, bottom_right),
                                    ws.data_ptr(), nbytes, _status_ptr(dev), _raw_stream(dev))))
     return [dQ, dK, dV]
 
@@ -634,7 +639,7 @@ def decode(q, k_cache, v_cache, cache_seqlens, softmax_scale, k_new=None, v_new=
                                          k_new.data_ptr() if k_new is not None else 0,
                                          v_new.data_ptr() if v_new is not None else 0,
                                          o.data_ptr(), lse.data_ptr() if lse is not None else 0,
-                                         B, Hq, Hkv, S, d, softmax_scale, *ks, *vs,
+                                         B, Hq, Hkv, S, d, _scale(softmax_scale), *ks, *vs,
                                          ws.data_ptr(), nbytes, _status_ptr(dev), _raw_stream(dev))))
     return (o, lse) if return_lse else o
 

@@ -1,5 +1,6 @@
 """The one-block calls of the C ABI: the block layouts of the Python binding and the argument checks behind them."""
 import ctypes
+import struct
 
 import pytest
 
@@ -23,3 +24,13 @@ def test_blocks_of_zeros_and_null_are_refused():
     for run, layout in ((ext._fwd_run, ext._FWD_ARGS), (ext._bwd_run, ext._BWD_ARGS), (ext._decode_run, ext._DECODE_ARGS)):
         assert run(bytes(layout.size)) == INVALID
         assert run(ctypes.c_char_p(None)) == INVALID
+
+
+@pytest.mark.parametrize("given", ["0.125", 1e39, -1e39, 1e-50, 0.1, 2])
+def test_scales_are_converted_as_ctypes_converts_them(given):
+    """Whatever float() takes goes into the block as the 32-bit float a C argument would be."""
+    want = ctypes.c_float(float(given)).value
+    block = _fwd(scale=ext._scale(given))
+    assert struct.unpack_from("@f", block, 6 * 8 + 6 * 4 + 12 * 8)[0] == want
+    if want <= 0:
+        assert ext._fwd_run(block) == INVALID
