@@ -191,15 +191,18 @@ int forward_variant(int head_dim, int64_t blocks_of_256_rows, int64_t units, int
 
 // CTAs that share the keys of each query block of a chunk behind a cache.  A chunk with fewer than half as many
 // 128-row blocks as there are SMs is bound by one CTA's walk over the cache; its keys are then dealt to as many
-// CTAs as the SMs hold, two key tiles or more each.  us a call, one CTA per block against this: 1 entry (32 / 8 heads of 128)
-// behind 4 000 keys, 16 queries 83 / 32, 128 queries 85 / 38, 512 queries 95 / 64; 1 entry (8 / 1 of 64) behind
-// 8 000, 40 queries 101 / 30; 2 entries (16 of 256) behind 1 500 and 3 000, 60 queries 99 / 48.
+// CTAs as the SMs hold, two key tiles or more each in a full cache.  Each entry's tiles are dealt evenly, two or more
+// to a CTA, and a short entry's to one (chunk_shared_tiles).  us on the GPU, one CTA per block against this, 32 / 8
+// heads of 128 in caches of 4 096 and of 32 768: 16 queries behind 100 keys 6.7 / 8.0, 500 10.8 / 10.8, 900 13.8 / 11.0,
+// 3 400 33.1 / 16.0; 130 queries behind 100 8.1 / 9.5, 500 10.9 / 12.1, 900 15.4 / 16.0, 3 400 34.8 / 25.6.
+// 2 entries (16 of 256), 60 queries: 40 keys 7.3 / 9.0, 940 22.3 / 17.0, 7 940 138 / 55.8.
 int chunk_kv_splits(int64_t blocks, int capacity) {
   const int64_t sms = sm_count() > 0 ? sm_count() : 148;
   const int64_t most = (capacity + 255) / 256;
   int64_t s = blocks > 0 ? sms / blocks : 1;
   if (s > most) s = most;
-  return s < 2 ? 1 : static_cast<int>(s < 32 ? s : 32);  // (the merge takes a split per lane)
+  if (s > 32) s = 32;  // (the merge takes a split per lane)
+  return s < 2 || (capacity + 127) / 128 < fal::chunk_shared_tiles(static_cast<int>(s)) ? 1 : static_cast<int>(s);
 }
 size_t chunk_split_bytes(int splits, int batch, int heads_q, int seqlen_q, int head_dim) {
   return splits < 2 ? 0 : static_cast<size_t>(splits) * batch * heads_q * seqlen_q * (head_dim + 1) * sizeof(float);

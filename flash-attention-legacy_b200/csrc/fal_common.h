@@ -19,6 +19,14 @@ struct RowStrides {
   int64_t row;
 };
 
+// Key tiles (of 128) from which on the keys of a chunk's query block are dealt to `splits` CTAs; with fewer, one of
+// them takes all keys and writes the result itself.  The merge of the partial results costs about 3 us where a block
+// is halved (its rows are many then) and 1 us where it is cut finer.  us on the GPU, one CTA takes all / shared, 32
+// heads of 128: 130 queries, 2 splits of 630 keys 12.1 / 13.3, of 1 030 16.6 / 16.0; 4 splits, 2 queries of 502 keys
+// 10.4 / 10.3, 16 queries of 516 11.8 / 10.7; 8 heads of 64, 18 splits, 40 queries of 500 keys 9.1 / 9.5.
+// (Not splitting such a call at all would save the merge's launch, about 1.2 us, but only the GPU knows the lengths.)
+__host__ __device__ constexpr int chunk_shared_tiles(int splits) { return splits < 3 ? 8 : 5; }
+
 struct FwdParams {
   void* o;     // fp16 output
   float* lse;  // natural-log LSE of the scaled scores

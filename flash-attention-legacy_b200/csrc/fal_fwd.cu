@@ -209,9 +209,11 @@ __device__ __forceinline__ void fwd_heaviest_block(const FwdParams& p, int slot,
   }
 }
 
-// Key tiles of a sequence of `keys` keys that one of `splits` CTAs takes.
+// Key tiles of a sequence of `keys` keys that one of at most `splits` CTAs takes: two or more, and all of them where
+// they are few.
 __device__ __forceinline__ int fwd_split_tiles(int keys, int splits) {
-  return ((keys + kTileN - 1) / kTileN + splits - 1) / splits;
+  const int tiles = (keys + kTileN - 1) / kTileN;
+  return tiles < chunk_shared_tiles(splits) ? max(tiles, 1) : max((tiles + splits - 1) / splits, 2);
 }
 
 // Maps blockIdx.x to a unit of work.  Returns false when the block has none
@@ -301,7 +303,9 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t sr
 
 // SHIFTED (causal only): the mask's diagonal is moved by seqlen_k - seqlen_q keys (bottom-right
 // alignment); the kernels of the reference's own top-left mask are compiled without it.
-template <int D, bool CAUSAL, bool SHIFTED, int SHAPE>
+// SPLIT: the keys of a query block are dealt to gridDim.y CTAs.  A kernel of its own: the code costs the others up
+// to 5 % (short rows at head_dim 256 without a mask 12.8 -> 13.3 us, 16 heads x 16 384 of 64 causal 755 -> 791).
+template <int D, bool CAUSAL, bool SHIFTED, int SHAPE, bool SPLIT>
 __global__ void __launch_bounds__(FwdSmem<D, SHAPE>::kThreads, FwdSmem<D, SHAPE>::kCtasPerSm)
 fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -309,9 +313,8 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   using L = FwdSmem<D, SHAPE>;
   constexpr int NS = L::kStages;
   constexpr int kSmWarps = L::kSmWarps;
-  // Instances that a chunk behind a cache does not run carry no code for it: with it the two-tile kernel at
-  // head_dim 64 spilled more in its main loop (16 heads x 16 384 causal 755 -> 791 us).
-  constexpr bool kMaySplit = SHAPE == kOneTile && (SHIFTED || !CAUSAL);
+  static_assert(!SPLIT || (SHAPE == kOneTile && (SHIFTED || !CAUSAL)), "a split chunk behind a cache");
+  if (SPLIT) grid_dependency_launch();  // the merge waits for this grid's end
 
   FwdWork wk;
   constexpr int kCtaRows = L::kCtaRows;
@@ -341,13 +344,15 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   // Several CTAs share this block's keys: this one takes its range of the entry's key tiles, as a shorter key
   // sequence with the diagonal moved along.  A range that no row of the block sees is left alone: the merge knows
   // that it has no part in them.  (Visited for its hidden scores, an infinity among its values would reach rows
-  // that cannot see it.)
-  if (kMaySplit && p.kv_splits > 1) {
-    const int per = fwd_split_tiles(wk.seqlen_k, p.kv_splits);
-    const int key0 = static_cast<int>(blockIdx.y) * per * kTileN;
+  // that cannot see it.)  Where the range is all the keys the first CTA finishes the block by itself.
+  bool shared = false;
+  if (SPLIT) {
+    const int range = fwd_split_tiles(wk.seqlen_k, p.kv_splits) * kTileN;
+    const int key0 = static_cast<int>(blockIdx.y) * range;
     const int seen = SHIFTED ? min(wk.seqlen_k, (wk.qblk + 1) * kTileM + cshift) : wk.seqlen_k;
-    if (key0 >= seen) return;
-    wk.seqlen_k = min(wk.seqlen_k - key0, per * kTileN);
+    shared = range < wk.seqlen_k;
+    if (shared ? key0 >= seen : blockIdx.y != 0) return;
+    wk.seqlen_k = min(wk.seqlen_k - key0, range);
     wk.k_row0 += key0;
     if (SHIFTED) cshift -= key0;
   }
@@ -808,7 +813,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const bool tile_used = (kAlt || wg < L::kQTiles) && q_tile0 < wk.seqlen_q;
     // (Not at head_dim 256: measured 5 - 10 % slower there -- the CTA then waits for the TMA unit to read
     // 64 KB of staging before it can exit, where plain stores drain behind its back.)
-    const bool by_tma = D != 256 && p.store_by_tma != 0 && !(kMaySplit && p.kv_splits > 1) && tile_used &&
+    const bool by_tma = D != 256 && p.store_by_tma != 0 && !shared && tile_used &&
                         (p.cu_q == nullptr || q_tile0 + kTileM <= wk.seqlen_q);
     const int64_t part_row =
         ((static_cast<int64_t>(blockIdx.y) * p.batch + wk.batch) * p.heads_q + wk.head) * p.seqlen_q + q_local;
@@ -835,7 +840,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           // box c / 2, 16-byte chunk (c % 2) * 4 + v of the row, 128-byte XOR swizzle
           *reinterpret_cast<uint4*>(stage_row + (c >> 1) * L::kBoxBytes + ((((c & 1) * 4 + v) ^ (row & 7)) << 4)) = out;
         }
-      } else if (kMaySplit && row_ok && p.kv_splits > 1) {
+      } else if (SPLIT && row_ok && shared) {
         float* part = p.part_o + part_row * p.head_dim + c * 32;
         if (c * 32 < p.head_dim) {
 #pragma unroll
@@ -860,7 +865,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     if (row_ok && (!kAlt || wg == 0)) {
       const float lse = (nt > 0 && m_ref != kNegInf) ? m_ref * p.scale + logf(fmaxf(l, 1e-20f))
                                                       : kNegInf;
-      if (kMaySplit && p.kv_splits > 1) p.part_lse[part_row] = lse;
+      if (SPLIT && shared) p.part_lse[part_row] = lse;
       else p.lse[wk.lse_base + static_cast<int64_t>(q_local) * p.lse_strides.row] = lse;
     }
     if (by_tma) {  // the same for every thread that wrote into the tile's staging buffer
@@ -890,19 +895,21 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 // Merges the splits of a query block's keys: a warp per (batch, head, row), split s on lane s for the weights,
 // 16 bytes of every split's row per lane for the sum.  Only the splits with keys that the row sees are read: the
 // others have nothing to add, and what they hold may be another row's infinity (or memory nobody wrote).
-// Bound by the partials' traffic, at most 128 rows per SM.
+// Bound by the partials' traffic, at most 128 rows per SM, and by its launch, which therefore does not wait for the
+// end of the split grid; the kernel does, before it reads a partial.
 __global__ void __launch_bounds__(128) fal_fwd_combine_kernel(const FwdParams p) {
   const int lane = threadIdx.x & 31;
   const int row = static_cast<int>(blockIdx.x) * 4 + (threadIdx.x >> 5);
-  if (row >= p.seqlen_q) return;
   const int head = blockIdx.y;
   const int64_t b = blockIdx.z;
   const int64_t rows = static_cast<int64_t>(p.batch) * p.heads_q * p.seqlen_q;
   const int64_t id = (b * p.heads_q + head) * p.seqlen_q + row;
   const int keys = max(min(__ldg(p.seqused_k + b), p.seqlen_k), 0);
+  const int range = fwd_split_tiles(keys, p.kv_splits) * kTileN;
   const int seen = p.shift_per_sequence != 0 ? row + 1 + keys - p.seqlen_q : keys;
-  const int split_keys = fwd_split_tiles(keys, p.kv_splits) * kTileN;
-  const int splits = seen > 0 ? (seen + split_keys - 1) / split_keys : 0;
+  const int splits = seen > 0 ? (seen + range - 1) / range : 0;
+  grid_dependency_wait();
+  if (row >= p.seqlen_q || range >= keys) return;  // (range >= keys: the entry's blocks are finished)
   const float l = lane < splits ? p.part_lse[lane * rows + id] : kNegInf;
   float m = l;
 #pragma unroll
@@ -918,6 +925,7 @@ __global__ void __launch_bounds__(128) fal_fwd_combine_kernel(const FwdParams p)
   for (int base = 0; base < p.head_dim; base += 128) {
     const int c = base + lane * 4;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
     for (int s = 0; s < splits; ++s) {
       const float ws = __shfl_sync(0xffffffffu, w, s);
       if (c < p.head_dim) {
@@ -939,23 +947,29 @@ __global__ void __launch_bounds__(128) fal_fwd_combine_kernel(const FwdParams p)
     p.lse[b * p.lse_strides.batch + head * p.lse_strides.head + row] = m == kNegInf ? kNegInf : m + logf(fmaxf(sum, 1e-20f));
 }
 
-template <int D, bool CAUSAL, bool SHIFTED, int SHAPE>
+template <int D, bool CAUSAL, bool SHIFTED, int SHAPE, bool SPLIT = false>
 cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const CUtensorMap& to, const FwdParams& p, int grid, cudaStream_t stream) {
   using L = FwdSmem<D, SHAPE>;
-  auto kern = fal_fwd_kernel<D, CAUSAL, SHIFTED, SHAPE>;
+  auto kern = fal_fwd_kernel<D, CAUSAL, SHIFTED, SHAPE, SPLIT>;
   static DeviceOnce configured;  // one per template instance
   cudaError_t e = configured.run([&] {
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAllocBytes);
   });
   if (e != cudaSuccess) return e;
-  kern<<<dim3(grid, p.kv_splits > 1 ? p.kv_splits : 1), L::kThreads, L::kAllocBytes, stream>>>(tq, tk, tv, to, p);
+  kern<<<dim3(grid, SPLIT ? p.kv_splits : 1), L::kThreads, L::kAllocBytes, stream>>>(tq, tk, tv, to, p);
   return cudaGetLastError();
 }
 
 template <int D, int SHAPE>
 cudaError_t launch_fwd_d(bool causal, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const CUtensorMap& to, const FwdParams& p, int grid, cudaStream_t stream) {
+  if constexpr (SHAPE == kOneTile) {
+    if (p.kv_splits > 1 && causal && p.shift_per_sequence != 0)
+      return launch_fwd_t<D, true, true, SHAPE, true>(tq, tk, tv, to, p, grid, stream);
+    if (p.kv_splits > 1 && !causal) return launch_fwd_t<D, false, false, SHAPE, true>(tq, tk, tv, to, p, grid, stream);
+  }
+  if (p.kv_splits > 1) return cudaErrorInvalidValue;  // no instance for a share of the keys
   if (causal && (p.causal_shift != 0 || p.shift_per_sequence != 0))
     return launch_fwd_t<D, true, true, SHAPE>(tq, tk, tv, to, p, grid, stream);
   return causal ? launch_fwd_t<D, true, false, SHAPE>(tq, tk, tv, to, p, grid, stream)
@@ -966,8 +980,7 @@ cudaError_t launch_fwd_d(bool causal, const CUtensorMap& tq, const CUtensorMap& 
 
 cudaError_t launch_fwd_combine(const FwdParams& p, cudaStream_t stream) {
   // (heads and entries fit the grid's y and z: a chunk of more than half as many blocks as SMs is not split)
-  fal_fwd_combine_kernel<<<dim3((p.seqlen_q + 3) / 4, p.heads_q, p.batch), 128, 0, stream>>>(p);
-  return cudaGetLastError();
+  return launch_dependent(fal_fwd_combine_kernel, dim3((p.seqlen_q + 3) / 4, p.heads_q, p.batch), dim3(128), 0, stream, p);
 }
 
 cudaError_t launch_fwd(int head_dim, bool causal, const CUtensorMap& tq, const CUtensorMap& tk,

@@ -111,3 +111,20 @@ def test_a_forced_variant_is_not_split(ext, variant):
         ext.set_forward_variant(ext.FWD_AUTO)
     assert torch.equal(o, o_whole) and torch.equal(lse, lse_whole)
     assert torch.isnan(ws).all()   # nobody wrote a partial result
+
+
+@pytest.mark.parametrize("nq,hq,capacity,splits,most", [(16, 32, 3000, 4, 512), (130, 32, 3000, 2, 896), (40, 8, 9000, 18, 512)])
+@pytest.mark.parametrize("mask", [0, 2])
+def test_entries_of_few_keys_are_not_shared(ext, nq, hq, capacity, splits, most, mask):
+    """A large cache that holds little so far: one thread block finishes each query block without partial results,
+    up to `most` keys; with one more the keys are shared.  (The first 4 KB of the workspace hold the first rows of
+    split 0, which computes the keys that every row sees.)"""
+    for keys in (most + 1, most, nq, 1):
+        q, kc, vc, lens, ws = _inputs(ext, hq, hq, 64, nq, [keys], capacity)
+        assert ws.numel() == splits * hq * nq * 65
+        o, lse = _call(ext, q, kc, vc, lens, mask, ws)
+        assert torch.isnan(ws).all().item() == (keys <= most) and torch.isnan(ws[:1024]).any().item() == (keys <= most)
+        o_whole, lse_whole = _call(ext, q, kc, vc, lens, mask)
+        assert orc.rel_max_err(o, o_whole) <= orc.TOL_O
+        seen = torch.isfinite(lse_whole)
+        assert torch.equal(seen, torch.isfinite(lse)) and orc.abs_max_err(lse[seen], lse_whole[seen]) <= orc.TOL_LSE
