@@ -408,6 +408,15 @@ int fwd_batched(const void* q, const void* k, const void* v, void* o, float* lse
   p.num_qblk = (seqlen_q + p.cta_rows - 1) / p.cta_rows;
   const int64_t grid = static_cast<int64_t>(p.num_qblk) * batch * heads_q;
   if (grid > 0x7fffffff) return FAL_ERR_INVALID_ARGUMENT;
+  // Ragged caches: heaviest blocks first, where the order matters: more blocks than the SMs take at once, and not
+  // so many that the last wave is nothing beside the search, which costs every CTA about half a microsecond.
+  // us, as they come / heaviest first (heads of 128, queries behind 100 to 4 000 keys): 16 x 32 heads x 4 queries, 3.5
+  // waves 142 / 129; 16 x 32 x 300, 7 waves 299 / 285; 64 x 32 x 4, 14 waves behind 2 000 keys 244 / 251; 100 x 32 x 64,
+  // 22 waves 391 / 410; 64 x 8 of 64 x 257, 5 waves 118 / 110; 128 x 16 of 64 x 130, 14 waves 391 / 395.
+  constexpr int64_t kOrderedWaves = 8;
+  const int64_t at_once = static_cast<int64_t>(sm_count() > 0 ? sm_count() : 148) * (p.half_sm != 0 ? 2 : 1);
+  p.heaviest_first = seqused_k != nullptr && p.shift_per_sequence != 0 && batch > 1 &&
+                     batch <= fal::kOrderedEntries && grid > at_once && grid <= kOrderedWaves * at_once;
   const int rec = g_timer.begin(FAL_KERNEL_FWD, st);
   cudaError_t e = fal::launch_fwd(kdim, is_causal != 0, tq, tk, tv, to, p, static_cast<int>(grid), st);
   g_timer.end(FAL_KERNEL_FWD, rec, st);

@@ -19,6 +19,9 @@ struct RowStrides {
   int64_t row;
 };
 
+// Batch entries whose lengths a warp of the forward holds in registers to order their blocks by weight.
+constexpr int kOrderedEntries = 128;
+
 // Key tiles (of 128) from which on the keys of a chunk's query block are dealt to `splits` CTAs; with fewer, one of
 // them takes all keys and writes the result itself.  The merge of the partial results costs about 3 us where a block
 // is halved (its rows are many then) and 1 us where it is cut finer.  us on the GPU, one CTA takes all / shared, 32
@@ -50,6 +53,7 @@ struct FwdParams {
   int store_by_tma;  // O tiles leave through shared memory and TMA stores (the output's tensor map is valid)
   const int32_t* seqused_k;  // batched mode, optional: keys in use per batch entry (a cache filled to different
                              // lengths); seqlen_k is then the capacity, and shift_per_sequence applies per entry
+  int heaviest_first;  // (shift_per_sequence, seqused_k, at most kOrderedEntries entries) blocks with most keys first
   int kv_splits;     // (seqused_k) CTAs that share a query block's keys, each a range of key tiles; 1: none
   float* part_o;     // kv_splits > 1: [split, batch, heads_q, seqlen_q, head_dim] fp32, normalised per split
   float* part_lse;   // [split, batch, heads_q, seqlen_q]

@@ -168,23 +168,42 @@ struct FwdWork {
 };
 
 // The slot-th heaviest (entry, query block) of a chunk of queries behind caches of different lengths, by key
-// tiles: entry b's block q sees about lens[b] + q * cta_rows keys.  Every warp finds it for itself: a binary
-// search over the tile count (how many blocks have at least v tiles: a closed form per entry, entries on the
-// lanes), then the rank among the blocks of exactly that count, of which an entry has at most one.
-__device__ __forceinline__ void fwd_heaviest_block(const FwdParams& p, int slot, int& entry, int& qblk) {
+// tiles: entry b's block q sees about lens[b] + q * ROWS keys.  Every warp finds it for itself: a binary search over
+// the tile count (how many blocks have at least v tiles: a closed form per entry, entries on the lanes, their lengths
+// in registers), then the rank among the blocks of exactly that count, of which an entry has at most one.
+// Returns false, at less cost, when the lengths differ by less than a block: a grid with the last blocks of all
+// entries first is then in that order by itself.
+template <int ROWS>
+__device__ __forceinline__ bool fwd_heaviest_block(const FwdParams& p, int slot, int& entry, int& qblk) {
+  static_assert(ROWS >= kTileN && (ROWS & (ROWS - 1)) == 0, "an entry's blocks differ by a key tile or more");
+  constexpr int kPerLane = kOrderedEntries / 32;
   const int lane = threadIdx.x & 31;
-  auto blocks_from = [&](int b, int v) -> int {  // blocks of entry b with at least v tiles
-    const int len = max(min(__ldg(p.seqused_k + b), p.seqlen_k), 0);
-    const int short_by = v * kTileN - len;
-    return p.num_qblk - min(max((short_by + p.cta_rows - 1) / p.cta_rows, 0), p.num_qblk);
+  int len[kPerLane];
+  int longest = 0, shortest = p.seqlen_k;
+#pragma unroll
+  for (int i = 0; i < kPerLane; ++i) {
+    const int b = i * 32 + lane;
+    len[i] = -(1 << 30);  // (no entry: no block)
+    if (b < p.batch) {
+      len[i] = max(min(__ldg(p.seqused_k + b), p.seqlen_k), 0);
+      longest = max(longest, len[i]);
+      shortest = min(shortest, len[i]);
+    }
+  }
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  if (longest - __reduce_min_sync(0xffffffffu, shortest) < ROWS) return false;
+  auto blocks_from = [&](int length, int v) -> int {  // blocks of an entry with at least v tiles
+    return p.num_qblk - min(max((v * kTileN - length + ROWS - 1) / ROWS, 0), p.num_qblk);
   };
   auto count = [&](int v) -> int {
     int n = 0;
-    for (int b = lane; b < p.batch; b += 32) n += blocks_from(b, v);
+#pragma unroll
+    for (int i = 0; i < kPerLane; ++i)
+      if (i * 32 < p.batch) n += blocks_from(len[i], v);
     return __reduce_add_sync(0xffffffffu, n);
   };
   int lo = 0;  // count(lo) > slot
-  int hi = (p.seqlen_k + p.num_qblk * p.cta_rows) / kTileN + 1;  // count(hi) == 0
+  int hi = (longest + p.num_qblk * ROWS) / kTileN + 1;  // count(hi) == 0
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
     if (count(mid) > slot) lo = mid;
@@ -193,20 +212,20 @@ __device__ __forceinline__ void fwd_heaviest_block(const FwdParams& p, int slot,
   int rank = slot - count(lo + 1);
   entry = 0;
   qblk = 0;
-  for (int base = 0; base < p.batch; base += 32) {
-    const int b = base + lane;
-    const int n = b < p.batch ? blocks_from(b, lo) : 0;
-    const bool has = b < p.batch && n > blocks_from(b, lo + 1);
+#pragma unroll
+  for (int i = 0; i < kPerLane; ++i) {
+    const int n = blocks_from(len[i], lo);
+    const bool has = n > blocks_from(len[i], lo + 1);
     const unsigned mask = __ballot_sync(0xffffffffu, has);
-    if (rank < __popc(mask)) {
+    if (rank >= 0 && rank < __popc(mask)) {
       const unsigned hit = __ballot_sync(0xffffffffu, has && __popc(mask & ((1u << lane) - 1u)) == rank);
       const int src = __ffs(hit) - 1;
-      entry = base + src;
+      entry = i * 32 + src;
       qblk = p.num_qblk - __shfl_sync(0xffffffffu, n, src);
-      return;
     }
-    rank -= __popc(mask);
+    rank -= __popc(mask);  // (negative: found)
   }
+  return true;
 }
 
 // Key tiles of a sequence of `keys` keys that one of at most `splits` CTAs takes: two or more, and all of them where
@@ -218,8 +237,9 @@ __device__ __forceinline__ int fwd_split_tiles(int keys, int splits) {
 
 // Maps blockIdx.x to a unit of work.  Returns false when the block has none
 // (packed mode launches an upper bound of blocks).
-template <bool SHIFTED>
-__device__ __forceinline__ bool fwd_decode_work(const FwdParams& p, int cta_rows, FwdWork& w) {
+template <bool SHIFTED, int ROWS>
+__device__ __forceinline__ bool fwd_decode_work(const FwdParams& p, FwdWork& w) {
+  constexpr int cta_rows = ROWS;
   const int idx = blockIdx.x;
   if (p.cu_q == nullptr) {
     const int bh_count = p.batch * p.heads_q;
@@ -228,12 +248,11 @@ __device__ __forceinline__ bool fwd_decode_work(const FwdParams& p, int cta_rows
     const int bh = idx % bh_count;
     w.batch = bh / p.heads_q;
     w.head = bh % p.heads_q;
-    if (SHIFTED && p.seqused_k != nullptr && p.shift_per_sequence != 0 && p.batch > 1) {
+    if (SHIFTED && p.heaviest_first != 0) {
       // Entries of 1 500 and of 8 000 keys in one grid: in the order above the longest entry's last blocks
       // start late and the SMs wait for them.  Heaviest first, 4 entries x 1 024 queries (32 / 8 heads of 128)
       // behind 512 to 7 000 keys: 329 -> 310 us a call; the search costs a CTA well under a microsecond.
-      w.head = idx % p.heads_q;
-      fwd_heaviest_block(p, idx / p.heads_q, w.batch, w.qblk);
+      fwd_heaviest_block<ROWS>(p, idx / p.heads_q, w.batch, w.qblk);
     }
     w.q_row0 = 0;
     w.k_row0 = 0;
@@ -318,7 +337,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 
   FwdWork wk;
   constexpr int kCtaRows = L::kCtaRows;
-  if (!fwd_decode_work<SHIFTED>(p, kCtaRows, wk)) return;
+  if (!fwd_decode_work<SHIFTED, kCtaRows>(p, wk)) return;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
