@@ -166,27 +166,53 @@ std::atomic<int> g_fwd_variant{FAL_FWD_AUTO};  // fal_set_fwd_variant
 
 // At head_dim 64 the TMEM and shared memory of an SM hold two CTAs of one tile and one softmax warpgroup.
 // They overlap as the two tiles of a two-tile CTA do, and each one's prologue and epilogue run under the
-// other's main loop besides, which is what short rows spend their time on; the price is that every K / V
-// tile is fetched once per 128 query rows.  us, two tiles against half-SM CTAs: 32 x 16 heads x 577 142 / 123,
-// 48 x 32 x 65 59 / 37, 20 x 8 x 257 causal 29 / 21, 8 x 16 x 512 causal 27 / 25, 4 x 16 x 2 048 133 / 129 and
-// causal 80 / 76; 2 x 16 x 4 096 232 / 236, 16 x 8 192 causal 213 / 219, 16 x 16 384 causal 757 / 796: the line
-// lies at 2 048 keys a row on average.  With no more than one CTA per SM the alternating warpgroups of the
-// one-tile CTA are faster (2 x 8 x 1 024 causal: 17 against 21).  At head_dim 128, the same shape with single
-// K and V buffers measured 89 against 93 us on 16 x 16 x 577 but 665 against 578 on 4 x 32 x 4 096 causal and
-// 116 against 112 on 2 x 32 x 1 500 (64 KB of K and V per tile and CTA); it is not built.
+// other's main loop besides, which is what short rows spend their time on; a sequence ends in at most one partial
+// tile instead of two, and under a causal mask the upper tile does not wait for the lower.  The price is that every
+// K / V tile is fetched once per 128 query rows.  us, the better of the others against half-SM CTAs (units: batch x
+// heads of 64):
+//   causal: 256 units x 257 rows 30.3 / 21.1, 64 x 577 18.2 / 13.1, 128 x 1 024 47.9 / 43.3, 32 x 1 300 25.1 / 21.8,
+//     256 x 2 600 454 / 423, 128 x 4 000 463 / 456, 256 x 4 000 1 030 / 1 007; 16 x 4 000 58.1 / 59.0;
+//     with at most two per SM, against one tile per CTA, 32 x 1 143 17.4 / 18.2;
+//   no mask, an odd number of 128-row tiles: 256 x 100 10.8 / 7.2, 256 x 257 33.8 / 27.5, 128 x 577 36.6 / 34.5,
+//     640 x 1 300 579 / 577; with at most two CTAs per SM, where the last two tiles of two-tile CTAs run at once just
+//     the same, 64 x 257 10.7 / 11.3, 32 x 577 13.5 / 14.7, 16 x 1 600 26.8 / 29.4;
+//   no mask, an even number: 208 x 145 17.1 / 13.5, 640 x 400 103 / 97, 320 x 696 101.8 / 96.8, but 128 x 400 (3.5 CTAs
+//     per SM) 23.0 / 23.9, 640 x 1 024 310 / 324, 256 x 2 048 429 / 473.
+// Packed sequences without a mask end in odd and even tiles: 24 of 500 to 1 500 (16 heads) 228 / 218, 200 of 10 to 300
+// 215 / 174, 8 of 2 048 216 / 223.  With one CTA per SM or fewer the alternating warpgroups of the one-tile CTA are faster
+// (16 x 1 024 causal: 12 against 16), for rows of a single tile the half-SM CTA still is (128 x 100: 6.0 / 5.75).  At
+// head_dim 128, the same shape with single K and V buffers measured 89 against 93 us on 16 x 16 x 577 but 665 against
+// 578 on 4 x 32 x 4 096 causal and 116 against 112 on 2 x 32 x 1 500 (64 KB of K and V per tile and CTA); it is not built.
 constexpr int kHalfSmMaxKeys = 2048;
 
-int forward_variant(int head_dim, int64_t blocks_of_256_rows, int64_t units, int64_t mean_keys) {
+// rows: of every sequence, or 0 for packed sequences of their own lengths; blocks: of 256 and of 128 rows per unit;
+// one_tile: the better of the other two shapes.
+bool half_sm_pays(int rows, int64_t blocks_of_256, int64_t blocks_of_128, int64_t units, int64_t mean_keys, bool masked,
+                  bool one_tile, int64_t sms) {
+  if (mean_keys > kHalfSmMaxKeys || 2 * blocks_of_256 * units <= sms) return false;
+  const int64_t ctas = blocks_of_128 * units;
+  if (rows > 0 && rows <= 128) return true;
+  if (ctas <= sms) return false;
+  if (ctas <= 2 * sms) return masked ? !one_tile : blocks_of_256 * units > sms;
+  if (masked) return true;
+  if (rows == 0) return mean_keys <= 1024;
+  return blocks_of_128 % 2 != 0 || (mean_keys <= 768 && ctas > (mean_keys <= 256 ? 2 : 4) * sms);
+}
+
+int forward_variant(int head_dim, int rows, int64_t blocks_of_256, int64_t blocks_of_128, int64_t units,
+                    int64_t mean_keys, bool masked) {
   const int forced = g_fwd_variant.load(std::memory_order_relaxed);
   if (head_dim == 256) return FAL_FWD_ONE_TILE;
   if (forced == FAL_FWD_HALF_SM) return head_dim == 64 ? forced : FAL_FWD_TWO_TILES;
   if (forced != FAL_FWD_AUTO) return forced;
   const int64_t sms = sm_count() > 0 ? sm_count() : 148;
-  const int64_t ctas2 = blocks_of_256_rows * units;
+  const int64_t ctas2 = blocks_of_256 * units;
   const int64_t waves2 = (ctas2 + sms - 1) / sms;
   const int64_t waves1 = (2 * ctas2 + sms - 1) / sms;
-  if (head_dim == 64 && 2 * ctas2 > sms && mean_keys <= kHalfSmMaxKeys) return FAL_FWD_HALF_SM;
-  return 6 * waves1 < 10 * waves2 ? FAL_FWD_ONE_TILE : FAL_FWD_TWO_TILES;
+  const bool one_tile = 6 * waves1 < 10 * waves2;
+  if (head_dim == 64 && half_sm_pays(rows, blocks_of_256, blocks_of_128, units, mean_keys, masked, one_tile, sms))
+    return FAL_FWD_HALF_SM;
+  return one_tile ? FAL_FWD_ONE_TILE : FAL_FWD_TWO_TILES;
 }
 
 // CTAs that share the keys of each query block of a chunk behind a cache.  A chunk with fewer than half as many
@@ -386,8 +412,9 @@ int fwd_batched(const void* q, const void* k, const void* v, void* o, float* lse
   p.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int kdim = kernel_head_dim(head_dim);
-  int variant = forward_variant(kdim, (seqlen_q + 255) / 256, static_cast<int64_t>(batch) * heads_q,
-                                is_causal == 1 ? seqlen_k / 2 : seqlen_k);
+  int variant = forward_variant(kdim, seqlen_q, (seqlen_q + 255) / 256, (seqlen_q + 127) / 128,
+                                static_cast<int64_t>(batch) * heads_q, is_causal == 1 ? seqlen_k / 2 : seqlen_k,
+                                is_causal != 0);
   p.kv_splits = 1;
   // (the kernel instances of the top-left mask carry no code for a share of the keys; a variant forced by
   // fal_set_fwd_variant runs as it was asked for)
@@ -506,8 +533,8 @@ int fal_fwd_varlen(const void* q, const void* k, const void* v, void* o, float* 
   // The lengths stay on the device.  Every sequence rounds up to whole query blocks: at most one
   // extra block each.
   const int kdim = kernel_head_dim(head_dim);
-  const int variant = forward_variant(kdim, total_q / 256 + num_seqs, heads_q,
-                                      total_k / num_seqs / (is_causal == 1 ? 2 : 1));
+  const int variant = forward_variant(kdim, 0, total_q / 256 + num_seqs, total_q / 128 + num_seqs, heads_q,
+                                      total_k / num_seqs / (is_causal == 1 ? 2 : 1), is_causal != 0);
   p.half_sm = variant == FAL_FWD_HALF_SM;
   p.cta_rows = variant == FAL_FWD_TWO_TILES ? 256 : 128;
   p.num_qblk = total_q / p.cta_rows + num_seqs;
