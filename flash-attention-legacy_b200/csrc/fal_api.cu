@@ -259,39 +259,43 @@ BwdWorkspace bwd_workspace_layout(int batch, int heads_q, int rows, int head_dim
 // 0.081 ms per step against 0.089 with 2 048 or with 512); once the batch alone fills the GPU many
 // times over, 2 048 halves the partials and the combine work (64 entries of up to 32 768 positions:
 // 0.714 against 0.745 ms per step).
-constexpr int kDecodeSplitLen = 1024;
-int decode_split_len(int batch, int capacity) {
-  const int64_t long_splits = static_cast<int64_t>(batch) * ((capacity + 2 * kDecodeSplitLen - 1) / (2 * kDecodeSplitLen));
-  return long_splits >= 192 ? 2 * kDecodeSplitLen : kDecodeSplitLen;
+constexpr int kDecodeSplitShift = 10;
+int decode_split_shift(int batch, int capacity) {
+  const int64_t long_splits = static_cast<int64_t>(batch) * (((capacity - 1) >> (kDecodeSplitShift + 1)) + 1);
+  return long_splits >= 192 ? kDecodeSplitShift + 1 : kDecodeSplitShift;
 }
 
 // Decode scratch layout: [partial O fp32 rows*d][partial (max, sum) fp32 rows*2], rows =
 // batch*heads_q*splits.  Nothing in it needs initialising.  (Sized for 1 024-position splits
 // whichever length is used, so the size a caller was told does not depend on the choice.)
-size_t decode_partial_bytes(int batch, int heads_q, int capacity, int head_dim, int split_len) {
-  const int64_t rows = static_cast<int64_t>(batch) * heads_q * ((capacity + split_len - 1) / split_len);
+size_t decode_partial_bytes(int batch, int heads_q, int splits, int head_dim) {
+  const int64_t rows = static_cast<int64_t>(batch) * heads_q * splits;
   return static_cast<size_t>(rows) * (kernel_head_dim(head_dim) + 2) * sizeof(float);
 }
 
-// A grid that leaves SMs without a CTA is bound by the latency of one CTA's chain of slices, not by HBM:
-// splits are halved, down to 256 positions (four 16-key slices for each of the four warps), until there are
-// two CTAs per SM -- as far as the partials fit the workspace.  Only the first 4 MiB of it count, so that
-// the result does not depend on how much more a caller has.  Split-K and combine together, 1 024 positions
-// against 256: 1 entry of 1 999 (32 / 8 heads of 128) 24.4 -> 14.3 us, 8 of 2 049 (32 / 4 of 64) 18.4 -> 14.4,
-// 4 of 4 000 to 8 000 (8 / 1 of 128) 24.6 -> 16.4, 1 of 2 299 (16 / 2 of 256) 31.7 -> 18.4.  128 positions
-// measured 14.3, 16.4, 20.5 and 16.4: the partials then cost what the shorter chains save.
-constexpr int kDecodeMinSplit = 256;
-constexpr int kDecodeCtasPerSm = 2;
+// A grid that leaves SMs without work is bound by the latency of one CTA's chain of slices, not by HBM: an entry is
+// then cut finer, down to 256 positions (four 16-key slices for each of the four warps), as long as all CTAs still
+// run at once.  Only the GPU knows the lengths, so the kernels choose (decode_split_shift); this gives them the number
+// of splits per entry up to which a finer cut is taken: what the SMs hold (one CTA per SM at head_dim 256, two at 128,
+// four at 64: their shared memory) over the (entry, KV head) pairs, as far as the partials fit the workspace.  Only
+// the first 4 MiB of that count, so that the result does not depend on how much more a caller has.
+// us on the GPU with 256 / 512 / 1 024 positions a split (the choice in brackets), 8 KV heads of 128, capacity 8 192:
+// 4 entries of 983 [11.5] / 14.2 / 17.3, 2 048 [12.9] / 14.8 / 22.2, 4 096 18.6 / [16.0] / 22.4, 8 191 37.1 / 30.9 / [27.3];
+// 1 entry (capacity 32 768) of 8 192 [12.2] / 14.8 / 17.9, 16 384 20.0 / [15.9] / 18.2, 32 767 42.3 / 33.3 / [28.4];
+// 2 entries of 16 KV heads of 256: 983 [13.6] / 16.1 / 24.3, 4 096 37.4 / 30.9 / [27.2], 8 191 69.3 / 59.2 / [51.5]; 4 of 16 of 64:
+// 2 048 [11.6] / 12.5 / 14.6, 4 096 16.6 / [15.2] / 18.4, 8 191 32.2 / 28.5 / [27.9].  128 positions are slower almost throughout.
+// With one length for all entries, by the capacity, full caches ran in two waves of CTAs (30.8 and 58.8 us in the
+// first and third of these rows) and short texts in large caches in one CTA each.
 constexpr size_t kDecodeFineBytes = size_t{4} << 20;
-int decode_split_len_for(int batch, int heads_q, int heads_kv, int capacity, int head_dim, size_t workspace_bytes) {
-  int len = decode_split_len(batch, capacity);
+int decode_fine_splits(int batch, int heads_q, int heads_kv, int capacity, int head_dim, size_t workspace_bytes) {
   const int64_t units = static_cast<int64_t>(batch) * heads_kv * ((heads_q / heads_kv + 15) / 16);
-  const int64_t want = kDecodeCtasPerSm * static_cast<int64_t>(sm_count() > 0 ? sm_count() : 148);
+  const int64_t sms = sm_count() > 0 ? sm_count() : 148;
+  const int64_t at_once = sms * 256 / kernel_head_dim(head_dim) / units;
   const size_t room = workspace_bytes < kDecodeFineBytes ? workspace_bytes : kDecodeFineBytes;
-  while (len > kDecodeMinSplit && units * ((capacity + len - 1) / len) < want &&
-         decode_partial_bytes(batch, heads_q, capacity, head_dim, len / 2) <= room)
-    len /= 2;
-  return len;
+  const int64_t fit = static_cast<int64_t>(room / decode_partial_bytes(batch, heads_q, 1, head_dim));
+  int64_t splits = ((capacity - 1) >> fal::kDecodeFinestShift) + 1;
+  if (splits > at_once) splits = at_once;
+  return static_cast<int>(splits < fit ? splits : fit);
 }
 
 // ---------------------------------------------------------------------------
@@ -862,7 +866,7 @@ int fal_scale_cast_f16(void* dst, const float* src, int batch, int heads, int ro
 
 size_t fal_decode_workspace_bytes(int batch, int heads_q, int capacity, int head_dim) {
   if (batch <= 0 || heads_q <= 0 || capacity <= 0 || head_dim <= 0) return 0;
-  return decode_partial_bytes(batch, heads_q, capacity, head_dim, kDecodeSplitLen);
+  return decode_partial_bytes(batch, heads_q, ((capacity - 1) >> kDecodeSplitShift) + 1, head_dim);
 }
 
 namespace {
@@ -898,7 +902,7 @@ int decode_with_workspace(const void* q, void* k_cache, void* v_cache, const fal
   if (rc != FAL_OK) return rc;
   if (!workspace) return FAL_ERR_INVALID_ARGUMENT;
   if ((reinterpret_cast<uintptr_t>(workspace) & 15u) != 0) return FAL_ERR_INVALID_ARGUMENT;
-  if (workspace_bytes < decode_partial_bytes(batch, heads_q, capacity, head_dim, kDecodeSplitLen))
+  if (workspace_bytes < fal_decode_workspace_bytes(batch, heads_q, capacity, head_dim))
     return FAL_ERR_WORKSPACE_TOO_SMALL;
   rc = check_device();
   if (rc != FAL_OK) return rc;
@@ -921,8 +925,10 @@ int decode_with_workspace(const void* q, void* k_cache, void* v_cache, const fal
   p.capacity = capacity;
   p.head_dim = kernel_head_dim(head_dim);
   p.head_dim_real = head_dim;
-  p.split_len = decode_split_len_for(batch, heads_q, heads_kv, capacity, head_dim, workspace_bytes);
-  p.splits = (capacity + p.split_len - 1) / p.split_len;
+  p.split_shift = decode_split_shift(batch, capacity);
+  p.fine_splits = decode_fine_splits(batch, heads_q, heads_kv, capacity, head_dim, workspace_bytes);
+  p.splits = ((capacity - 1) >> p.split_shift) + 1;
+  if (p.splits < p.fine_splits) p.splits = p.fine_splits;
   p.scale = softmax_scale;
   p.status = status;
   p.part_o = static_cast<float*>(workspace);

@@ -9,8 +9,8 @@
 //
 // The pass is bound by HBM bandwidth (4 flops per cache byte), so the kernel is
 // organised around keeping 16-byte loads in flight:
-//   - grid (kv_head x head-chunk, split, batch); each CTA streams `split_len`
-//     cache positions of one KV head exactly once for all the query heads that
+//   - grid (kv_head x head-chunk, split, batch); each CTA streams a split (256
+//     to 2 048 cache positions, by the entry's length) of one KV head exactly once for all the query heads that
 //     share it (up to 16 per CTA);
 //   - every warp runs its own cp.async pipeline over interleaved 16-key slices
 //     (no block-level barrier inside the main loop), shared memory XOR-swizzled
@@ -101,6 +101,13 @@ __device__ __forceinline__ DecodeRange decode_range(const DecodeParams& p, int b
   return r;
 }
 
+// log2 of the positions per split of an entry of `len`: the finest cut that leaves it with no more than fine_splits.
+__device__ __forceinline__ int decode_split_shift(const DecodeParams& p, int len) {
+  int shift = kDecodeFinestShift;
+  while (shift < p.split_shift && ((len - 1) >> shift) + 1 > p.fine_splits) ++shift;
+  return shift;
+}
+
 template <int D>
 struct DecSmem {
   static constexpr int kRowBytes = D * 2;
@@ -137,7 +144,8 @@ fal_decode_splitk_kernel(const DecodeParams p) {
   const bool can_append = rg.can_append;
   if (p.k_new != nullptr && !can_append && split == 0 && blockIdx.x == 0 && threadIdx.x == 0 && p.status)
     atomicCAS(p.status, 0, kDevAppendOverflow);
-  const int pos0 = split * p.split_len;
+  const int split_shift = decode_split_shift(p, len);
+  const int pos0 = split << split_shift;
 
   const int rows_valid = min(16, group - head_chunk * 16);
   const int hq0 = kv_head * group + head_chunk * 16;  // first query head of this CTA
@@ -146,7 +154,7 @@ fal_decode_splitk_kernel(const DecodeParams p) {
   // other (split 0 stores it when the position lies before `start` and nobody attends to it) ----
   if (can_append) {
     const int new_local = len_old - start;
-    const int store_split = new_local >= 0 ? new_local / p.split_len : 0;
+    const int store_split = new_local >= 0 ? new_local >> split_shift : 0;
     if (split == store_split) {
       const int real_chunks = p.head_dim_real / 8;  // head_dim 32 / 96 run on the 64 / 128 kernels
       for (int c = threadIdx.x; c < 2 * real_chunks; c += kDecThreads) {
@@ -164,7 +172,7 @@ fal_decode_splitk_kernel(const DecodeParams p) {
     }
   }
   if (pos0 >= len) return;  // this split lies beyond the sequence
-  const int pos_end = min(pos0 + p.split_len, len);
+  const int pos_end = min(pos0 + (1 << split_shift), len);
   const int num_slices = (pos_end - pos0 + kSliceKeys - 1) / kSliceKeys;
 
   const int warp = threadIdx.x >> 5;
@@ -363,12 +371,18 @@ fal_decode_splitk_kernel(const DecodeParams p) {
 // ---------------------------------------------------------------------------
 // Combine: merge the splits a sequence actually reaches.
 // ---------------------------------------------------------------------------
-// One block per (batch, head).  The statistics of all splits are reduced by the whole block at once and
-// the partial rows are summed by groups of D / 4 threads (16-byte loads), a split each: with one thread
+// WARPS warps per (batch, head), blocks of four warps.  The statistics of all splits are reduced by all lanes at
+// once and the partial rows are summed by groups of D / 4 threads (16-byte loads), a split each: with one thread
 // per column walking every split three times the kernel took 4.8 us at 2 splits, most of it exposed
 // load latency that grows with the number of splits.
+// Four warps per row where a row's partials are many, one where they are few and the rows make the grid large.
+// Whole decode step, four against one, us: 64 x 32 heads of 64, 4 splits 8.7 / 7.0 (12 positions) and 50.5 / 49.5
+// (4 095); 256 x 32 of 128, 1 split 36.5 / 30.0; 8 x 32 of 64, 9 splits 8.2 / 8.0; 1 x 32 of 128, 16 splits 9.1 / 10.8;
+// 4 x 32 of 128, 32 splits 93.1 / 101.3; 1 x 8 of 64, 64 splits 8.8 / 13.2.
 // It is launched while the split-K grid still runs and waits here for that grid's results.
 constexpr int kCombineThreads = 128;
+constexpr int kCombineWarpBytes = 2048;  // of partials of a row, up to which one warp merges them;
+constexpr int kCombineManyRows = 256;    // twice as many in a grid of this many rows
 
 // (m, l) <- the merge with another running maximum and sum (log2 domain).
 __device__ __forceinline__ void merge_stats(float& m, float& l, float m2, float l2) {
@@ -378,24 +392,32 @@ __device__ __forceinline__ void merge_stats(float& m, float& l, float m2, float 
   m = m_new;
 }
 
-template <int D>
+template <int D, int WARPS>
 __global__ void __launch_bounds__(kCombineThreads)
 fal_decode_combine_kernel(const DecodeParams p) {
-  constexpr int kLanes = D / 4;                        // threads per partial row
-  constexpr int kGroups = kCombineThreads / kLanes;    // rows in flight
-  __shared__ float2 warp_ml[kCombineThreads / 32];
+  static_assert(WARPS == 1 || WARPS * 32 == kCombineThreads, "a row per warp or per block");
+  constexpr int kRows = kCombineThreads / (32 * WARPS);      // (batch, head) rows per block
+  constexpr int kThreads = 32 * WARPS;                       // threads per row
+  constexpr int kLanes = D / 4 < kThreads ? D / 4 : kThreads;  // threads per partial row
+  constexpr int kVecs = D / (4 * kLanes);                    // 16-byte pieces of it per thread
+  constexpr int kGroups = kThreads / kLanes;                 // partial rows in flight
+  __shared__ float2 warp_ml[WARPS];
   __shared__ float4 part[kGroups][kLanes];
-  const int bh = blockIdx.x;
-  const int b = bh / p.heads_q;
-  const int tid = threadIdx.x;
-  const int len = decode_range(p, b).len;
-  const int n = (len + p.split_len - 1) / p.split_len;
+  const int tid = threadIdx.x % kThreads;
+  const int bh = blockIdx.x * kRows + threadIdx.x / kThreads;
+  const bool row_ok = bh < p.batch * p.heads_q;
+  int n = 0;
+  if (row_ok) {
+    const int len = decode_range(p, bh / p.heads_q).len;
+    n = ((len - 1) >> decode_split_shift(p, len)) + 1;  // (an empty entry: (-1 >> shift) + 1 = 0)
+  }
   const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + static_cast<int64_t>(bh) * p.splits;
-  const float4* po = reinterpret_cast<const float4*>(p.part_o) + static_cast<int64_t>(bh) * p.splits * kLanes;
+  const float4* po = reinterpret_cast<const float4*>(p.part_o) + static_cast<int64_t>(bh) * p.splits * (D / 4);
   grid_dependency_wait();
+  if (!row_ok) return;  // (whole warps; a block of one row has that row)
 
   float m = kNegInfD, l = 0.f;
-  for (int i = tid; i < n; i += kCombineThreads) {
+  for (int i = tid; i < n; i += kThreads) {
     const float2 x = ml[i];
     merge_stats(m, l, x.x, x.y);
   }
@@ -405,42 +427,66 @@ fal_decode_combine_kernel(const DecodeParams p) {
     const float l2 = __shfl_xor_sync(0xffffffffu, l, off);
     merge_stats(m, l, m2, l2);
   }
-  if ((tid & 31) == 0) warp_ml[tid >> 5] = make_float2(m, l);
-  __syncthreads();
-  m = warp_ml[0].x;
-  l = warp_ml[0].y;
+  if constexpr (WARPS > 1) {
+    if ((tid & 31) == 0) warp_ml[tid >> 5] = make_float2(m, l);
+    __syncthreads();
+    m = warp_ml[0].x;
+    l = warp_ml[0].y;
 #pragma unroll
-  for (int w = 1; w < kCombineThreads / 32; ++w) merge_stats(m, l, warp_ml[w].x, warp_ml[w].y);
+    for (int w = 1; w < WARPS; ++w) merge_stats(m, l, warp_ml[w].x, warp_ml[w].y);
+  }
   const float muse = (m == kNegInfD) ? 0.f : m;
   const float inv = l > 0.f ? 1.f / l : 0.f;
 
   const int lane = tid % kLanes;
   const int grp = tid / kLanes;
-  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 o[kVecs];
+#pragma unroll
+  for (int v = 0; v < kVecs; ++v) o[v] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
   for (int i = grp; i < n; i += kGroups) {
     const float w = fast_exp2(ml[i].x - muse);
-    const float4 x = po[static_cast<int64_t>(i) * kLanes + lane];
-    o.x += w * x.x;
-    o.y += w * x.y;
-    o.z += w * x.z;
-    o.w += w * x.w;
-  }
-  part[grp][lane] = o;
-  __syncthreads();
-  if (grp == 0 && lane * 4 < p.head_dim_real) {
 #pragma unroll
-    for (int g = 1; g < kGroups; ++g) {
-      const float4 x = part[g][lane];
-      o.x += x.x;
-      o.y += x.y;
-      o.z += x.z;
-      o.w += x.w;
+    for (int v = 0; v < kVecs; ++v) {
+      const float4 x = po[static_cast<int64_t>(i) * (D / 4) + v * kLanes + lane];
+      o[v].x += w * x.x;
+      o[v].y += w * x.y;
+      o[v].z += w * x.z;
+      o[v].w += w * x.w;
     }
-    uint2 out;
-    out.x = pack_half2(o.x * inv, o.y * inv);
-    out.y = pack_half2(o.z * inv, o.w * inv);
-    *reinterpret_cast<uint2*>(static_cast<__half*>(p.o) + static_cast<int64_t>(bh) * p.head_dim_real + lane * 4) = out;
+  }
+  auto add = [&](float4& a, const float4& x) {
+    a.x += x.x;
+    a.y += x.y;
+    a.z += x.z;
+    a.w += x.w;
+  };
+  if constexpr (WARPS > 1) {
+    static_assert(kVecs == 1, "one piece per thread");
+    part[grp][lane] = o[0];
+    __syncthreads();
+    if (grp == 0) {
+#pragma unroll
+      for (int g = 1; g < kGroups; ++g) add(o[0], part[g][lane]);
+    }
+  } else {
+#pragma unroll
+    for (int off = kLanes; off < 32; off <<= 1) {  // (one piece per thread then)
+      const float4 x = make_float4(__shfl_xor_sync(0xffffffffu, o[0].x, off), __shfl_xor_sync(0xffffffffu, o[0].y, off),
+                                   __shfl_xor_sync(0xffffffffu, o[0].z, off), __shfl_xor_sync(0xffffffffu, o[0].w, off));
+      add(o[0], x);
+    }
+  }
+  __half* out_row = static_cast<__half*>(p.o) + static_cast<int64_t>(bh) * p.head_dim_real;
+#pragma unroll
+  for (int v = 0; v < kVecs; ++v) {
+    const int col = (v * kLanes + lane) * 4;
+    if (grp == 0 && col < p.head_dim_real) {
+      uint2 out;
+      out.x = pack_half2(o[v].x * inv, o[v].y * inv);
+      out.y = pack_half2(o[v].z * inv, o[v].w * inv);
+      *reinterpret_cast<uint2*>(out_row + col) = out;
+    }
   }
   if (p.lse != nullptr && tid == 0) p.lse[bh] = (l > 0.f) ? (m + log2f(l)) * 0.6931471805599453f : kNegInfD;
 }
@@ -537,10 +583,16 @@ cudaError_t launch_cache_append(const CacheAppendParams& p, cudaStream_t stream)
 }
 
 cudaError_t launch_decode_combine(const DecodeParams& p, cudaStream_t stream) {
-  const dim3 grid(p.batch * p.heads_q), block(kCombineThreads);
-  if (p.head_dim == 128) return launch_dependent(fal_decode_combine_kernel<128>, grid, block, 0, stream, p);
-  if (p.head_dim == 64) return launch_dependent(fal_decode_combine_kernel<64>, grid, block, 0, stream, p);
-  if (p.head_dim == 256) return launch_dependent(fal_decode_combine_kernel<256>, grid, block, 0, stream, p);
+  const int rows = p.batch * p.heads_q;
+  const dim3 block(kCombineThreads);
+  auto launch = [&](auto by_warp, auto by_block) {
+    const int most = rows >= kCombineManyRows ? 2 * kCombineWarpBytes : kCombineWarpBytes;
+    return p.splits * p.head_dim * 4 <= most ? launch_dependent(by_warp, dim3((rows + 3) / 4), block, 0, stream, p)
+                                             : launch_dependent(by_block, dim3(rows), block, 0, stream, p);
+  };
+  if (p.head_dim == 128) return launch(fal_decode_combine_kernel<128, 1>, fal_decode_combine_kernel<128, 4>);
+  if (p.head_dim == 64) return launch(fal_decode_combine_kernel<64, 1>, fal_decode_combine_kernel<64, 4>);
+  if (p.head_dim == 256) return launch(fal_decode_combine_kernel<256, 1>, fal_decode_combine_kernel<256, 4>);
   return cudaErrorInvalidValue;
 }
 

@@ -140,6 +140,8 @@ cudaError_t launch_scale_cast(const ScaleCastParams& p, cudaStream_t stream);
 
 // Decode over a KV cache: split-K streaming pass (which also appends the new row), then the
 // log-sum-exp combine.
+constexpr int kDecodeFinestShift = 8;  // log2 of the positions of the finest split
+
 struct DecodeParams {
   const void* q;        // [batch, heads_q, head_dim] fp16, contiguous
   void* k_cache;        // fp16
@@ -160,8 +162,9 @@ struct DecodeParams {
   int capacity;         // cache positions per batch entry
   int head_dim;         // kernel head_dim (64, 128, 256): row length of the partial results
   int head_dim_real;    // the tensors' head_dim (32 and 96 run on the 64 / 128 kernels)
-  int split_len;        // positions per split (multiple of the key tile)
-  int splits;           // ceil(capacity / split_len)
+  int split_shift;      // log2 of the positions per split of an entry that is not cut finer
+  int fine_splits;      // an entry is cut finer as long as it has no more splits than this
+  int splits;           // most splits an entry can have: the larger of fine_splits and those of a full cache
   float scale;
   int* status;
 };

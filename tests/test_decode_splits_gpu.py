@@ -40,3 +40,32 @@ def test_small_batches_against_the_oracle(ext, hq, hkv, d, lens, capacity):
     out = torch.empty_like(o)
     assert torch.equal(ext.decode_static(*args, out=out), o)
     assert ext.device_status() == 0
+
+
+# Entries on both sides of where a cut gets coarser, in one call (batch x KV heads leave 3 to 30 splits per entry to
+# the SMs); the new token in the last position of a split and in the first of the next; one warp and one block per row
+# of the merge, and a number of rows that is not a multiple of four.
+@pytest.mark.parametrize("hq,hkv,d", [(8, 8, 128), (6, 2, 64), (9, 3, 256), (4, 1, 32), (32, 8, 96)])
+@pytest.mark.parametrize("append", [False, True])
+@pytest.mark.parametrize("capacity", [9216, 2500])
+def test_cuts_of_different_fineness_in_one_batch(ext, hq, hkv, d, append, capacity):
+    gen = torch.Generator().manual_seed(hq * d)
+    lens = [n for n in (0, 1, 255, 256, 767, 768, 769, 1024, 1535, 1536, 1537, 2304, 3072, 3073, 4607, 4608, 6143, 6145, 9215)
+            if n < capacity]
+    b, scale = len(lens), 1 / math.sqrt(d)
+    q = torch.randn(b, hq, d, generator=gen).half()
+    kc, vc = (torch.randn(b, capacity, hkv, d, generator=gen).half() for _ in range(2))
+    kn, vn = (torch.randn(b, hkv, d, generator=gen).half() for _ in range(2)) if append else (None, None)
+    lens = torch.tensor(lens, dtype=torch.int32)
+    dev = [t.cuda() if t is not None else None for t in (q, kc, vc, lens, kn, vn)]
+    o, lse = ext.decode(*dev[:4], scale, k_new=dev[4], v_new=dev[5], return_lse=True)
+    if append:
+        for i, n in enumerate(lens.tolist()):
+            kc[i, n], vc[i, n] = kn[i], vn[i]
+        assert torch.equal(dev[1].cpu(), kc) and torch.equal(dev[2].cpu(), vc)
+        lens = lens + 1
+    o_ref, lse_ref = orc.decode_fwd(q, kc, vc, lens, scale)
+    assert orc.rel_max_err(o, o_ref) <= orc.TOL_O
+    seen = lens > 0
+    assert orc.abs_max_err(lse.cpu()[seen], lse_ref[seen]) <= orc.TOL_LSE
+    assert ext.device_status() == 0
