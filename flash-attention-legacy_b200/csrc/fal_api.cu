@@ -579,7 +579,29 @@ struct BwdCall {
   float* dk_f32 = nullptr;
   float* dv_f32 = nullptr;
   fal::RowStrides s_dq_acc{};
+  int longest_q = 0;  // packed: the caller's bound on a sequence's rows (0: rows_q); only the order of blocks depends on it
 };
+
+// (batch, KV head) groups whose CTAs are handed out in turn.  The CTAs of a group share Q, dO and the dQ accumulator
+// through L2 while they stay near each other; on long rows they drift apart, and with eight groups in turn it depended
+// on chance (on which buffers the call got) whether they all found their way back: when they did not, every tile came
+// from DRAM.  Two groups at a time do not drift that far.  ms of this kernel over six or seven calls with fresh buffers,
+// eight groups at a time / two (heads of 128, causal): 32 / 8 heads x 131 072 rows 340 - 500 / 331 - 334, 98 304 rows
+// 190 - 276 / 187 - 188, 80 000 rows 125 - 176 / 122 - 125; 65 536 rows 81 - 84 / 83 - 86; without a mask 131 072 rows
+// 687 - 888 / 664 - 668.  A narrow wave costs short rows up to 8 % (4 x 32 / 8 x 4 096 1.56 / 1.68), so it is taken where Q,
+// dO and dQ of eight groups come to more than 2 GiB: none of the shapes up to there showed the two speeds.
+constexpr int kBwdWaveGroups = 8;
+constexpr int kBwdLongWaveGroups = 2;
+constexpr int64_t kBwdLongBytes = int64_t{1} << 31;
+int bwd_wave_groups(const BwdCall& c, int kdim) {
+  const bool packed = c.cu_k != nullptr;
+  const int64_t rows = packed && c.longest_q > 0 && c.longest_q < c.rows_q ? c.longest_q : c.rows_q;
+  const int64_t group_bytes = rows * (c.heads_q / c.heads_kv) * kdim * 8;
+  // packed sequences are short as a rule: all KV heads of a key block in turn
+  int64_t groups = packed ? c.heads_kv : static_cast<int64_t>(c.batch) * c.heads_kv;
+  if (!packed && groups > kBwdWaveGroups) groups = kBwdWaveGroups;
+  return static_cast<int>(groups * group_bytes > kBwdLongBytes ? kBwdLongWaveGroups : groups);
+}
 
 int run_bwd(const BwdCall& c) {
   const bool partial = c.dq_acc != nullptr;
@@ -681,6 +703,7 @@ int run_bwd(const BwdCall& c) {
   p.seqlen_q = c.cu_q ? 0 : c.rows_q;
   p.seqlen_k = c.cu_k ? 0 : c.rows_k;
   p.num_kvblk = c.cu_k ? (c.rows_k / 128 + c.num_seqs) : (c.rows_k + 127) / 128;
+  p.wave_groups = bwd_wave_groups(c, kdim);
   p.causal_shift = (c.causal == FAL_CAUSAL_BOTTOM_RIGHT && !c.cu_k) ? c.rows_k - c.rows_q : 0;
   p.shift_per_sequence = (c.causal == FAL_CAUSAL_BOTTOM_RIGHT && c.cu_k) ? 1 : 0;
   p.scale = c.scale;
@@ -750,7 +773,6 @@ int fal_bwd_varlen(const void* d_out, const void* q, const void* k, const void* 
                    const fal_strides* dk_strides, const fal_strides* dv_strides,
                    float softmax_scale, int is_causal, void* workspace, size_t workspace_bytes,
                    int* status, void* stream) {
-  (void)max_seqlen_q;
   (void)max_seqlen_k;
   if (!do_strides || !q_strides || !k_strides || !v_strides || !o_strides || !dq_strides ||
       !dk_strides || !dv_strides || !cu_seqlens_q || !cu_seqlens_k || num_seqs <= 0)
@@ -761,6 +783,7 @@ int fal_bwd_varlen(const void* d_out, const void* q, const void* k, const void* 
   c.cu_q = cu_seqlens_q; c.cu_k = cu_seqlens_k; c.num_seqs = num_seqs;
   c.batch = 1; c.heads_q = heads_q; c.heads_kv = heads_kv;
   c.rows_q = total_q; c.rows_k = total_k; c.head_dim = head_dim;
+  c.longest_q = max_seqlen_q;
   auto packed = [](const fal_strides* s) { return fal::RowStrides{0, s->head, s->row}; };
   c.s_do = packed(do_strides); c.s_q = packed(q_strides); c.s_k = packed(k_strides);
   c.s_v = packed(v_strides); c.s_o = packed(o_strides); c.s_dq = packed(dq_strides);

@@ -130,21 +130,16 @@ struct BwdWork {
   int seqlen_k;
 };
 
-#ifndef FAL_BWD_WAVE_GROUPS
-#define FAL_BWD_WAVE_GROUPS 8
-#endif
-constexpr int kWaveGroups = FAL_BWD_WAVE_GROUPS;
-
 __device__ __forceinline__ bool bwd_decode_work(const BwdParams& p, int idx, BwdWork& w) {
   if (p.cu_k == nullptr) {
-    // CTAs are numbered in waves of up to kWaveGroups (batch, KV head) groups; inside a wave the first key
+    // CTAs are numbered in waves of up to p.wave_groups (batch, KV head) groups; inside a wave the first key
     // blocks come first (under a causal mask they see the most queries).  The CTAs that run at the
     // same time then add into the fp32 dQ accumulators of a few groups only (8 MB per group at
     // 4 heads x 4096 rows), which stay in L2 between the 32 key tiles that touch them.
     const int bh_count = p.batch * p.heads_kv;
     const int nkvblk = (p.seqlen_k + kKvTile - 1) / kKvTile;
-    // equal waves of at most kWaveGroups groups (a short last wave leaves SMs idle at the end)
-    const int num_waves = (bh_count + kWaveGroups - 1) / kWaveGroups;
+    // equal waves (a short last wave leaves SMs idle at the end)
+    const int num_waves = (bh_count + p.wave_groups - 1) / p.wave_groups;
     const int wave_groups = (bh_count + num_waves - 1) / num_waves;
     const int wave = idx / (wave_groups * nkvblk);
     const int first_group = wave * wave_groups;
@@ -160,8 +155,15 @@ __device__ __forceinline__ bool bwd_decode_work(const BwdParams& p, int idx, Bwd
     w.seqlen_k = p.seqlen_k;
     return true;
   }
-  const int slot = idx / p.heads_kv;
-  w.kv_head = idx % p.heads_kv;
+  // Packed: sequence by sequence, every key block for all KV heads in turn, or for p.wave_groups of them at a time.
+  const int num_waves = (p.heads_kv + p.wave_groups - 1) / p.wave_groups;
+  const int wave_groups = (p.heads_kv + num_waves - 1) / num_waves;
+  const int wave = idx / (wave_groups * p.num_kvblk);
+  const int first_head = wave * wave_groups;
+  const int heads_here = min(wave_groups, p.heads_kv - first_head);
+  const int r = idx - wave * wave_groups * p.num_kvblk;
+  const int slot = r / heads_here;
+  w.kv_head = first_head + r % heads_here;
   w.batch = 0;
   // Which sequence owns key block `slot`: every warp scans the lengths 32 sequences at a time (one
   // coalesced load, a prefix sum of the block counts, a vote) instead of walking them one by one.
@@ -230,7 +232,7 @@ __device__ __forceinline__ void red_add_v4(float* dst, const uint32_t (&v)[4]) {
 
 // Adds 16 rows of a dQ tile to the accumulator rows at `rows` (row_floats apart; the first `valid` of them).
 // r[c][4 k + 0, 1]: columns 64 c + 8 k + 2 (lane % 4) + {0, 1} of row lane / 4; r[c][4 k + 2, 3]: of row
-// lane / 4 + 8.  Lanes trade registers until an instruction covers RED_SHAPE
+// lane / 4 + 8.  Lane pairs trade registers so that an instruction covers 64 contiguous bytes of each of 8 rows.
 template <int D>
 __device__ __forceinline__ void dq_reduce(float* rows, int row_floats, const uint32_t (&r)[D / 64][32], int valid) {
   const int lane = threadIdx.x & 31;

@@ -90,6 +90,7 @@ struct BwdParams {
   int seqlen_k;
   int head_dim;   // the tensors' head_dim (32 / 96 run on the 64 / 128 kernels); dK, dV columns beyond it are not written
   int num_kvblk;  // batched: ceil(seqlen_k / 128); packed: bound over all sequences
+  int wave_groups;         // (batch, KV head) groups whose key blocks are numbered in turn
   int causal_shift;        // causal, batched: query row i sees keys <= i + causal_shift (0: top-left aligned mask)
   int shift_per_sequence;  // causal, packed: the shift of a sequence is its seqlen_k - seqlen_q
   float scale;

@@ -251,7 +251,7 @@ __device__ __forceinline__ bool fwd_decode_work(const FwdParams& p, FwdWork& w) 
     if (SHIFTED && p.heaviest_first != 0) {
       // Entries of 1 500 and of 8 000 keys in one grid: in the order above the longest entry's last blocks
       // start late and the SMs wait for them.  Heaviest first, 4 entries x 1 024 queries (32 / 8 heads of 128)
-      // behind 512 to 7 000 keys: 329 -> 310 us a call; the search costs a CTA well under a microsecond.
+      // behind 512 to 7 000 keys: 297 -> 281 us on the GPU; the search costs a CTA about half a microsecond.
       fwd_heaviest_block<ROWS>(p, idx / p.heads_q, w.batch, w.qblk);
     }
     w.q_row0 = 0;
