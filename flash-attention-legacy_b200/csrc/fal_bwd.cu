@@ -309,7 +309,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sgen + L::kMiscOff + 4);
   const WaitCtx wctx{abort_flag, p.status};
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   const int group = p.heads_q / p.heads_kv;
@@ -360,7 +360,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   if (warp == 8) {
     // ===================== producer: TMA ======================================
     if constexpr (SPLIT) {
-      if (lane == 0 && n_iter > 0) {
+      if (n_iter > 0 && elect_one()) {
         tma_prefetch_desc(&tm_q);
         tma_prefetch_desc(&tm_k);
         tma_prefetch_desc(&tm_v);
@@ -407,7 +407,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       }
       __syncwarp();
     } else {
-      if (lane == 0 && n_iter > 0) {
+      if (n_iter > 0 && elect_one()) {
         tma_prefetch_desc(&tm_q);
         tma_prefetch_desc(&tm_k);
         tma_prefetch_desc(&tm_v);
@@ -421,29 +421,24 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         for (int bx = 0; bx < L::kBoxes; ++bx)
           tma_load_4d(sbase + L::kVOff + bx * L::kBoxBytes, &tm_v, bar(iVFull), bx * 64,
                       wk.k_row0 + kv0, wk.kv_head, wk.batch);
-      }
-      for (int i = 0; i < n_iter; ++i) {
-        const int st = i % NS;
-        const int head = wk.kv_head * group + i / nq;
-        const int qt = qt0 + i % nq;
-        const int row = wk.q_row0 + qt * kQTile;
-        if (i >= NS) mbar_wait(bar(iQEmpty + st), ((i / NS) - 1) & 1, wctx, kBbQEmpty + st);
-        if (lane == 0) {
+        for (int i = 0; i < n_iter; ++i) {
+          const int st = i % NS;
+          const int head = wk.kv_head * group + i / nq;
+          const int row = wk.q_row0 + (qt0 + i % nq) * kQTile;
+          if (i >= NS) mbar_wait(bar(iQEmpty + st), ((i / NS) - 1) & 1, wctx, kBbQEmpty + st);
           mbar_arrive_expect_tx(bar(iQFull + st), L::kTileBytes);
           for (int bx = 0; bx < L::kBoxes; ++bx)
             tma_load_4d(sbase + L::kQOff + st * L::kTileBytes + bx * L::kBoxBytes, &tm_q,
                         bar(iQFull + st), bx * 64, row, head, wk.batch);
-        }
-        // dO has a single buffer: it is reloaded as soon as dV of the previous step has read it.
-        if (lane == 0) {
+          // dO has a single buffer: it is reloaded as soon as dV of the previous step has read it.
           if (i >= 1) mbar_wait(bar(iDoEmpty), (i - 1) & 1, wctx, kBbDoEmpty);
           mbar_arrive_expect_tx(bar(iDoFull), L::kTileBytes);
           for (int bx = 0; bx < L::kBoxes; ++bx)
             tma_load_4d(sbase + L::kDoOff + bx * L::kBoxBytes, &tm_do, bar(iDoFull), bx * 64, row, head,
                         wk.batch);
         }
-        __syncwarp();
       }
+      __syncwarp();
     }
   } else if (warp == 14) {
     // ===================== per-row statistics: lse * log2(e) and delta ========
@@ -473,7 +468,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     }
   } else if (warp == 9) {
     // ===================== MMA issuer =========================================
-    if (lane == 0 && n_iter > 0) {
+    if (n_iter > 0 && elect_one()) {
       constexpr uint32_t idesc_st = make_idesc_f16(kKvTile, kQTile, 0, 0);   // S^T, dP^T
       constexpr uint32_t idesc_dkv = make_idesc_f16(kKvTile, D, 0, 1);       // dV, dK
       constexpr uint32_t idesc_dq = make_idesc_f16(kQTile, D, 1, 1);         // dQ = dS K (queries on lanes)
@@ -777,7 +772,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     if (by_tma) {  // uniform over the CTA
       fence_proxy_async_smem();
       named_barrier_sync(2 + half, 128);
-      if (quarter == 0 && lane == 0) {
+      if (quarter == 0 && elect_one()) {
         const uint32_t src = sbase + (is_dk ? L::kKOff : L::kVOff);
         for (int bx = 0; bx < L::kBoxes; ++bx)
           tma_store_4d(is_dk ? &tm_dk : &tm_dv, src + bx * L::kBoxBytes, col_own + bx * 64, wk.k_row0 + kv0,
@@ -849,7 +844,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
         for (int c = 0; c < kGroups; ++c) {
           const uint32_t box = (c & 1) * kDqBoxBytes;
-          if (lane == 0) bulk_wait_group_read<1>();  // the box's last reduction has read it
+          if (elect_one()) bulk_wait_group_read<1>();  // the box's last reduction has read it
           __syncwarp();
 #pragma unroll
           for (int v = 0; v < 8; ++v)
@@ -858,7 +853,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                            r[c % kAhead][4 * v + 3]);
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) {
+          if (elect_one()) {
             tma_reduce_add_4d(&tm_dq, sbase + box_off + box, c * 32, grow, head, wk.batch);
             bulk_commit_group();
           }
@@ -870,7 +865,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           }
         }
       }
-      if (lane == 0) bulk_wait_group0();
+      if (elect_one()) bulk_wait_group0();
     } else {
       // head_dim 64: the tile is 64 columns wide and leaves at once, a row per thread into the two swizzled
       // [128 rows][32 floats] boxes, by two reductions.  (By warps as above 235 -> 254 us on 4 x 16 x 2 048: here
@@ -878,7 +873,6 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       // unit's and the issue slots' time than two.)
       const int qrow = quarter * 32 + lane;
       const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-      const bool issuer = warp == 10 && lane == 0;
       uint8_t* box_row = sgen + L::kStageOff + qrow * 128;
       for (int i = 0; i < n_iter; ++i) {
         const int head = wk.kv_head * group + i / nq;
@@ -897,7 +891,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             mbar_arrive(bar(iDqFree));
           }
           // Earlier reductions must be done reading the staging boxes.
-          if (issuer) bulk_wait_group_read<0>();
+          if (warp == 10 && elect_one()) bulk_wait_group_read<0>();
           named_barrier_sync(1, 128);
 #pragma unroll
           for (int c = 0; c < 2; ++c)
@@ -907,14 +901,14 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                   make_uint4(r[c][4 * v + 0], r[c][4 * v + 1], r[c][4 * v + 2], r[c][4 * v + 3]);
           fence_proxy_async_smem();
           named_barrier_sync(1, 128);
-          if (issuer) {
+          if (warp == 10 && elect_one()) {
             tma_reduce_add_4d(&tm_dq, sbase + L::kStageOff, hf * 64, grow, head, wk.batch);
             tma_reduce_add_4d(&tm_dq, sbase + L::kStageOff + L::kBoxBytes, hf * 64 + 32, grow, head, wk.batch);
             bulk_commit_group();
           }
         }
       }
-      if (issuer) bulk_wait_group0();
+      if (warp == 10 && elect_one()) bulk_wait_group0();
     }
   }
 

@@ -352,7 +352,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sgen + L::kMiscOff + 4);
   const WaitCtx wctx{abort_flag, p.status};
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   // SHIFTED: keys the causal diagonal is moved by (batched: one value; packed, or a cache with its
@@ -419,7 +419,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       tma_load_4d(sbase + L::kVOff + s * L::kTileBytes + bx * L::kBoxBytes, &tm_v, bar(iVFull + s),
                   bx * 64, wk.k_row0 + j * kTileN, wk.kv_head, wk.batch);
   };
-  if (threadIdx.x == kSmWarps * 32) {
+  if (warp == kSmWarps && elect_one()) {
     *abort_flag = 0;
     mbar_init(bar(iQFull + 0), 1);
     mbar_init(bar(iQFull + 1), 1);
@@ -467,7 +467,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // K tiles from warp 8, V tiles from warp 10: each ring refills as soon as its own stage is free
     // (the first tiles went out during setup).
     if (warp == kSmWarps) {
-      if (lane == 0) {
+      if (elect_one()) {
         for (int j = (NS > 1) ? 2 : 1; j < n_max; ++j) {
           const int s = j % NS;
           const int use = j / NS;
@@ -476,7 +476,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
       }
     } else {
-      if (lane == 0) {
+      if (elect_one()) {
         for (int j = 1; j < n_max; ++j) {
           const int s = j % NS;
           const int use = j / NS;
@@ -499,13 +499,13 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(iVFixed));
+        if (elect_one()) mbar_arrive(bar(iVFixed));
       }
     }
     __syncwarp();
   } else if (warp == kSmWarps + 1) {
     // ===================== MMA issuer =======================================
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc_f16(kTileM, kTileN, 0, 0);
       constexpr uint32_t idesc_pv = make_idesc_f16(kTileM, D, 0, 1);
       // Descriptors are stepped with 32-bit adds on their low words (address field = addr >> 4).
@@ -597,32 +597,36 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
         tc_commit(bar(iKEmpty + 0));
       }
-      for (int j = 0; j < n_max; ++j) {
-        const int s = j % NS;
-        const int use = j / NS;
-        for (int w = 0; w < 2; ++w) {
-          if (j >= ntile[w]) continue;
-          // P arrives in two halves of 64 keys, so that PV starts while the softmax warps are
-          // still exponentiating the second half.
-          mbar_wait(bar(iPHalf + w), j & 1, wctx, kBarPReady + w);
-          mbar_wait(bar(iVFull + s), use & 1, wctx, kBarVFull + s);
-          if (v_fix && j == n_max - 1) mbar_wait(bar(iVFixed), 0, wctx, kBarVFull + s);
-          tc_fence_after_sync();
-          issue_pv(w, w, j, 0);
-          mbar_wait(bar(iPReady + w), j & 1, wctx, kBarPReady + w);
-          tc_fence_after_sync();
-          issue_pv(w, w, j, 1);
-          tc_commit(bar(iODone + w));
-          if (w == 1 || j >= ntile[1]) tc_commit(bar(iVEmpty + s));
-          if (j + 1 < ntile[w]) {
-            const int s1 = (j + 1) % NS;
+      // P arrives in two halves of 64 keys, so that PV starts while the softmax warps are still exponentiating the
+      // second half.  V and the next K are waited for by the first tile that reads them, K under the first half of
+      // PV: what stands between P's arrival and the next scores is one wait and the MMAs.
+      auto step = [&](int w, int j, bool first_v, bool first_k) {
+        const int s = j % NS, s1 = (j + 1) % NS;
+        const bool more = j + 1 < ntile[w];
+        if (first_v) mbar_wait(bar(iVFull + s), (j / NS) & 1, wctx, kBarVFull + s);
+        if (v_fix && j == n_max - 1) mbar_wait(bar(iVFixed), 0, wctx, kBarVFull + s);
+        mbar_wait(bar(iPHalf + w), j & 1, wctx, kBarPReady + w);
+        tc_fence_after_sync();
+        issue_pv(w, w, j, 0);
+        if (NS > 1 && more && first_k) mbar_wait(bar(iKFull + s1), ((j + 1) / NS) & 1, wctx, kBarKFull + s1);
+        mbar_wait(bar(iPReady + w), j & 1, wctx, kBarPReady + w);
+        tc_fence_after_sync();
+        issue_pv(w, w, j, 1);
+        tc_commit(bar(iODone + w));
+        if (w == 1 || j >= ntile[1]) tc_commit(bar(iVEmpty + s));
+        if (more) {
+          if (NS == 1) {  // (one K buffer: the next tile may take longer than the second half of P)
             mbar_wait(bar(iKFull + s1), ((j + 1) / NS) & 1, wctx, kBarKFull + s1);
             tc_fence_after_sync();
-            issue_qk(w, w, j + 1);
-            tc_commit(bar(iSReady + w));
-            if (w == 1 || j + 1 >= ntile[1]) tc_commit(bar(iKEmpty + s1));
           }
+          issue_qk(w, w, j + 1);
+          tc_commit(bar(iSReady + w));
+          if (w == 1 || j + 1 >= ntile[1]) tc_commit(bar(iKEmpty + s1));
         }
+      };
+      for (int j = 0; j < n_max; ++j) {
+        if (j < ntile[0]) step(0, j, true, true);
+        if (L::kQTiles == 2 && j < ntile[1]) step(1, j, j >= ntile[0], j + 1 >= ntile[0]);
       }
       }
     }
@@ -891,7 +895,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       if (kAlt) asm volatile("bar.sync 15, 256;" ::: "memory");
       else asm volatile("bar.sync %0, 128;" ::"r"(13 + wg) : "memory");
-      if (quarter == 0 && lane == 0 && (!kAlt || wg == 0)) {
+      if (quarter == 0 && (!kAlt || wg == 0) && elect_one()) {
         const uint32_t src = sbase + L::kQOff + (kAlt ? 0 : wg * L::kTileBytes);
         for (int bx = 0; bx < L::kBoxes; ++bx)
           tma_store_4d(&tm_o, src + bx * L::kBoxBytes, bx * 64, wk.q_row0 + q_tile0, wk.head, wk.batch);
