@@ -20,8 +20,8 @@
 //   dV  += P^T dO     (M=128, N=head_dim, K=128)                TMEM x smem
 //   dK  += dS^T Q     (M=128, N=head_dim, K=128)                smem x smem
 //   dQ   = dS K       (M=128 queries, N=head_dim, K=128)        smem x smem (dS^T read M-contiguous)
-// P^T is produced in place over S^T, each compute thread owns one key row, and dS^T is
-// written to shared memory once and serves both dK and dQ.  The dQ tile leaves TMEM through
+// P^T is produced in place over S^T, a compute thread holds 16 columns of four key rows (the layout of
+// stmatrix), and dS^T is written to shared memory once and serves both dK and dQ.  The dQ tile leaves TMEM through
 // a swizzled shared-memory staging buffer and TMA tensor reductions (fp32 add) into the
 // accumulator that the post-pass casts.
 //
@@ -199,21 +199,12 @@ __device__ __forceinline__ bool bwd_decode_work(const BwdParams& p, int idx, Bwd
   return false;
 }
 
-// Of every 8 consecutive score columns, this many take the FMA-pipe exp2 instead of the
-// special-function unit (two compute warps per scheduler share 4 ex2 lanes per clock).
-#ifndef FAL_BWD_EXP_EMU_PER8
-#define FAL_BWD_EXP_EMU_PER8 0
-#endif
-template <int K>
-__device__ __forceinline__ float bwd_exp2(int j, float x) {
-  // j is a multiple of 4 under full unrolling, so the choice folds at compile time.
-  return (((j + K) & 7) < FAL_BWD_EXP_EMU_PER8) ? exp2_fma(x) : fast_exp2(x);
+// Where the per-query values (-lse * log2(e), -delta) of query row r of a tile stand: a compute thread reads columns
+// 8 k + 2 t + {0, 1} for its t = lane % 4, two k to a 16-byte load.
+__device__ __forceinline__ int stat_slot(int r) {
+  const int k = r >> 3, t = (r >> 1) & 3;
+  return ((k >> 1) * 4 + t) * 4 + (k & 1) * 2 + (r & 1);
 }
-
-// One elected lane per compute warp arrives on p_ready / ds_ready (1) or every thread (0).
-#ifndef FAL_BWD_ELECT_ARRIVE
-#define FAL_BWD_ELECT_ARRIVE 1
-#endif
 
 // fp32 add-reduction of one swizzled shared-memory box into a 4-D tensor (TMA).
 __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* map, uint32_t src_smem, int c0, int c1,
@@ -338,8 +329,8 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     mbar_init(bar(iDpReady), 1);
     mbar_init(bar(iDqReady), 1);
     mbar_init(bar(iDqFree), 128);
-    mbar_init(bar(iPReady), FAL_BWD_ELECT_ARRIVE ? 8 : 256);
-    mbar_init(bar(iDsReady), FAL_BWD_ELECT_ARRIVE ? 8 : 256);
+    mbar_init(bar(iPReady), 8);
+    mbar_init(bar(iDsReady), 8);
     mbar_init(bar(iAllDone), 1);
     mbar_init(bar(iDsFree), 1);
     mbar_init(bar(iAFull), 1);
@@ -442,29 +433,39 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     }
   } else if (warp == 14) {
     // ===================== per-row statistics: lse * log2(e) and delta ========
+    // A tile's values are fetched, all at once, while the tile before is worked on.  Fetched row by row when their
+    // buffer came free, they were what every step waited for at head_dim 128 (1 000 to 1 500 of 4 600 cycles; now the
+    // loads of Q behind the dQ reductions set the pace there, 1 382 -> 1 362 us on 4 x 32 / 8 x 4 096 causal; at head_dim
+    // 64 16 x 16 384 causal 1 660 -> 1 530).
+    float lse[kQTile / 32], delta[kQTile / 32];
+    int fetched = 0;
+    auto fetch = [&](int i) {
+      const int head = wk.kv_head * group + i / nq;
+      fetched = (qt0 + i % nq) * kQTile;
+      const float* lse_head = p.lse + wk.batch * p.lse_strides.batch + head * p.lse_strides.head;
+      const float* delta_head = p.delta + wk.batch * p.delta_batch_stride + head * p.delta_head_stride;
+#pragma unroll
+      for (int rr = 0; rr < kQTile / 32; ++rr) {
+        const int64_t row = static_cast<int64_t>(wk.q_row0) + min(fetched + lane + rr * 32, wk.seqlen_q - 1);
+        lse[rr] = __ldg(lse_head + row * p.lse_strides.row);
+        delta[rr] = __ldg(delta_head + row);
+      }
+    };
+    if (n_iter > 0) fetch(0);
     for (int i = 0; i < n_iter; ++i) {
       const int st = i % NS;
-      const int head = wk.kv_head * group + i / nq;
-      const int qt = qt0 + i % nq;
       if (i >= NS) mbar_wait(bar(iQEmpty + st), ((i / NS) - 1) & 1, wctx, kBbQEmpty + st);
       float* stat = reinterpret_cast<float*>(sgen + L::kStatOff) + st * 2 * kQTile;
 #pragma unroll
       for (int rr = 0; rr < kQTile / 32; ++rr) {
         const int r = lane + rr * 32;
-        const int q_local = qt * kQTile + r;
-        float lse2 = INFINITY;  // exp2(x - inf) = 0: rows past the sequence contribute nothing
-        float dl = 0.f;
-        if (q_local < wk.seqlen_q) {
-          const int64_t grow = static_cast<int64_t>(wk.q_row0) + q_local;
-          const float l = __ldg(p.lse + wk.batch * p.lse_strides.batch + head * p.lse_strides.head +
-                                grow * p.lse_strides.row);
-          if (l > -INFINITY) lse2 = l * kLog2e;
-          dl = __ldg(p.delta + wk.batch * p.delta_batch_stride + head * p.delta_head_stride + grow);
-        }
-        stat[r] = lse2;
-        stat[kQTile + r] = dl;
+        const bool row_ok = fetched + r < wk.seqlen_q;
+        // exp2(x - inf) = 0: rows past the sequence, and rows that see no key, contribute nothing
+        stat[stat_slot(r)] = row_ok && lse[rr] > -INFINITY ? -lse[rr] * kLog2e : -INFINITY;
+        stat[kQTile + stat_slot(r)] = row_ok ? -delta[rr] : 0.f;
       }
       mbar_arrive(bar(iStatFull + st));
+      if (i + 1 < n_iter) fetch(i + 1);
     }
   } else if (warp == 9) {
     // ===================== MMA issuer =========================================
@@ -599,112 +600,124 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // ===================== compute ============================================
     const int quarter = warp & 3;
     const int half = warp >> 2;                       // query columns [64*half, 64*half+64)
-    const int kv_row = quarter * 32 + lane;           // key row inside the tile (= TMEM lane)
+    const int kv_row = quarter * 32 + lane;           // key row of the epilogue (= TMEM lane)
     const int kv_local = kv0 + kv_row;
     const bool kv_ok = kv_local < wk.seqlen_k;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    const float c2 = p.scale_log2;
-    // this thread's dS^T row: box `half` (64 query columns = 128 bytes per key row)
-    uint8_t* ds_row = sgen + L::kDsOff + half * L::kBoxBytes + kv_row * 128;
+    const uint64_t c2p = pack_f32x2(p.scale_log2, p.scale_log2);
+    // What a compute thread needs of the queries are two numbers per column it holds.  With a key row of 64 columns to a
+    // thread those were 32 broadcast loads of 16 bytes a step, as many wavefronts of the shared-memory pipe -- the unit
+    // that bounds head_dim 128 -- as storing dS^T and staging dQ take together.  With 16 columns of four rows they are 8, and
+    // neighbouring columns sit in one register pair for the two-float instructions.  us on the GPU: 4 x 32 / 8 x 4 096 of
+    // 128 causal 1 401 -> 1 382, 4 x 16 x 2 048 of 64 causal 191 -> 185; with the statistics fetched ahead (warp 14) 1 362
+    // and 153.
+    // In the main loop a thread holds columns 8 k + 2 (lane % 4) + {0, 1} of the four key rows lane / 4 + 8 g of
+    // the warp's 32: register [g / 2][4 k + 2 (g % 2) + {0, 1}].
+    const int frag_row = quarter * 32 + (lane >> 2);
+    const int frag_col = half * 64 + 2 * (lane & 3);
+    // this lane's row of the dS^T matrices it names to stmatrix: row lane % 8 of key rows 8 (lane / 8 % 2), 16-byte
+    // chunk lane / 16 (+ k), 128-byte XOR swizzle
+    const int ds_row = quarter * 32 + (lane & 15);
+    const uint32_t ds_base = sbase + L::kDsOff + half * L::kBoxBytes + ds_row * 128;
+    const uint32_t ds_chunk = static_cast<uint32_t>((lane >> 4) ^ (lane & 7)) << 4;
 
     for (int i = 0; i < n_iter; ++i) {
       const int st = i % NS;
       const int qt = qt0 + i % nq;
-      const int q_col0 = qt * kQTile + half * 64;  // local query index of this thread's first column
-      const float* stat = reinterpret_cast<const float*>(sgen + L::kStatOff) + st * 2 * kQTile + half * 64;
-      const bool tile_mask = !kv_ok || (CAUSAL && (kv0 + kKvTile - 1 > qt * kQTile + cshift));
+      // per-query values of this thread's columns: 4 (of columns 8 k and 8 k + 8) to a 16-byte load
+      const float4* stat = reinterpret_cast<const float4*>(sgen + L::kStatOff) + st * (2 * kQTile / 4) + half * 16 + (lane & 3);
+      const bool tile_mask = kv0 + kKvTile > wk.seqlen_k || (CAUSAL && (kv0 + kKvTile - 1 > qt * kQTile + cshift));
 
       mbar_wait(bar(iStatFull + st), (i / NS) & 1, wctx, kBbStatFull + st);
       mbar_wait(bar(iSReady), i & 1, wctx, kBbSReady);
       tc_fence_after_sync();
 
       // ---- P^T = exp2(S^T * c2 - lse2), kept as packed fp16 for the dS step ----
-      uint32_t pk[32];
+      uint32_t pk[2][16];
       {
         uint32_t r[2][32];
-        tmem_ld_32x32b_x32(tmem_base + lane_addr + kColS + half * 64, r[0]);
-        tmem_ld_32x32b_x32(tmem_base + lane_addr + kColS + half * 64 + 32, r[1]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          tmem_ld_16x256b_x8(tmem_base + lane_addr + (static_cast<uint32_t>(h * 16) << 16) + kColS + half * 64, r[h]);
         tmem_wait_ld();
         if (tile_mask) {  // hidden scores become -inf before the exponential (exp2(-inf) = 0)
 #pragma unroll
-          for (int c = 0; c < 2; ++c)
+          for (int g = 0; g < 4; ++g) {
+            const int key = kv0 + frag_row + 8 * g;
+            // the first of this thread's columns (less 2 (lane % 4)) that sees the key
+            int first = CAUSAL ? key - cshift - (qt * kQTile + frag_col) : 0;
+            if (key >= wk.seqlen_k) first = 64;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const bool vis = kv_ok && (!CAUSAL || kv_local <= q_col0 + cshift + c * 32 + j);
-              r[c][j] = vis ? r[c][j] : 0xff800000u;
-            }
-        }
+            for (int k = 0; k < 8; ++k)
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            const float4 l4 = *reinterpret_cast<const float4*>(stat + c * 32 + j);
-#ifdef FAL_BWD_EXP_F16X2
-            // exponent rounded to fp16 first, two exponentials per MUFU instruction
-            pk[c * 16 + (j >> 1) + 0] = exp2_f16x2(pack_half2(fmaf(__uint_as_float(r[c][j + 0]), c2, -l4.x),
-                                                              fmaf(__uint_as_float(r[c][j + 1]), c2, -l4.y)));
-            pk[c * 16 + (j >> 1) + 1] = exp2_f16x2(pack_half2(fmaf(__uint_as_float(r[c][j + 2]), c2, -l4.z),
-                                                              fmaf(__uint_as_float(r[c][j + 3]), c2, -l4.w)));
-#else
-            const float p0 = bwd_exp2<0>(j, fmaf(__uint_as_float(r[c][j + 0]), c2, -l4.x));
-            const float p1 = bwd_exp2<1>(j, fmaf(__uint_as_float(r[c][j + 1]), c2, -l4.y));
-            const float p2 = bwd_exp2<2>(j, fmaf(__uint_as_float(r[c][j + 2]), c2, -l4.z));
-            const float p3 = bwd_exp2<3>(j, fmaf(__uint_as_float(r[c][j + 3]), c2, -l4.w));
-            pk[c * 16 + (j >> 1) + 0] = pack_half2(p0, p1);
-            pk[c * 16 + (j >> 1) + 1] = pack_half2(p2, p3);
-#endif
+              for (int e = 0; e < 2; ++e) {
+                uint32_t& x = r[g >> 1][4 * k + 2 * (g & 1) + e];
+                x = 8 * k + e >= first ? x : 0xff800000u;
+              }
           }
         }
-        // P^T overwrites this thread's own S^T columns: 32 packed columns at [64*half, 64*half+32)
-        tmem_st_32x32b_x32(tmem_base + lane_addr + kColS + half * 64, pk);
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+          const float4 l4 = stat[(k >> 1) * 4];
+          const uint64_t nl[2] = {pack_f32x2(l4.x, l4.y), pack_f32x2(l4.z, l4.w)};
+#pragma unroll
+          for (int g = 0; g < 4; ++g)
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) {
+              const uint32_t* x = &r[g >> 1][4 * (k + kk) + 2 * (g & 1)];
+              float p0, p1;
+              unpack_f32x2(ffma2(pack_f32x2(__uint_as_float(x[0]), __uint_as_float(x[1])), c2p, nl[kk]), p0, p1);
+              pk[g >> 1][2 * (k + kk) + (g & 1)] = pack_half2(fast_exp2(p0), fast_exp2(p1));
+            }
+        }
+        // P^T overwrites this warp's own S^T columns: 32 packed columns at [64*half, 64*half+32)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          tmem_st_16x128b_x8(tmem_base + lane_addr + (static_cast<uint32_t>(h * 16) << 16) + kColS + half * 64, pk[h]);
         tmem_wait_st();
       }
       tc_fence_before_sync();
-#if FAL_BWD_ELECT_ARRIVE
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(iPReady));
-#else
-      mbar_arrive(bar(iPReady));
-#endif
 
       // ---- dS^T = P^T o (dP^T - delta) ------------------------------------------
       mbar_wait(bar(iDpReady), i & 1, wctx, kBbDpReady);
       tc_fence_after_sync();
-      uint32_t dsp[32];
       {
         uint32_t r[2][32];
-        tmem_ld_32x32b_x32(tmem_base + lane_addr + kColDpq + half * 64, r[0]);
-        tmem_ld_32x32b_x32(tmem_base + lane_addr + kColDpq + half * 64 + 32, r[1]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          tmem_ld_16x256b_x8(tmem_base + lane_addr + (static_cast<uint32_t>(h * 16) << 16) + kColDpq + half * 64, r[h]);
         tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int k = 0; k < 8; k += 2) {
+          // (dP - delta) in fp32 (it cancels), rounded to fp16, then one packed multiply by the
+          // fp16 P: the product is the fp16 dS the GEMMs consume.
+          const float4 d4 = stat[kQTile / 4 + (k >> 1) * 4];
+          const uint64_t nd[2] = {pack_f32x2(d4.x, d4.y), pack_f32x2(d4.z, d4.w)};
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            // (dP - delta) in fp32 (it cancels), rounded to fp16, then one packed multiply by the
-            // fp16 P: the product is the fp16 dS the GEMMs consume.
-            const float4 d4 = *reinterpret_cast<const float4*>(stat + kQTile + c * 32 + j);
-            const uint32_t e0 = pack_half2(__uint_as_float(r[c][j + 0]) - d4.x, __uint_as_float(r[c][j + 1]) - d4.y);
-            const uint32_t e1 = pack_half2(__uint_as_float(r[c][j + 2]) - d4.z, __uint_as_float(r[c][j + 3]) - d4.w);
-            dsp[c * 16 + (j >> 1) + 0] = hmul2_bits(pk[c * 16 + (j >> 1) + 0], e0);
-            dsp[c * 16 + (j >> 1) + 1] = hmul2_bits(pk[c * 16 + (j >> 1) + 1], e1);
-          }
+          for (int g = 0; g < 4; ++g)
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) {
+              const uint32_t* x = &r[g >> 1][4 * (k + kk) + 2 * (g & 1)];
+              float e0, e1;
+              unpack_f32x2(fadd2(pack_f32x2(__uint_as_float(x[0]), __uint_as_float(x[1])), nd[kk]), e0, e1);
+              uint32_t& ds = pk[g >> 1][2 * (k + kk) + (g & 1)];
+              ds = hmul2_bits(ds, pack_half2(e0, e1));
+            }
         }
       }
       if (i > 0) mbar_wait(bar(iDsFree), (i - 1) & 1, wctx, kBbDqReady);
-      // dS^T row -> shared memory, 128-byte XOR swizzle (16-byte chunk index ^ row % 8)
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        *reinterpret_cast<uint4*>(ds_row + ((c ^ (kv_row & 7)) << 4)) =
-            make_uint4(dsp[4 * c + 0], dsp[4 * c + 1], dsp[4 * c + 2], dsp[4 * c + 3]);
-      }
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int k = 0; k < 8; k += 2)
+          stmatrix_x4(ds_base + h * (16 * 128) + (ds_chunk ^ (k << 4)), pk[h][2 * k], pk[h][2 * k + 1], pk[h][2 * k + 2],
+                      pk[h][2 * k + 3]);
       fence_proxy_async_smem();
       tc_fence_before_sync();
-#if FAL_BWD_ELECT_ARRIVE
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(iDsReady));
-#else
-      mbar_arrive(bar(iDsReady));
-#endif
     }
 
     // ---- epilogue: dV (warps 0-3) and dK (warps 4-7) -------------------------
