@@ -35,6 +35,10 @@
 //
 // TMEM columns: S^T/P^T [0,128), dP^T/dQ [128,256) (the dQ tile of a step reuses the columns of
 //               that step's consumed dP^T), dV [256,256+D), dK [256+D,256+2D).
+// At head_dim 64 there is room for more, and a step is bound by the compute warps' chain (exponentials, dS, its
+// stores) where nothing holds them up: S^T / P^T of odd steps have columns [384,512), so that the scores of a step are
+// computed under the exponentials of the step before instead of behind its dV, Q has three buffers and dO two.  us:
+// 16 x 16 384 causal 1 530 -> 1 447, 4 x 16 x 2 048 235 -> 216, 32 x 16 x 577 278 -> 260.
 // Shared memory at head_dim 128: K 32K, V 32K, Q 2 x 32K, dO 32K, dS^T 32K, dQ staging 2 x 16K.
 //
 // head_dim 256 (SPLIT = true): two CTAs share a key tile, each owning 128 of the 256 columns of dV, dK and
@@ -70,15 +74,17 @@ enum BwdBarrier : int {
 
 template <int D>
 struct BwdSmem {
-  static constexpr int kQStages = 2;                           // Q tiles and row statistics
+  static constexpr int kQStages = D == 64 ? 3 : 2;             // Q tiles and row statistics
+  static constexpr int kDoStages = D == 64 ? 2 : 1;
+  static constexpr int kSBuffers = D == 64 ? 2 : 1;            // S^T / P^T blocks in TMEM
   static constexpr int kBoxes = D / 64;
   static constexpr int kBoxBytes = 128 * 128;                  // one 128-row x 128-byte box
   static constexpr int kTileBytes = kBoxes * kBoxBytes;        // K, V, Q and dO tiles are 128 x D
   static constexpr int kKOff = 0;
   static constexpr int kVOff = kTileBytes;
   static constexpr int kQOff = 2 * kTileBytes;
-  static constexpr int kDoOff = kQOff + kQStages * kTileBytes;  // single stage
-  static constexpr int kDsOff = kDoOff + kTileBytes;            // [2 boxes][128 keys][64 queries] fp16
+  static constexpr int kDoOff = kQOff + kQStages * kTileBytes;
+  static constexpr int kDsOff = kDoOff + kDoStages * kTileBytes;  // [2 boxes][128 keys][64 queries] fp16
   static constexpr int kDsBytes = 2 * kBoxBytes;
   static constexpr int kStageOff = kDsOff + kDsBytes;           // dQ staging: 2 x [128 rows][32 fp32], or per warp 2 x [32][32]
   static constexpr bool kWarpDq = D == 128;                     // the write-back warps work independently
@@ -87,9 +93,9 @@ struct BwdSmem {
   static constexpr int kStatOff = kStageOff + kStageBytes;      // per Q stage: lse2[128], delta[128]
   static constexpr int kStatBytes = kQStages * 2 * kQTile * 4;
   static constexpr int kBarOff = kStatOff + kStatBytes;
-  // k_full v_full q_full[2] q_empty[2] stat_full[2] do_full do_empty
-  // s_ready dp_ready dq_ready dq_free p_ready ds_ready all_done ds_free a_full a_done b_full
-  static constexpr int kNumBars = 2 + 6 + 2 + 8 + 3;
+  // k_full v_full q_full[NQ] q_empty[NQ] stat_full[NQ] do_full[ND] do_empty[ND] s_ready[NB] p_ready[NB]
+  // dp_ready dq_ready dq_free ds_ready all_done ds_free a_full a_done b_full
+  static constexpr int kNumBars = 2 + 3 * kQStages + 2 * kDoStages + 2 * kSBuffers + 9;
   static constexpr int kMiscOff = kBarOff + kNumBars * 8;
   static constexpr int kBytes = kMiscOff + 16;
   // No slack for re-aligning the base: at head_dim 128 the layout fills the 227 KB limit, so the
@@ -103,6 +109,8 @@ struct BwdSmem {
 // dO buffer (own columns), and X = kDsOff: Q's other columns, then dO's, then dS^T.
 struct BwdSplitSmem {
   static constexpr int kQStages = 1;
+  static constexpr int kDoStages = 1;
+  static constexpr int kSBuffers = 1;
   static constexpr int kBoxes = 2;
   static constexpr int kBoxBytes = 128 * 128;
   static constexpr int kTileBytes = kBoxes * kBoxBytes;
@@ -113,7 +121,7 @@ struct BwdSplitSmem {
   static constexpr int kDsOff = 6 * kTileBytes;
   static constexpr int kStatOff = 7 * kTileBytes;
   static constexpr int kBarOff = kStatOff + 2 * kQTile * 4;
-  static constexpr int kNumBars = 21;
+  static constexpr int kNumBars = 2 + 3 + 2 + 2 + 9;
   static constexpr int kMiscOff = kBarOff + kNumBars * 8;
   static constexpr int kBytes = kMiscOff + 16;
   static constexpr int kAllocBytes = kBytes;
@@ -275,7 +283,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_dk,
                const __grid_constant__ CUtensorMap tm_dv, const BwdParams p) {
   using L = std::conditional_t<SPLIT, BwdSplitSmem, BwdSmem<D>>;
-  constexpr int NS = L::kQStages;
+  constexpr int NS = L::kQStages, ND = L::kDoStages, NB = L::kSBuffers;
   // SPLIT: head_dim is 2 * D; CTAs 2n and 2n+1 share key tile n and own columns [0, D) and [D, 2D).
   const int col_own = SPLIT ? static_cast<int>(blockIdx.x & 1) * D : 0;
   const int col_other = SPLIT ? D - col_own : 0;
@@ -292,10 +300,12 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   }
   const uint32_t bar0 = sbase + L::kBarOff;
   auto bar = [&](int i) { return bar0 + 8u * i; };
-  constexpr int iKFull = 0, iVFull = 1, iQFull = 2, iQEmpty = 4, iStatFull = 6, iDoFull = 8, iDoEmpty = 9,
-                iSReady = 10, iDpReady = 11, iDqReady = 12, iDqFree = 13, iPReady = 14, iDsReady = 15,
-                iAllDone = 16, iDsFree = 17, iAFull = 18, iADone = 19,
-                iBFull = 20;
+  constexpr int iKFull = 0, iVFull = 1, iQFull = 2, iQEmpty = iQFull + NS, iStatFull = iQEmpty + NS,
+                iDoFull = iStatFull + NS, iDoEmpty = iDoFull + ND, iSReady = iDoEmpty + ND, iPReady = iSReady + NB,
+                iDpReady = iPReady + NB, iDqReady = iDpReady + 1, iDqFree = iDpReady + 2, iDsReady = iDpReady + 3,
+                iAllDone = iDpReady + 4, iDsFree = iDpReady + 5, iAFull = iDpReady + 6, iADone = iDpReady + 7,
+                iBFull = iDpReady + 8;
+  static_assert(iBFull + 1 == L::kNumBars, "barrier count");
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sgen + L::kMiscOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sgen + L::kMiscOff + 4);
   const WaitCtx wctx{abort_flag, p.status};
@@ -323,13 +333,17 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       mbar_init(bar(iQEmpty + s), 1);
       mbar_init(bar(iStatFull + s), 32);
     }
-    mbar_init(bar(iDoFull), 1);
-    mbar_init(bar(iDoEmpty), 1);
-    mbar_init(bar(iSReady), 1);
+    for (int s = 0; s < ND; ++s) {
+      mbar_init(bar(iDoFull + s), 1);
+      mbar_init(bar(iDoEmpty + s), 1);
+    }
+    for (int s = 0; s < NB; ++s) {
+      mbar_init(bar(iSReady + s), 1);
+      mbar_init(bar(iPReady + s), 8);
+    }
     mbar_init(bar(iDpReady), 1);
     mbar_init(bar(iDqReady), 1);
     mbar_init(bar(iDqFree), 128);
-    mbar_init(bar(iPReady), 8);
     mbar_init(bar(iDsReady), 8);
     mbar_init(bar(iAllDone), 1);
     mbar_init(bar(iDsFree), 1);
@@ -347,6 +361,8 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   constexpr uint32_t kColS = 0, kColDpq = 128, kColDv = 256, kColDk = 256 + D;
+  constexpr uint32_t kColS1 = NB == 2 ? kColDk + D : kColS;  // S^T / P^T of odd steps
+  static_assert(NB == 1 || kColS1 + 128 <= 512, "TMEM columns");
 
   if (warp == 8) {
     // ===================== producer: TMA ======================================
@@ -421,12 +437,13 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           for (int bx = 0; bx < L::kBoxes; ++bx)
             tma_load_4d(sbase + L::kQOff + st * L::kTileBytes + bx * L::kBoxBytes, &tm_q,
                         bar(iQFull + st), bx * 64, row, head, wk.batch);
-          // dO has a single buffer: it is reloaded as soon as dV of the previous step has read it.
-          if (i >= 1) mbar_wait(bar(iDoEmpty), (i - 1) & 1, wctx, kBbDoEmpty);
-          mbar_arrive_expect_tx(bar(iDoFull), L::kTileBytes);
+          // a dO buffer is reloaded as soon as dV of its last step has read it
+          const int sd = i % ND;
+          if (i >= ND) mbar_wait(bar(iDoEmpty + sd), ((i / ND) - 1) & 1, wctx, kBbDoEmpty);
+          mbar_arrive_expect_tx(bar(iDoFull + sd), L::kTileBytes);
           for (int bx = 0; bx < L::kBoxes; ++bx)
-            tma_load_4d(sbase + L::kDoOff + bx * L::kBoxBytes, &tm_do, bar(iDoFull), bx * 64, row, head,
-                        wk.batch);
+            tma_load_4d(sbase + L::kDoOff + sd * L::kTileBytes + bx * L::kBoxBytes, &tm_do, bar(iDoFull + sd), bx * 64,
+                        row, head, wk.batch);
         }
       }
       __syncwarp();
@@ -505,11 +522,20 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         issue_xyT(kColDpq, v_lo_k, sbase + L::kDoOff);
         tc_commit(bar(iDpReady));
       }
-      const uint32_t do_lo_mn = smem_desc_lo(sbase + L::kDoOff, L::kBoxBytes);
 
       for (int i = 0; i < n_iter; ++i) {
         const int st = i % NS;
         const int st1 = (i + 1) % NS;
+        const uint32_t col_s = (NB == 2 && (i & 1) != 0) ? kColS1 : kColS;
+        const uint32_t do_lo_mn = smem_desc_lo(sbase + L::kDoOff + (i % ND) * L::kTileBytes, L::kBoxBytes);
+        // S^T(i+1) overwrites P^T(i+1-NB): issued behind dV(i+1-NB), which reads it.
+        auto next_scores = [&]() {
+          mbar_wait(bar(iQFull + st1), ((i + 1) / NS) & 1, wctx, kBbQFull + st1);
+          tc_fence_after_sync();
+          issue_xyT(NB == 2 ? kColS + kColS1 - col_s : kColS, k_lo_k, sbase + L::kQOff + st1 * L::kTileBytes);
+          tc_commit(bar(iSReady + (i + 1) % NB));
+        };
+        if (NB == 2 && i + 1 < n_iter) next_scores();
         const uint32_t q_lo_mn = smem_desc_lo(sbase + L::kQOff + st * L::kTileBytes, L::kBoxBytes);
         if constexpr (SPLIT) {
           // S^T(i) and dP^T(i) in two parts, the other column half (from X) first.  S^T goes over P^T(i-1),
@@ -537,23 +563,17 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           tc_commit(bar(iDpReady));
         }
         // dV += P^T(i) dO(i): P^T as packed fp16 in TMEM; query columns [0,64) at +0, [64,128) at +64
-        mbar_wait(bar(iPReady), i & 1, wctx, kBbPReady);
+        mbar_wait(bar(iPReady + i % NB), (i / NB) & 1, wctx, kBbPReady);
         tc_fence_after_sync();
 #pragma unroll
         for (int ks = 0; ks < kQTile / 16; ++ks) {
-          const uint32_t a_col = kColS + (ks >> 2) * 64 + (ks & 3) * 8;
+          const uint32_t a_col = col_s + (ks >> 2) * 64 + (ks & 3) * 8;
           umma_ts(tmem_base + kColDv, tmem_base + a_col,
                   smem_desc_join(do_lo_mn + ((ks * 2048) >> 4), kHi), idesc_dkv,
                   (i > 0 || ks > 0) ? 1u : 0u);
         }
-        tc_commit(bar(iDoEmpty));  // dO(i) has no reader left once dV(i) is done
-        // S^T(i+1) overwrites P^T(i): issued after dV(i), which reads it.
-        if (!SPLIT && i + 1 < n_iter) {
-          mbar_wait(bar(iQFull + st1), ((i + 1) / NS) & 1, wctx, kBbQFull + st1);
-          tc_fence_after_sync();
-          issue_xyT(kColS, k_lo_k, sbase + L::kQOff + st1 * L::kTileBytes);
-          tc_commit(bar(iSReady));
-        }
+        tc_commit(bar(iDoEmpty + i % ND));  // dO(i) has no reader left once dV(i) is done
+        if (!SPLIT && NB == 1 && i + 1 < n_iter) next_scores();
         mbar_wait(bar(iDsReady), i & 1, wctx, kBbDsReady);
         tc_fence_after_sync();
         // dK += dS^T(i) Q(i)
@@ -586,10 +606,11 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         tc_commit(bar(iDsFree));  // both readers of the dS^T buffer are done
         // dP^T(i+1) goes where dQ(i) is: the write-back warps must have read it out first.
         if (!SPLIT && i + 1 < n_iter) {
-          mbar_wait(bar(iDoFull), (i + 1) & 1, wctx, kBbDoFull);
+          const int sd1 = (i + 1) % ND;
+          mbar_wait(bar(iDoFull + sd1), ((i + 1) / ND) & 1, wctx, kBbDoFull);
           mbar_wait(bar(iDqFree), i & 1, wctx, kBbDqFree);
           tc_fence_after_sync();
-          issue_xyT(kColDpq, v_lo_k, sbase + L::kDoOff);
+          issue_xyT(kColDpq, v_lo_k, sbase + L::kDoOff + sd1 * L::kTileBytes);
           tc_commit(bar(iDpReady));
         }
       }
@@ -626,10 +647,11 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       const int qt = qt0 + i % nq;
       // per-query values of this thread's columns: 4 (of columns 8 k and 8 k + 8) to a 16-byte load
       const float4* stat = reinterpret_cast<const float4*>(sgen + L::kStatOff) + st * (2 * kQTile / 4) + half * 16 + (lane & 3);
+      const uint32_t t_s = tmem_base + lane_addr + ((NB == 2 && (i & 1) != 0) ? kColS1 : kColS) + half * 64;
       const bool tile_mask = kv0 + kKvTile > wk.seqlen_k || (CAUSAL && (kv0 + kKvTile - 1 > qt * kQTile + cshift));
 
       mbar_wait(bar(iStatFull + st), (i / NS) & 1, wctx, kBbStatFull + st);
-      mbar_wait(bar(iSReady), i & 1, wctx, kBbSReady);
+      mbar_wait(bar(iSReady + i % NB), (i / NB) & 1, wctx, kBbSReady);
       tc_fence_after_sync();
 
       // ---- P^T = exp2(S^T * c2 - lse2), kept as packed fp16 for the dS step ----
@@ -638,7 +660,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         uint32_t r[2][32];
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-          tmem_ld_16x256b_x8(tmem_base + lane_addr + (static_cast<uint32_t>(h * 16) << 16) + kColS + half * 64, r[h]);
+          tmem_ld_16x256b_x8(t_s + (static_cast<uint32_t>(h * 16) << 16), r[h]);
         tmem_wait_ld();
         if (tile_mask) {  // hidden scores become -inf before the exponential (exp2(-inf) = 0)
 #pragma unroll
@@ -673,12 +695,12 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         // P^T overwrites this warp's own S^T columns: 32 packed columns at [64*half, 64*half+32)
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-          tmem_st_16x128b_x8(tmem_base + lane_addr + (static_cast<uint32_t>(h * 16) << 16) + kColS + half * 64, pk[h]);
+          tmem_st_16x128b_x8(t_s + (static_cast<uint32_t>(h * 16) << 16), pk[h]);
         tmem_wait_st();
       }
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar(iPReady));
+      if (lane == 0) mbar_arrive(bar(iPReady + i % NB));
 
       // ---- dS^T = P^T o (dP^T - delta) ------------------------------------------
       mbar_wait(bar(iDpReady), i & 1, wctx, kBbDpReady);
