@@ -36,10 +36,13 @@
 // (head_dim 256 has no columns left for this: one warpgroup takes every key tile, as in a two-tile CTA.)
 //
 // Half an SM (128 query rows, head_dim 64, 256 threads): one softmax warpgroup and its tile, two CTAs per SM.
-// TMEM columns: S [0,128) O [128,192).
+// TMEM columns: S [0,128) O [128,192) P [192,256).
 //
-// P (fp16) feeds the PV MMA straight from TMEM; except in the one-tile CTA it overwrites the first 64
-// columns of its S block.
+// P (fp16) feeds the PV MMA straight from TMEM.  At head_dim 128 with two tiles and at 256 it overwrites the first 64
+// columns of its S block, and the next scores wait for P V.  At head_dim 64 it has columns of its own (two tiles: P0
+// [384,448) P1 [448,512)): the next scores are computed while a warpgroup works on the last, which it then never waits for;
+// two tiles' 32 768 exponentials (2 048 cycles of the special-function unit) bound a step of about 2 400 cycles.  us:
+// 16 x 16 384 causal 722 -> 652, 4 x 16 x 2 048 111.6 -> 103.7, 32 x 16 x 577 (half an SM) 102.7 -> 98.8.
 #define FAL_WAIT_SLOW_PATH_INLINE  // this kernel uses setmaxnreg, which rules out calls
 #include "fal_common.h"
 #include "fal_launch.h"
@@ -133,6 +136,10 @@ struct FwdSmem {
   // One tile at head_dim 64 / 128: the softmax warpgroups take alternate key tiles (kAlt).  At 256 there
   // is no TMEM left for that (P needs columns of its own), one warpgroup takes every key tile.
   static constexpr bool kAlt = SHAPE == kOneTile && D != 256;
+  // head_dim 64, a warpgroup per tile: TMEM has columns for P apart from the scores (kSepP), at kPCol + 64 w.
+  static constexpr bool kSepP = D == 64 && SHAPE != kOneTile;
+  static constexpr int kPCol = kOCol + kQTiles * D;
+  static_assert(!kSepP || kPCol + kQTiles * 64 <= kTmemCols, "TMEM columns");
   static constexpr int kCtaRows = kQTiles * kTileM;
   static constexpr int kStages = SHAPE == kHalfSm ? 2 : (D == 256) ? 1 : (D == 128) ? 2 : 4;
   static constexpr int kBoxes = D / 64;                 // 64-element (128-byte) column boxes
@@ -531,7 +538,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       auto issue_pv = [&](int sb, int ot, int j, int half) {
         const uint32_t v_lo = smem_desc_lo(sbase + L::kVOff + (j % NS) * L::kTileBytes, L::kBoxBytes);
         const uint32_t t_o = L::kAlt ? tmem_base + 384 : tmem_base + L::kOCol + ot * D;
-        const uint32_t t_p = L::kAlt ? tmem_base + 256 + sb * 64 : tmem_base + sb * kTileN;
+        const uint32_t t_p = L::kAlt ? tmem_base + 256 + sb * 64 : L::kSepP ? tmem_base + L::kPCol + sb * 64 : tmem_base + sb * kTileN;
 #pragma unroll
         for (int kk = 0; kk < kTileN / 32; ++kk) {
           const int ks = half * (kTileN / 32) + kk;
@@ -597,6 +604,41 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
         tc_commit(bar(iKEmpty + 0));
       }
+      if constexpr (L::kSepP) {
+        // The scores of the next key tile are issued as soon as the warpgroup has read this one's, so it finds them
+        // waiting.  The order is that of two warpgroups half a step apart.
+        auto next_scores = [&](int w, int j, bool first) {
+          if (j + 1 >= ntile[w]) return;
+          const int s1 = (j + 1) % NS;
+          if (first) mbar_wait(bar(iKFull + s1), ((j + 1) / NS) & 1, wctx, kBarKFull + s1);
+          mbar_wait(bar(iSFree + w), j & 1, wctx, kBarSReady + w);
+          tc_fence_after_sync();
+          issue_qk(w, w, j + 1);
+          tc_commit(bar(iSReady + w));
+          if (w == 1 || j + 1 >= ntile[1]) tc_commit(bar(iKEmpty + s1));
+        };
+        auto add_pv = [&](int w, int j, bool first) {
+          if (j < 0 || j >= ntile[w]) return;
+          const int s = j % NS;
+          if (first) mbar_wait(bar(iVFull + s), (j / NS) & 1, wctx, kBarVFull + s);
+          if (v_fix && j == n_max - 1) mbar_wait(bar(iVFixed), 0, wctx, kBarVFull + s);
+          mbar_wait(bar(iPReady + w), j & 1, wctx, kBarPReady + w);
+          tc_fence_after_sync();
+          issue_pv(w, w, j, 0);
+          issue_pv(w, w, j, 1);
+          tc_commit(bar(iODone + w));
+          if (w == 1 || j >= ntile[1]) tc_commit(bar(iVEmpty + s));
+        };
+        for (int j = 0; j < n_max; ++j) {
+          next_scores(0, j, true);
+          if (L::kQTiles == 2) {
+            add_pv(1, j - 1, j - 1 >= ntile[0]);
+            next_scores(1, j, j + 1 >= ntile[0]);
+          }
+          add_pv(0, j, true);
+        }
+        if (L::kQTiles == 2) add_pv(1, n_max - 1, n_max - 1 >= ntile[0]);
+      } else {
       // P arrives in two halves of 64 keys, so that PV starts while the softmax warps are still exponentiating the
       // second half.  V and the next K are waited for by the first tile that reads them, K under the first half of
       // PV: what stands between P's arrival and the next scores is one wait and the MMAs.
@@ -629,6 +671,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (L::kQTiles == 2 && j < ntile[1]) step(1, j, j >= ntile[0], j + 1 >= ntile[0]);
       }
       }
+      }
     }
     __syncwarp();
   }
@@ -647,7 +690,8 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t tS = tmem_base + lane_addr + wg * kTileN;
     const uint32_t tO = tmem_base + lane_addr + (kAlt ? 384 : L::kOCol + wg * D);
-    const uint32_t tP = kAlt ? tmem_base + lane_addr + 256 + wg * 64 : tS;  // packed fp16 P
+    const uint32_t tP = kAlt ? tmem_base + lane_addr + 256 + wg * 64
+                             : L::kSepP ? tmem_base + lane_addr + L::kPCol + wg * 64 : tS;  // packed fp16 P
     const int nt = kAlt ? ntile[0] : ntile[wg];
     const float c2 = p.scale_log2;
     // kAlt: the reference maximum of a row travels between the two threads that own the row (same
@@ -683,7 +727,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(tS + c * 32, sr[c]);
       tmem_wait_ld();
-      if (kAlt) {  // the scores are in registers: the buffer may take those of key tile j + 2
+      if (kAlt || L::kSepP) {  // the scores are in registers: the buffer may take those of key tile j + 2 (kSepP: j + 1)
         tc_fence_before_sync();
         mbar_arrive(bar(iSFree + wg));
       }
@@ -723,6 +767,10 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
       }
       const float m_new = fmaxf(m_ref, mx);
+      if (L::kSepP && j > 0) {  // P V of the previous step has read P and added to O
+        mbar_wait(bar(iODone + wg), (j - 1) & 1, wctx, kBarODone + wg);
+        tc_fence_after_sync();
+      }
 
       if (j == 0) {
         m_ref = m_new;
@@ -731,7 +779,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (__any_sync(0xffffffffu, need)) {
           // PV of the previous step must have landed before O is touched.
           if (kAlt) mbar_wait(bar(iODone + (wg ^ 1)), ((j - 1) >> 1) & 1, wctx, kBarODone + (wg ^ 1));
-          else mbar_wait(bar(iODone + wg), (j - 1) & 1, wctx, kBarODone + wg);
+          else if (!L::kSepP) mbar_wait(bar(iODone + wg), (j - 1) & 1, wctx, kBarODone + wg);
           tc_fence_after_sync();
           const float alpha = (m_new == kNegInf) ? 1.f : fast_exp2((m_ref - m_new) * c2);
 #pragma unroll
@@ -782,7 +830,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           pk[(i >> 1) + 1] = pack_half2(p2, p3);
         }
         tmem_st_32x32b_x16(tP + c * 16, pk);
-        if (c == 1) {  // the first 64 keys of P are in TMEM: the PV MMA may start on them
+        if (!L::kSepP && c == 1) {  // the first 64 keys of P are in TMEM: the PV MMA may start on them
           tmem_wait_st();
           tc_fence_before_sync();
           mbar_arrive(bar(iPHalf + wg));
