@@ -7,8 +7,12 @@ Usage:  python build.py [--force] [--verbose] [--out PATH] [--define NAME[=VALUE
 the product library.  A library built elsewhere is used through FAL_B200_LIB.
 
 This replaces the reference's torch CUDAExtension build (setup.py:48-82 of
-sirCamp/flash-attention-legacy): there are no torch headers on the native side,
+sirCamp/flash-attention-legacy): there are no torch headers in the library,
 and exactly one target architecture.
+
+Beside it, `lib/_fal_host.so` is the host path of short calls as a Python extension (csrc/fal_host.cpp, g++ with torch's
+headers).  It is tied to the Python and torch it was built with; where it cannot be built or loaded, the binding makes
+the same calls from Python.
 """
 import argparse
 import os
@@ -22,6 +26,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB_PATH = os.path.join(LIB_DIR, "libfal_b200.so")
+HOST_SOURCE = os.path.join(CSRC, "fal_host.cpp")
+HOST_PATH = os.path.join(LIB_DIR, "_fal_host.so")
 
 SOURCES = ["fal_api.cu", "fal_fwd.cu", "fal_bwd.cu", "fal_decode.cu", "fal_ring.cu", "fal_selftest.cu"]
 NVCC_FLAGS = [
@@ -52,14 +58,54 @@ def up_to_date():
     return os.path.exists(LIB_PATH) and os.path.getmtime(LIB_PATH) >= _newest_source_mtime()
 
 
+def _host_up_to_date():
+    inputs = [HOST_SOURCE, os.path.join(HERE, "..", "include", "fal_b200.h"), os.path.abspath(__file__)]
+    return os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= max(os.path.getmtime(p) for p in inputs)
+
+
+def build_host(force=False, verbose=False):
+    """Compiles the host path of short calls.  Returns its path, or None (with a message) where that is not possible."""
+    if not force and _host_up_to_date():
+        return HOST_PATH
+    try:
+        import sysconfig
+
+        from torch.utils import cpp_extension
+        includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"],
+                    os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+        libs = cpp_extension.library_paths()
+    except Exception as e:
+        sys.stderr.write(f"host path not built: {e}\n")
+        return None
+    os.makedirs(LIB_DIR, exist_ok=True)
+    tmp = f"{HOST_PATH}.{os.getpid()}"
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           *(f"-isystem{p}" for p in includes), HOST_SOURCE, "-o", tmp, *(f"-L{p}" for p in libs),
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    try:
+        res = subprocess.run(cmd, capture_output=True, text=True)
+    except OSError as e:
+        sys.stderr.write(f"host path not built: {e}\n")
+        return None
+    if verbose or res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+    if res.returncode != 0:
+        sys.stderr.write("host path not built: short calls are made from Python\n")
+        return None
+    os.replace(tmp, HOST_PATH)
+    return HOST_PATH
+
+
 def build(force=False, verbose=False, out=None, defines=()):
     """Compiles every source file and links the shared library. Returns its path."""
     variant = out is not None or bool(defines)
     lib_path = os.path.abspath(out) if out else LIB_PATH
     if variant and lib_path == LIB_PATH:
         raise RuntimeError("a build with --define needs --out: the product library takes no tuning flags")
-    if not variant and not force and up_to_date():
-        return LIB_PATH
+    if not variant:
+        build_host(force, verbose)
+        if not force and up_to_date():
+            return LIB_PATH
     nvcc = _nvcc()
     obj_dir = OBJ_DIR if not variant else lib_path + ".obj"
     os.makedirs(os.path.dirname(lib_path), exist_ok=True)

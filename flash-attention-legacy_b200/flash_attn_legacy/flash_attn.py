@@ -104,6 +104,10 @@ def flash_attention(
     inputs that are strided views with a contiguous head_dim are read in place, and
     `out_layout="bnhd"` returns the [B,Hq,N,d] result as a view of [B,N,Hq,d] memory.
     """
+    # the ordinary call without gradients in one native function; None: any other, which goes through autograd
+    o = flash_attn_legacy_cuda.forward_plain(q, k, v, softmax_scale, is_causal, out_layout)
+    if o is not None:
+        return o
     assert q.dtype == torch.float16, f"Q must be float16, got {q.dtype}"
     d = q.shape[-1]
     assert d in SUPPORTED_HEAD_DIMS, f"head_dim must be 32, 64, 96, 128, or 256, got {d}"
@@ -267,6 +271,10 @@ def flash_attn_with_kvcache(
     to the end of every entry's keys); it runs on the forward kernel with a key length per entry.
     The reference computes both cases eagerly over the whole cache.
     """
+    if cache_starts is None:  # the ordinary decode step in one native function; None: any other call
+        out = flash_attn_legacy_cuda.decode_plain(q, k_cache, v_cache, k, v, cache_seqlens, softmax_scale, cache_layout)
+        if out is not None:
+            return out
     assert q.dim() == 4, "q must be [B, L_q, H_q, d]"
     assert q.dtype == torch.float16, f"Q must be float16, got {q.dtype}"
     b, lq, hq, d = q.shape

@@ -12,6 +12,8 @@ PyTorch is used only to allocate outputs / workspaces and to hand over raw
 device pointers and the current stream.
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import struct
 
@@ -118,6 +120,35 @@ _lib.fal_set_fwd_variant.argtypes = [_i]
 
 __version__ = _lib.fal_version().decode()
 
+
+def _load_host():
+    """The native host path of short calls (csrc/fal_host.cpp), or None where it was not built for this Python and torch."""
+    path = os.path.join(_HERE, "lib", "_fal_host.so")
+    if not os.path.exists(path):
+        return None
+    loader = importlib.machinery.ExtensionFileLoader("_fal_host", path)
+    try:
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fal_host", loader))
+        loader.exec_module(module)
+    except ImportError:
+        return None
+    address = [ctypes.cast(f, _vp).value for f in (_fwd_run, _decode_run, _lib.fal_decode_workspace_bytes)]
+    return module.Calls(*address, _decode_ws, _DECODE_WS_MIN)
+
+
+def _general(*args):
+    return None
+
+
+# Decode workspaces by (device, stream); the native path reads them too.
+_decode_ws = {}
+_DECODE_WS_MIN = 4 << 20  # what the library uses at most to split a small batch finer than its minimum
+
+_host = _load_host()
+# Each answers None for whatever is not an ordinary call: make it through the functions below.
+forward_plain = _general if _host is None else _host.forward
+decode_plain = _general if _host is None else _host.decode
+
 KERNEL_FWD, KERNEL_BWD, KERNEL_DECODE_SPLITK = 0, 1, 2
 
 
@@ -174,6 +205,8 @@ def _status_word(device):
     if t is None:
         t = torch.zeros(1, dtype=torch.int32, device=device)
         _status[idx] = t
+        if _host is not None:
+            _host.set_status(idx, t.data_ptr())
     return t
 
 
@@ -553,10 +586,6 @@ def scale_cast_f16(src, scale=1.0, out=None):
     _check(_lib.fal_scale_cast_f16(dst.data_ptr(), src.data_ptr(), B, H, N, d, _bhn_strides(dst),
                                    _bhn_strides(src), float(scale), _stream(src)))
     return dst
-
-
-_decode_ws = {}
-_DECODE_WS_MIN = 4 << 20  # what the library uses at most to split a small batch finer than its minimum
 
 
 def _decode_workspace(device, nbytes):
