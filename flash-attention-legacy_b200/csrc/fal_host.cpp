@@ -112,7 +112,10 @@ bool fits_int(std::initializer_list<int64_t> sizes) {
 PyObject* calls_forward(PyObject* self_obj, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   Calls* self = reinterpret_cast<Calls*>(self_obj);
-  if (nargs != 6 || !PyBool_Check(args[4]) || !ordinary_call()) Py_RETURN_NONE;
+  if (nargs != 6 || !PyBool_Check(args[4])) Py_RETURN_NONE;
+  if (!THPVariable_CheckExact(args[0]) || (c10::GradMode::is_enabled() && THPVariable_Unpack(args[0]).requires_grad()))
+    Py_RETURN_NONE;  // (a training step is sent on at once)
+  if (!ordinary_call()) Py_RETURN_NONE;
   const at::Tensor* in[3];
   for (int i = 0; i < 3; ++i) {
     in[i] = plain(args[i], at::kHalf, 4);
@@ -163,12 +166,13 @@ PyObject* calls_forward(PyObject* self_obj, PyObject* const* args, Py_ssize_t na
 PyObject* calls_decode(PyObject* self_obj, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   Calls* self = reinterpret_cast<Calls*>(self_obj);
-  if (nargs != 8 || !ordinary_call()) Py_RETURN_NONE;
+  if (nargs != 8) Py_RETURN_NONE;
   const at::Tensor* q = plain(args[0], at::kHalf, 4);
+  if (q == nullptr || q->size(1) != 1 || !ordinary_call()) Py_RETURN_NONE;  // (a chunk is sent on at once)
   const at::Tensor* kc = plain(args[1], at::kHalf, 4);
   const at::Tensor* vc = plain(args[2], at::kHalf, 4);
   const at::Tensor* lens = plain(args[5], at::kInt, 1);
-  if (!q || !kc || !vc || !lens || q->size(1) != 1 || !q->is_contiguous() || kc->sizes() != vc->sizes()) Py_RETURN_NONE;
+  if (!kc || !vc || !lens || !q->is_contiguous() || kc->sizes() != vc->sizes()) Py_RETURN_NONE;
   const int layout = layout_of(args[7], "bshd", "bhsd");
   const int64_t b = q->size(0), h = q->size(2), d = q->size(3);
   fal_decode_args a{};
