@@ -181,8 +181,8 @@ __device__ __forceinline__ bool bwd_decode_work(const BwdParams& p, int idx, Bwd
     const int s = base + lane;
     int a = 0, e = 0;
     if (s < p.num_seqs) {
-      a = __ldg(p.cu_k + s);
-      e = __ldg(p.cu_k + s + 1);
+      a = p.cu_k[s];
+      e = p.cu_k[s + 1];
     }
     const int nblk = (e - a + kKvTile - 1) / kKvTile;
     int incl = nblk;
@@ -198,8 +198,8 @@ __device__ __forceinline__ bool bwd_decode_work(const BwdParams& p, int idx, Bwd
       w.kvblk = slot - __shfl_sync(0xffffffffu, excl, src);
       w.k_row0 = __shfl_sync(0xffffffffu, a, src);
       w.seqlen_k = __shfl_sync(0xffffffffu, e, src) - w.k_row0;
-      w.q_row0 = __ldg(p.cu_q + base + src);
-      w.seqlen_q = __ldg(p.cu_q + base + src + 1) - w.q_row0;
+      w.q_row0 = p.cu_q[base + src];
+      w.seqlen_q = p.cu_q[base + src + 1] - w.q_row0;
       return true;
     }
     first += __shfl_sync(0xffffffffu, incl, 31);
@@ -288,13 +288,11 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   const int col_own = SPLIT ? static_cast<int>(blockIdx.x & 1) * D : 0;
   const int col_other = SPLIT ? D - col_own : 0;
 
-  BwdWork wk;
-  if (!bwd_decode_work(p, SPLIT ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x), wk)) return;
-
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t sbase = smem_u32(smem_raw);
   uint8_t* sgen = smem_raw;
   if ((sbase & 1023u) != 0) {  // the 128-byte swizzle needs 1024-byte aligned tiles
+    grid_dependency_wait();
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, kDevWaitTimeout + 999);
     return;
   }
@@ -312,17 +310,6 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 
   const int warp = warp_index();
   const int lane = threadIdx.x & 31;
-
-  const int group = p.heads_q / p.heads_kv;
-  const int kv0 = wk.kvblk * kKvTile;                       // local index of the tile's first key
-  const int nqt = (wk.seqlen_q + kQTile - 1) / kQTile;
-  // Keys the causal diagonal is moved by: query i sees keys <= i + cshift (0 = the reference's
-  // top-left-aligned mask; seqlen_k - seqlen_q aligns it to the end of the keys).
-  const int cshift = !CAUSAL ? 0
-                     : (p.cu_k != nullptr ? (p.shift_per_sequence ? wk.seqlen_k - wk.seqlen_q : 0) : p.causal_shift);
-  const int qt0 = CAUSAL ? min(max(kv0 - cshift, 0) / kQTile, nqt) : 0;  // first query tile that sees this key tile
-  const int nq = nqt - qt0;                                  // query tiles per head
-  const int n_iter = group * nq;
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -352,6 +339,21 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     mbar_init(bar(iBFull), 1);
     fence_mbar_init();
   }
+  grid_dependency_wait();  // (up to here the pre-pass may still run)
+  BwdWork wk;
+  if (!bwd_decode_work(p, SPLIT ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x), wk)) return;
+
+  const int group = p.heads_q / p.heads_kv;
+  const int kv0 = wk.kvblk * kKvTile;                       // local index of the tile's first key
+  const int nqt = (wk.seqlen_q + kQTile - 1) / kQTile;
+  // Keys the causal diagonal is moved by: query i sees keys <= i + cshift (0 = the reference's
+  // top-left-aligned mask; seqlen_k - seqlen_q aligns it to the end of the keys).
+  const int cshift = !CAUSAL ? 0
+                     : (p.cu_k != nullptr ? (p.shift_per_sequence ? wk.seqlen_k - wk.seqlen_q : 0) : p.causal_shift);
+  const int qt0 = CAUSAL ? min(max(kv0 - cshift, 0) / kQTile, nqt) : 0;  // first query tile that sees this key tile
+  const int nq = nqt - qt0;                                  // query tiles per head
+  const int n_iter = group * nq;
+
   if (warp == 9) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
     tmem_relinquish();
@@ -464,8 +466,8 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
       for (int rr = 0; rr < kQTile / 32; ++rr) {
         const int64_t row = static_cast<int64_t>(wk.q_row0) + min(fetched + lane + rr * 32, wk.seqlen_q - 1);
-        lse[rr] = __ldg(lse_head + row * p.lse_strides.row);
-        delta[rr] = __ldg(delta_head + row);
+        lse[rr] = lse_head[row * p.lse_strides.row];
+        delta[rr] = delta_head[row];
       }
     };
     if (n_iter > 0) fetch(0);
@@ -961,6 +963,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 // ---------------------------------------------------------------------------
 template <int D>
 __global__ void __launch_bounds__(256) fal_bwd_prep_kernel(const BwdPrepParams p) {
+  grid_dependency_launch();  // the main kernel's blocks set themselves up under this grid's last ones
   constexpr int kLanesPerRow = D / 8;
   constexpr int kRowsPerBlock = 256 / kLanesPerRow;
   const int sub = threadIdx.x % kLanesPerRow;
@@ -1046,27 +1049,24 @@ cudaError_t launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
       [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem); });
   if (e != cudaSuccess) return e;
   if (SPLIT && grid > 0x3fffffff) return cudaErrorInvalidValue;
-  kern<<<SPLIT ? 2 * grid : grid, kBwdThreads, kSmem, stream>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
-  return cudaGetLastError();
+  // Under the pre-pass's last blocks (2 x 8 x 1 024 of 64 causal 22.8 -> 22.4 us; the pre- and the post-pass started in the
+  // same way made that 23.4, and 32 / 8 x 2 987 of 128 256 -> 260).
+  return launch_dependent(kern, dim3(SPLIT ? 2 * grid : grid), dim3(kBwdThreads), kSmem, stream, tq, tk, tv, tdo, tdq, tdk,
+                          tdv, p);
 }
 
 }  // namespace
 
 cudaError_t launch_bwd_prep(const BwdPrepParams& p, cudaStream_t stream) {
   const int64_t total = static_cast<int64_t>(p.batch) * p.heads_q * p.rows;
-  if (p.head_dim == 256) {
-    const int64_t blocks = (total + 7) / 8;
-    fal_bwd_prep_kernel<256><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(p);
-  } else if (p.head_dim == 128) {
-    const int64_t blocks = (total + 15) / 16;
-    fal_bwd_prep_kernel<128><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(p);
-  } else if (p.head_dim == 64) {
-    const int64_t blocks = (total + 31) / 32;
-    fal_bwd_prep_kernel<64><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(p);
-  } else {
-    return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
+  auto launch = [&](auto kern, int rows_per_block) {
+    kern<<<static_cast<unsigned>((total + rows_per_block - 1) / rows_per_block), 256, 0, stream>>>(p);
+    return cudaGetLastError();
+  };
+  if (p.head_dim == 256) return launch(fal_bwd_prep_kernel<256>, 8);
+  if (p.head_dim == 128) return launch(fal_bwd_prep_kernel<128>, 16);
+  if (p.head_dim == 64) return launch(fal_bwd_prep_kernel<64>, 32);
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_bwd(int head_dim, bool causal, const CUtensorMap& tq, const CUtensorMap& tk,
