@@ -140,6 +140,10 @@ struct FwdSmem {
   static constexpr bool kSepP = D == 64 && SHAPE != kOneTile;
   static constexpr int kPCol = kOCol + kQTiles * D;
   static_assert(!kSepP || kPCol + kQTiles * 64 <= kTmemCols, "TMEM columns");
+  // Keys of P that P V starts on.  What is left then stands between P's end and the next scores: with 96 instead of
+  // 64, us: 4 x 32 / 8 x 4 096 causal 502 -> 495, 16 / 4 x 16 384 852 -> 835, 4 x 16 x 2 048 136.8 -> 135.3.  (At head_dim 256, where a step waits for its loads, and with one tile of 128, where the two warpgroups'
+  // products alternate, the later start costs more: 87 -> 92 us on 2 x 16 x 2 048 of 256.)
+  static constexpr int kPFirst = D == 128 && SHAPE == kTwoTiles ? 96 : 64;
   static constexpr int kCtaRows = kQTiles * kTileM;
   static constexpr int kStages = SHAPE == kHalfSm ? 2 : (D == 256) ? 1 : (D == 128) ? 2 : 4;
   static constexpr int kBoxes = D / 64;                 // 64-element (128-byte) column boxes
@@ -545,8 +549,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const uint32_t t_o = L::kAlt ? tmem_base + 384 : tmem_base + L::kOCol + ot * D;
         const uint32_t t_p = L::kAlt ? tmem_base + 256 + sb * 64 : L::kSepP ? tmem_base + L::kPCol + sb * 64 : tmem_base + sb * kTileN;
 #pragma unroll
-        for (int kk = 0; kk < kTileN / 32; ++kk) {
-          const int ks = half * (kTileN / 32) + kk;
+        for (int ks = half == 0 ? 0 : L::kPFirst / 16; ks < (half == 0 ? L::kPFirst : kTileN) / 16; ++ks) {
           umma_ts(t_o, t_p + ks * 8,
                   smem_desc_join(v_lo + ((ks * 2048) >> 4), kHi), idesc_pv,
                   (j > 0 || ks > 0) ? 1u : 0u);
@@ -644,8 +647,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
         if (L::kQTiles == 2) add_pv(1, n_max - 1, n_max - 1 >= ntile[0]);
       } else {
-      // P arrives in two halves of 64 keys, so that PV starts while the softmax warps are still exponentiating the
-      // second half.  V and the next K are waited for by the first tile that reads them, K under the first half of
+      // P arrives in two parts, so that PV starts while the softmax warps are still exponentiating the second.  V and the next K are waited for by the first tile that reads them, K under the first part of
       // PV: what stands between P's arrival and the next scores is one wait and the MMAs.
       auto step = [&](int w, int j, bool first_v, bool first_k) {
         const int s = j % NS, s1 = (j + 1) % NS;
@@ -662,7 +664,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         tc_commit(bar(iODone + w));
         if (w == 1 || j >= ntile[1]) tc_commit(bar(iVEmpty + s));
         if (more) {
-          if (NS == 1) {  // (one K buffer: the next tile may take longer than the second half of P)
+          if (NS == 1) {  // (one K buffer: the next tile may take longer than the rest of P)
             mbar_wait(bar(iKFull + s1), ((j + 1) / NS) & 1, wctx, kBarKFull + s1);
             tc_fence_after_sync();
           }
@@ -835,7 +837,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           pk[(i >> 1) + 1] = pack_half2(p2, p3);
         }
         tmem_st_32x32b_x16(tP + c * 16, pk);
-        if (!L::kSepP && c == 1) {  // the first 64 keys of P are in TMEM: the PV MMA may start on them
+        if (!L::kSepP && c == L::kPFirst / 32 - 1) {  // the first keys of P are in TMEM: the PV MMA may start on them
           tmem_wait_st();
           tc_fence_before_sync();
           mbar_arrive(bar(iPHalf + wg));
