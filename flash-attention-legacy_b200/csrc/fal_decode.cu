@@ -29,6 +29,8 @@
 //     a CUDA graph and 0.797 against 0.787 ms at batch 64.)
 // An optional first position per batch entry (cache_starts) skips a padded prefix
 // of the cache: the entry's row pointers start there and its length shrinks.
+#include <type_traits>
+
 #include "fal_common.h"
 #include "fal_launch.h"
 #include "sm100_ptx.cuh"
@@ -151,10 +153,15 @@ fal_decode_splitk_kernel(const DecodeParams p) {
   const int rows_valid = min(16, group - head_chunk * 16);
   const int hq0 = kv_head * group + head_chunk * 16;  // first query head of this CTA
 
-  // ---- append: the split that holds the new position stores the row, then streams it like any
-  // other (split 0 stores it when the position lies before `start` and nobody attends to it) ----
+  // ---- append: the split that holds the new position stores the row (split 0 does when the position lies before
+  // `start` and nobody attends to it), and streams it from where it came from: read back through L2 it would have to
+  // wait for a load, a store and a fence, at the head of the one CTA that all others then wait for.  us a step on the GPU,
+  // with the statistics and rows of the combine kernel fetched together: 1 entry of 1 999 positions, 32 / 8 heads of 128, 9.1 ->
+  // 7.7 (without a new row 8.2 -> 6.9), 8 of 2 049, 32 / 4 of 64, 8.5 -> 7.0, 16 of 2 000 27.4 -> 26.0.  The choice
+  // of the source stands outside the loop over a slice's loads: in it, it cost every load (3 entries of 8 000, 16 heads
+  // of 64, 30.1 against 20.9). ----
+  const int new_local = can_append ? len_old - start : -1;
   if (can_append) {
-    const int new_local = len_old - start;
     const int store_split = new_local >= 0 ? new_local >> split_shift : 0;
     if (split == store_split) {
       const int real_chunks = p.head_dim_real / 8;  // head_dim 32 / 96 run on the 64 / 128 kernels
@@ -168,8 +175,6 @@ fal_decode_splitk_kernel(const DecodeParams p) {
                       static_cast<int64_t>(len_old) * st.row + cc * 8;
         *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
       }
-      __threadfence();   // the row is read back through L2 by this CTA's asynchronous copies
-      __syncthreads();
     }
   }
   if (pos0 >= len) return;  // this split lies beyond the sequence
@@ -203,6 +208,7 @@ fal_decode_splitk_kernel(const DecodeParams p) {
                         kv_head * p.v_strides.head + static_cast<int64_t>(start) * p.v_strides.row;
   const uint32_t wbase = smem_u32(dec_smem) + warp * L::kWarpBytes;
   const int real_chunks = p.head_dim_real / 8;
+  const int64_t new_row = (static_cast<int64_t>(b) * p.heads_kv + kv_head) * p.head_dim_real;
 
   // Issues the loads of this warp's i-th slice (keys pos0 + (i*4 + warp)*16 ...).
   auto issue_slice = [&](int i) {
@@ -210,19 +216,29 @@ fal_decode_splitk_kernel(const DecodeParams p) {
     if (slice < num_slices) {
       const uint32_t sb = wbase + (i % kDecStages) * L::kStageBytes;
       const int key0 = pos0 + slice * kSliceKeys;
+      auto load = [&](auto with_new) {
 #pragma unroll
-      for (int it = 0; it < kLoadsPerLane; ++it) {
-        const int idx = it * 32 + lane;
-        const int row = idx / kChunks;
-        const int ch = idx % kChunks;
-        const int key = key0 + row;
-        const bool ok = key < pos_end && ch < real_chunks;  // chunks past the tensors' head_dim fill with zeros
-        const int64_t krow = static_cast<int64_t>(key < pos_end ? key : pos0);
-        const int src_ch = ch < real_chunks ? ch : 0;
-        const uint32_t soff = row * L::kRowBytes + ((ch ^ (row & 7)) << 4);
-        cp_async_16_zfill(sb + soff, kbase + krow * p.k_strides.row + src_ch * 8, ok);
-        cp_async_16_zfill(sb + L::kSliceBytes + soff, vbase + krow * p.v_strides.row + src_ch * 8, ok);
-      }
+        for (int it = 0; it < kLoadsPerLane; ++it) {
+          const int idx = it * 32 + lane;
+          const int row = idx / kChunks;
+          const int ch = idx % kChunks;
+          const int key = key0 + row;
+          const bool ok = key < pos_end && ch < real_chunks;  // chunks past the tensors' head_dim fill with zeros
+          const int64_t krow = static_cast<int64_t>(key < pos_end ? key : pos0);
+          const int src_ch = ch < real_chunks ? ch : 0;
+          const uint32_t soff = row * L::kRowBytes + ((ch ^ (row & 7)) << 4);
+          const __half* ks = kbase + krow * p.k_strides.row;
+          const __half* vs = vbase + krow * p.v_strides.row;
+          if (decltype(with_new)::value && krow == new_local) {
+            ks = static_cast<const __half*>(p.k_new) + new_row;
+            vs = static_cast<const __half*>(p.v_new) + new_row;
+          }
+          cp_async_16_zfill(sb + soff, ks + src_ch * 8, ok);
+          cp_async_16_zfill(sb + L::kSliceBytes + soff, vs + src_ch * 8, ok);
+        }
+      };
+      if (new_local >= key0) load(std::true_type{});  // (the entry's last slice: the new row is the last one)
+      else load(std::false_type{});
     }
     cp_async_commit();  // always commit so that group counting stays uniform
   };
@@ -418,6 +434,24 @@ fal_decode_combine_kernel(const DecodeParams p) {
   grid_dependency_wait();
   if (!row_ok) return;  // (whole warps; a block of one row has that row)
 
+  // The first partial rows of this thread are fetched with the statistics, not behind them: one round trip to L2 for three.
+  constexpr int kAhead = 4;
+  const int lane = tid % kLanes;
+  const int grp = tid / kLanes;
+  float mx[kAhead];
+  float4 px[kAhead][kVecs];
+#pragma unroll
+  for (int k = 0; k < kAhead; ++k) {
+    const int i = grp + k * kGroups;
+    mx[k] = kNegInfD;
+#pragma unroll
+    for (int v = 0; v < kVecs; ++v) px[k][v] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < n) {
+      mx[k] = ml[i].x;
+#pragma unroll
+      for (int v = 0; v < kVecs; ++v) px[k][v] = po[static_cast<int64_t>(i) * (D / 4) + v * kLanes + lane];
+    }
+  }
   float m = kNegInfD, l = 0.f;
   for (int i = tid; i < n; i += kThreads) {
     const float2 x = ml[i];
@@ -440,22 +474,28 @@ fal_decode_combine_kernel(const DecodeParams p) {
   const float muse = (m == kNegInfD) ? 0.f : m;
   const float inv = l > 0.f ? 1.f / l : 0.f;
 
-  const int lane = tid % kLanes;
-  const int grp = tid / kLanes;
   float4 o[kVecs];
 #pragma unroll
   for (int v = 0; v < kVecs; ++v) o[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto add_weighted = [&](float4& a, float w, const float4& x) {
+    a.x += w * x.x;
+    a.y += w * x.y;
+    a.z += w * x.z;
+    a.w += w * x.w;
+  };
+#pragma unroll
+  for (int k = 0; k < kAhead; ++k) {
+    if (grp + k * kGroups < n) {
+      const float w = fast_exp2(mx[k] - muse);
+#pragma unroll
+      for (int v = 0; v < kVecs; ++v) add_weighted(o[v], w, px[k][v]);
+    }
+  }
 #pragma unroll 4
-  for (int i = grp; i < n; i += kGroups) {
+  for (int i = grp + kAhead * kGroups; i < n; i += kGroups) {
     const float w = fast_exp2(ml[i].x - muse);
 #pragma unroll
-    for (int v = 0; v < kVecs; ++v) {
-      const float4 x = po[static_cast<int64_t>(i) * (D / 4) + v * kLanes + lane];
-      o[v].x += w * x.x;
-      o[v].y += w * x.y;
-      o[v].z += w * x.z;
-      o[v].w += w * x.w;
-    }
+    for (int v = 0; v < kVecs; ++v) add_weighted(o[v], w, po[static_cast<int64_t>(i) * (D / 4) + v * kLanes + lane]);
   }
   auto add = [&](float4& a, const float4& x) {
     a.x += x.x;
