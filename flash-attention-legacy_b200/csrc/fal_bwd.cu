@@ -77,6 +77,7 @@ struct BwdSmem {
   static constexpr int kQStages = D == 64 ? 3 : 2;             // Q tiles and row statistics
   static constexpr int kDoStages = D == 64 ? 2 : 1;
   static constexpr int kSBuffers = D == 64 ? 2 : 1;            // S^T / P^T blocks in TMEM
+  static constexpr bool kEarlyLoads = D == 64;                 // first tiles requested before the CTA-wide sync
   static constexpr int kBoxes = D / 64;
   static constexpr int kBoxBytes = 128 * 128;                  // one 128-row x 128-byte box
   static constexpr int kTileBytes = kBoxes * kBoxBytes;        // K, V, Q and dO tiles are 128 x D
@@ -111,6 +112,7 @@ struct BwdSplitSmem {
   static constexpr int kQStages = 1;
   static constexpr int kDoStages = 1;
   static constexpr int kSBuffers = 1;
+  static constexpr bool kEarlyLoads = false;
   static constexpr int kBoxes = 2;
   static constexpr int kBoxBytes = 128 * 128;
   static constexpr int kTileBytes = kBoxes * kBoxBytes;
@@ -311,7 +313,7 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
-  if (threadIdx.x == 0) {
+  if (warp == 8 && elect_one()) {
     *abort_flag = 0;
     mbar_init(bar(iKFull), 1);
     mbar_init(bar(iVFull), 1);
@@ -338,6 +340,12 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     mbar_init(bar(iADone), 1);
     mbar_init(bar(iBFull), 1);
     fence_mbar_init();
+    if (L::kEarlyLoads) {
+      tma_prefetch_desc(&tm_k);
+      tma_prefetch_desc(&tm_q);
+      tma_prefetch_desc(&tm_v);
+      tma_prefetch_desc(&tm_do);
+    }
   }
   grid_dependency_wait();  // (up to here the pre-pass may still run)
   BwdWork wk;
@@ -354,6 +362,20 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   const int nq = nqt - qt0;                                  // query tiles per head
   const int n_iter = group * nq;
 
+  // At head_dim 64 the first tiles are on their way before the TMEM allocation and the CTA-wide sync (a microsecond of
+  // the 13 that a CTA of five pairs takes): us, 32 x 16 x 577 261 -> 257, 128 x 16 x 128 causal 142 -> 138, 4 x 16 x 2 048
+  // causal 145 -> 143.  At head_dim 128 the same gave 16 x 16 x 577 196 -> 194 but 4 x 32 / 8 x 4 096 causal 1 355 -> 1 380.
+  auto load_tile = [&](uint32_t dst, const CUtensorMap* map, int b, int row, int head) {
+    mbar_arrive_expect_tx(bar(b), L::kTileBytes);
+    for (int bx = 0; bx < L::kBoxes; ++bx)
+      tma_load_4d(sbase + dst + bx * L::kBoxBytes, map, bar(b), bx * 64, row, head, wk.batch);
+  };
+  if (L::kEarlyLoads && warp == 8 && n_iter > 0 && elect_one()) {
+    load_tile(L::kKOff, &tm_k, iKFull, wk.k_row0 + kv0, wk.kv_head);
+    load_tile(L::kQOff, &tm_q, iQFull, wk.q_row0 + qt0 * kQTile, wk.kv_head * group);
+    load_tile(L::kVOff, &tm_v, iVFull, wk.k_row0 + kv0, wk.kv_head);
+    load_tile(L::kDoOff, &tm_do, iDoFull, wk.q_row0 + qt0 * kQTile, wk.kv_head * group);
+  }
   if (warp == 9) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
     tmem_relinquish();
@@ -417,35 +439,25 @@ fal_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       __syncwarp();
     } else {
       if (n_iter > 0 && elect_one()) {
-        tma_prefetch_desc(&tm_q);
-        tma_prefetch_desc(&tm_k);
-        tma_prefetch_desc(&tm_v);
-        tma_prefetch_desc(&tm_do);
+        if (!L::kEarlyLoads) {
+          tma_prefetch_desc(&tm_q);
+          tma_prefetch_desc(&tm_k);
+          tma_prefetch_desc(&tm_v);
+          tma_prefetch_desc(&tm_do);
+          load_tile(L::kKOff, &tm_k, iKFull, wk.k_row0 + kv0, wk.kv_head);
+          load_tile(L::kVOff, &tm_v, iVFull, wk.k_row0 + kv0, wk.kv_head);
+        }
         tma_prefetch_desc(&tm_dq);
-        mbar_arrive_expect_tx(bar(iKFull), L::kTileBytes);
-        for (int bx = 0; bx < L::kBoxes; ++bx)
-          tma_load_4d(sbase + L::kKOff + bx * L::kBoxBytes, &tm_k, bar(iKFull), bx * 64,
-                      wk.k_row0 + kv0, wk.kv_head, wk.batch);
-        mbar_arrive_expect_tx(bar(iVFull), L::kTileBytes);
-        for (int bx = 0; bx < L::kBoxes; ++bx)
-          tma_load_4d(sbase + L::kVOff + bx * L::kBoxBytes, &tm_v, bar(iVFull), bx * 64,
-                      wk.k_row0 + kv0, wk.kv_head, wk.batch);
-        for (int i = 0; i < n_iter; ++i) {
-          const int st = i % NS;
+        for (int i = L::kEarlyLoads ? 1 : 0; i < n_iter; ++i) {
+          // (where the tiles are is worked out before the wait for their buffer)
+          const int st = i % NS, sd = i % ND;
           const int head = wk.kv_head * group + i / nq;
           const int row = wk.q_row0 + (qt0 + i % nq) * kQTile;
           if (i >= NS) mbar_wait(bar(iQEmpty + st), ((i / NS) - 1) & 1, wctx, kBbQEmpty + st);
-          mbar_arrive_expect_tx(bar(iQFull + st), L::kTileBytes);
-          for (int bx = 0; bx < L::kBoxes; ++bx)
-            tma_load_4d(sbase + L::kQOff + st * L::kTileBytes + bx * L::kBoxBytes, &tm_q,
-                        bar(iQFull + st), bx * 64, row, head, wk.batch);
+          load_tile(L::kQOff + st * L::kTileBytes, &tm_q, iQFull + st, row, head);
           // a dO buffer is reloaded as soon as dV of its last step has read it
-          const int sd = i % ND;
           if (i >= ND) mbar_wait(bar(iDoEmpty + sd), ((i / ND) - 1) & 1, wctx, kBbDoEmpty);
-          mbar_arrive_expect_tx(bar(iDoFull + sd), L::kTileBytes);
-          for (int bx = 0; bx < L::kBoxes; ++bx)
-            tma_load_4d(sbase + L::kDoOff + sd * L::kTileBytes + bx * L::kBoxBytes, &tm_do, bar(iDoFull + sd), bx * 64,
-                        row, head, wk.batch);
+          load_tile(L::kDoOff + sd * L::kTileBytes, &tm_do, iDoFull + sd, row, head);
         }
       }
       __syncwarp();
