@@ -785,6 +785,10 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const bool need = (m_new - m_ref) * c2 > kRescaleThreshold;
         if (__any_sync(0xffffffffu, need)) {
           // PV of the previous step must have landed before O is touched.
+          // (kAlt: this warpgroup does not wait for the other's barrier at every step, and a wait by parity for phase n
+          // passes while phase n - 1 is still open.  Its own last P V, of key tile j - 2, was issued behind that of j - 3: once it
+          // has landed, the other's barrier is in the phase of j - 1.)
+          if (kAlt && j >= 2) mbar_wait(bar(iODone + wg), ((j - 2) >> 1) & 1, wctx, kBarODone + wg);
           if (kAlt) mbar_wait(bar(iODone + (wg ^ 1)), ((j - 1) >> 1) & 1, wctx, kBarODone + (wg ^ 1));
           else if (!L::kSepP) mbar_wait(bar(iODone + wg), (j - 1) & 1, wctx, kBarODone + wg);
           tc_fence_after_sync();
@@ -856,6 +860,8 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 
     // ---- epilogue: O / l -> fp16, LSE -----------------------------------------
     if (nt > 0) {
+      // (the same for the warpgroup that did not take the last key tile)
+      if (kAlt && nt >= 2 && ((nt - 1) & 1) != wg) mbar_wait(bar(iODone + wg), ((nt - 2) >> 1) & 1, wctx, kBarODone + wg);
       if (kAlt) mbar_wait(bar(iODone + ((nt - 1) & 1)), ((nt - 1) >> 1) & 1, wctx, kBarODone + ((nt - 1) & 1));
       else mbar_wait(bar(iODone + wg), (nt - 1) & 1, wctx, kBarODone + wg);
       tc_fence_after_sync();
