@@ -161,7 +161,11 @@ int sm_count() {
 // MMAs and fetch every K / V tile once for 256 query rows; a CTA of one tile (the softmax warpgroups
 // take alternate key tiles of it) takes about 0.6 of the time of a two-tile CTA, measured on grids of
 // many waves.  One tile per CTA is chosen where its larger number of shorter waves finishes first:
-// grids that leave SMs without a two-tile CTA, or that end in a mostly empty wave.
+// grids that leave SMs without a two-tile CTA, or that end in a mostly empty wave.  Under the top-left mask one wave of
+// two-tile CTAs takes as long as its longest, and twice as many CTAs of half the rows even out (us, two tiles / half an
+// SM / one tile): 8 heads x 4 000 of 64 47.8 / 38.1 / 30.5, of 128 55.0 / - / 32.1; 4 x 8 000 89.8 / 70.6 / 54.2, 102 / - / 55.9;
+// 16 x 2 048 26.4 / 21.6 / 19.8, 30.7 / - / 21.6; 16 x 1 100 15.2 / 13.2 / 11.5.  Not on short rows, where a CTA's fixed cost
+// counts: 36 x 1 024 of 64 15.9 / 13.2 / 15.2 (of 128 19.2 / - / 17.3), 60 x 512 10.3 / 9.0 / 11.5 (12.7 / - / 13.3).
 std::atomic<int> g_fwd_variant{FAL_FWD_AUTO};  // fal_set_fwd_variant
 
 // At head_dim 64 the TMEM and shared memory of an SM hold two CTAs of one tile and one softmax warpgroup.
@@ -170,19 +174,18 @@ std::atomic<int> g_fwd_variant{FAL_FWD_AUTO};  // fal_set_fwd_variant
 // tile instead of two, and under a causal mask the upper tile does not wait for the lower.  The price is that every
 // K / V tile is fetched once per 128 query rows.  us, the better of the others against half-SM CTAs (units: batch x
 // heads of 64):
-//   causal: 256 units x 257 rows 30.3 / 21.1, 64 x 577 18.2 / 13.1, 128 x 1 024 47.9 / 43.3, 32 x 1 300 25.1 / 21.8,
-//     256 x 2 600 454 / 423, 128 x 4 000 463 / 456, 256 x 4 000 1 030 / 1 007; 16 x 4 000 58.1 / 59.0;
-//     with at most two per SM, against one tile per CTA, 32 x 1 143 17.4 / 18.2;
-//   no mask, an odd number of 128-row tiles: 256 x 100 10.8 / 7.2, 256 x 257 33.8 / 27.5, 128 x 577 36.6 / 34.5,
-//     640 x 1 300 579 / 577; with at most two CTAs per SM, where the last two tiles of two-tile CTAs run at once just
-//     the same, 64 x 257 10.7 / 11.3, 32 x 577 13.5 / 14.7, 16 x 1 600 26.8 / 29.4;
-//   no mask, an even number: 208 x 145 17.1 / 13.5, 640 x 400 103 / 97, 320 x 696 101.8 / 96.8, but 128 x 400 (3.5 CTAs
-//     per SM) 23.0 / 23.9, 640 x 1 024 310 / 324, 256 x 2 048 429 / 473.
+//   causal: 256 units x 257 rows 26.0 / 19.2, 64 x 577 15.5 / 12.3, 128 x 1 024 41.1 / 37.3, 32 x 1 300 19.6 / 17.9,
+//     256 x 2 600 441 / 402, 64 x 2 048 65.0 / 59.5, 16 x 3 200 38.0 / 34.9, 128 x 4 000 458 / 444; but 16 x 4 000 49.9 / 56.2;
+//   no mask: 256 x 100 10.0 / 6.4, 256 x 257 29.4 / 24.3, 64 x 768 24.2 / 21.0, 512 x 577 118 / 99, 48 x 1 024 29.6 / 25.8,
+//     640 x 1 024 334 / 306, 640 x 1 300 610 / 553, 64 x 2 048 102.5 / 97.0; but 128 x 400 19.9 / 20.3, 256 x 2 048 460 / 462,
+//     16 x 4 096 95 / 105; with at most two CTAs per SM, where the last two tiles of two-tile CTAs run at once just the
+//     same, 64 x 257 10.0 / 10.6, 32 x 577 13.1 / 14.3, 16 x 1 600 23.6 / 26.5.
 // Packed sequences without a mask end in odd and even tiles: 24 of 500 to 1 500 (16 heads) 228 / 218, 200 of 10 to 300
-// 215 / 174, 8 of 2 048 216 / 223.  With one CTA per SM or fewer the alternating warpgroups of the one-tile CTA are faster
-// (16 x 1 024 causal: 12 against 16), for rows of a single tile the half-SM CTA still is (128 x 100: 6.0 / 5.75).  At
-// head_dim 128, the same shape with single K and V buffers measured 89 against 93 us on 16 x 16 x 577 but 665 against
-// 578 on 4 x 32 x 4 096 causal and 116 against 112 on 2 x 32 x 1 500 (64 KB of K and V per tile and CTA); it is not built.
+// 215 / 174, 8 of 2 048 216 / 223 (these before P had columns of its own).  With one CTA per SM or fewer the alternating
+// warpgroups of the one-tile CTA are faster (16 x 1 024 causal: 10.3 against 12.3), for rows of a single tile the half-SM CTA
+// still is (128 x 100: 6.7 / 6.3).  At head_dim 128, the same shape with single K and V buffers measured 89 against 93 us on
+// 16 x 16 x 577 but 665 against 578 on 4 x 32 x 4 096 causal and 116 against 112 on 2 x 32 x 1 500 (64 KB of K and V per
+// tile and CTA); it is not built.
 constexpr int kHalfSmMaxKeys = 2048;
 
 // rows: of every sequence, or 0 for packed sequences of their own lengths; blocks: of 256 and of 128 rows per unit;
@@ -195,12 +198,12 @@ bool half_sm_pays(int rows, int64_t blocks_of_256, int64_t blocks_of_128, int64_
   if (ctas <= sms) return false;
   if (ctas <= 2 * sms) return masked ? !one_tile : blocks_of_256 * units > sms;
   if (masked) return true;
-  if (rows == 0) return mean_keys <= 1024;
-  return blocks_of_128 % 2 != 0 || (mean_keys <= 768 && ctas > (mean_keys <= 256 ? 2 : 4) * sms);
+  return rows > 0 || mean_keys <= 1024;
 }
 
+// triangular: the top-left mask on rows of one length, whose last blocks have twice the average block's keys.
 int forward_variant(int head_dim, int rows, int64_t blocks_of_256, int64_t blocks_of_128, int64_t units,
-                    int64_t mean_keys, bool masked) {
+                    int64_t mean_keys, bool masked, bool triangular) {
   const int forced = g_fwd_variant.load(std::memory_order_relaxed);
   if (head_dim == 256) return FAL_FWD_ONE_TILE;
   if (forced == FAL_FWD_HALF_SM) return head_dim == 64 ? forced : FAL_FWD_TWO_TILES;
@@ -209,6 +212,8 @@ int forward_variant(int head_dim, int rows, int64_t blocks_of_256, int64_t block
   const int64_t ctas2 = blocks_of_256 * units;
   const int64_t waves2 = (ctas2 + sms - 1) / sms;
   const int64_t waves1 = (2 * ctas2 + sms - 1) / sms;
+  if (triangular && (blocks_of_128 * units <= sms || (ctas2 <= sms && rows >= (head_dim == 64 ? 1536 : 640))))
+    return FAL_FWD_ONE_TILE;
   const bool one_tile = 6 * waves1 < 10 * waves2;
   if (head_dim == 64 && half_sm_pays(rows, blocks_of_256, blocks_of_128, units, mean_keys, masked, one_tile, sms))
     return FAL_FWD_HALF_SM;
@@ -418,7 +423,7 @@ int fwd_batched(const void* q, const void* k, const void* v, void* o, float* lse
   const int kdim = kernel_head_dim(head_dim);
   int variant = forward_variant(kdim, seqlen_q, (seqlen_q + 255) / 256, (seqlen_q + 127) / 128,
                                 static_cast<int64_t>(batch) * heads_q, is_causal == 1 ? seqlen_k / 2 : seqlen_k,
-                                is_causal != 0);
+                                is_causal != 0, is_causal == 1 && seqlen_q > 128 && seqlen_k >= seqlen_q);
   p.kv_splits = 1;
   // (the kernel instances of the top-left mask carry no code for a share of the keys; a variant forced by
   // fal_set_fwd_variant runs as it was asked for)
@@ -538,7 +543,7 @@ int fal_fwd_varlen(const void* q, const void* k, const void* v, void* o, float* 
   // extra block each.
   const int kdim = kernel_head_dim(head_dim);
   const int variant = forward_variant(kdim, 0, total_q / 256 + num_seqs, total_q / 128 + num_seqs, heads_q,
-                                      total_k / num_seqs / (is_causal == 1 ? 2 : 1), is_causal != 0);
+                                      total_k / num_seqs / (is_causal == 1 ? 2 : 1), is_causal != 0, false);
   p.half_sm = variant == FAL_FWD_HALF_SM;
   p.cta_rows = variant == FAL_FWD_TWO_TILES ? 256 : 128;
   p.num_qblk = total_q / p.cta_rows + num_seqs;
