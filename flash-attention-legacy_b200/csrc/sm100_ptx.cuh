@@ -366,19 +366,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// exp2 on the FMA / ALU pipes instead of the special-function unit: 2^x = 2^floor(x) * 2^frac(x),
-// frac part by a degree-3 polynomial (max relative error 8.6e-5, below fp16 rounding), integer
-// part added into the exponent field.  Valid for x <= 127; x below -126 (masked scores are -inf)
-// is clamped and yields about 1e-38.
-__device__ __forceinline__ float exp2_fma(float x) {
-  x = fmaxf(x, -126.f);
-  float t;
-  asm("add.rm.ftz.f32 %0, %1, %2;" : "=f"(t) : "f"(x), "f"(12582912.f));  // low mantissa bits = floor(x)
-  const float fr = x - (t - 12582912.f);
-  const float p = fmaf(fmaf(fmaf(0.07706618f, fr, 0.22764593f), fr, 0.69511657f), fr, 1.0f);
-  return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
-}
-
 // ---- packed fp32 pairs (one instruction works on two floats held in a 64-bit register) ----
 __device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
   uint64_t r;
@@ -416,8 +403,10 @@ __device__ __forceinline__ uint64_t exp2_pair_mufu(uint64_t x) {
   return pack_f32x2(fast_exp2(a), fast_exp2(b));
 }
 
-// 2^x for a pair without the special-function unit: exp2_fma's arithmetic with the packed
-// instructions (same polynomial, same clamp).
+// 2^x for a pair on the FMA / ALU pipes instead of the special-function unit: 2^x = 2^floor(x) * 2^frac(x),
+// frac part by a degree-3 polynomial (max relative error 8.6e-5, below fp16 rounding), integer
+// part added into the exponent field.  Valid for x <= 127; x below -126 (masked scores are -inf)
+// is clamped and yields about 1e-38.
 __device__ __forceinline__ uint64_t exp2_pair_fma(uint64_t x) {
   float a, b;
   unpack_f32x2(x, a, b);
@@ -433,13 +422,6 @@ __device__ __forceinline__ uint64_t exp2_pair_fma(uint64_t x) {
   unpack_f32x2(t, t0, t1);
   return pack_f32x2(__int_as_float(__float_as_int(p0) + (__float_as_int(t0) << 23)),
                     __int_as_float(__float_as_int(p1) + (__float_as_int(t1) << 23)));
-}
-
-// Two exponentials per instruction on packed fp16 (input and result are half2 bit patterns).
-__device__ __forceinline__ uint32_t exp2_f16x2(uint32_t x) {
-  uint32_t y;
-  asm("ex2.approx.f16x2 %0, %1;" : "=r"(y) : "r"(x));
-  return y;
 }
 
 // Packed fp16 multiply on half2 bit patterns.
