@@ -10,12 +10,13 @@ This replaces the reference's torch CUDAExtension build (setup.py:48-82 of
 sirCamp/flash-attention-legacy): there are no torch headers in the library,
 and exactly one target architecture.
 
-Beside it, `lib/_fal_host.so` is the host path of short calls as a Python extension (csrc/fal_host.cpp, g++ with torch's
-headers).  It is tied to the Python and torch it was built with; where it cannot be built or loaded, the binding makes
-the same calls from Python.
+Beside it, `lib/_fal_host.<Python>.<torch>.so` is the host path of short calls as a Python extension (csrc/fal_host.cpp,
+g++ with torch's headers).  It is tied to the Python and torch it was built with (fal_host_file.py); where there is none
+for the running ones, the binding makes the same calls from Python.
 """
 import argparse
 import os
+import runpy
 import shutil
 import subprocess
 import sys
@@ -27,7 +28,6 @@ LIB_DIR = os.path.join(HERE, "lib")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB_PATH = os.path.join(LIB_DIR, "libfal_b200.so")
 HOST_SOURCE = os.path.join(CSRC, "fal_host.cpp")
-HOST_PATH = os.path.join(LIB_DIR, "_fal_host.so")
 
 SOURCES = ["fal_api.cu", "fal_fwd.cu", "fal_bwd.cu", "fal_decode.cu", "fal_ring.cu", "fal_selftest.cu"]
 NVCC_FLAGS = [
@@ -58,42 +58,44 @@ def up_to_date():
     return os.path.exists(LIB_PATH) and os.path.getmtime(LIB_PATH) >= _newest_source_mtime()
 
 
-def _host_up_to_date():
+def _host_up_to_date(path):
     inputs = [HOST_SOURCE, os.path.join(HERE, "..", "include", "fal_b200.h"), os.path.abspath(__file__)]
-    return os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= max(os.path.getmtime(p) for p in inputs)
+    return os.path.exists(path) and os.path.getmtime(path) >= max(os.path.getmtime(p) for p in inputs)
 
 
-def build_host(force=False, verbose=False):
-    """Compiles the host path of short calls.  Returns its path, or None (with a message) where that is not possible."""
-    if not force and _host_up_to_date():
-        return HOST_PATH
-    try:
-        import sysconfig
+def _compile_host(path, verbose):
+    import sysconfig
 
-        from torch.utils import cpp_extension
-        includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"],
-                    os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
-        libs = cpp_extension.library_paths()
-    except Exception as e:
-        sys.stderr.write(f"host path not built: {e}\n")
-        return None
-    os.makedirs(LIB_DIR, exist_ok=True)
-    tmp = f"{HOST_PATH}.{os.getpid()}"
+    from torch.utils import cpp_extension
+    includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"],
+                os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    os.makedirs(os.path.dirname(path), exist_ok=True)
+    tmp = f"{path}.{os.getpid()}"
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           *(f"-isystem{p}" for p in includes), HOST_SOURCE, "-o", tmp, *(f"-L{p}" for p in libs),
+           *(f"-isystem{p}" for p in includes), HOST_SOURCE, "-o", tmp, *(f"-L{p}" for p in cpp_extension.library_paths()),
            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
-    try:
-        res = subprocess.run(cmd, capture_output=True, text=True)
-    except OSError as e:
-        sys.stderr.write(f"host path not built: {e}\n")
-        return None
+    res = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)
     if res.returncode != 0:
-        sys.stderr.write("host path not built: short calls are made from Python\n")
+        raise RuntimeError(f"{cmd[0]} failed on fal_host.cpp")
+    os.replace(tmp, path)
+
+
+def build_host(force=False, verbose=False):
+    """Compiles the host path of short calls.  Returns its path, or None (with a message) where that is not possible;
+    a file of older sources does not stay behind then, as the binding would load it beside the newer library."""
+    path = None
+    try:
+        path = runpy.run_path(os.path.join(HERE, "fal_host_file.py"))["host_path"](LIB_DIR)
+        if force or not _host_up_to_date(path):
+            _compile_host(path, verbose)
+        return path
+    except Exception as e:
+        sys.stderr.write(f"host path not built, short calls are made from Python: {e}\n")
+        if path is not None and os.path.exists(path) and not _host_up_to_date(path):
+            os.remove(path)
         return None
-    os.replace(tmp, HOST_PATH)
-    return HOST_PATH
 
 
 def build(force=False, verbose=False, out=None, defines=()):

@@ -291,7 +291,10 @@ PyMODINIT_FUNC PyInit__fal_host() {
   if (PyType_Ready(&calls_type) < 0) return nullptr;
   PyObject* m = PyModule_Create(&module_def);
   if (m == nullptr) return nullptr;
-  if (PyModule_AddObjectRef(m, "Calls", reinterpret_cast<PyObject*>(&calls_type)) < 0) {
+  // sizes of the argument blocks it was compiled with
+  if (PyModule_AddObjectRef(m, "Calls", reinterpret_cast<PyObject*>(&calls_type)) < 0 ||
+      PyModule_AddIntConstant(m, "FWD_ARGS_BYTES", sizeof(fal_fwd_args)) < 0 ||
+      PyModule_AddIntConstant(m, "DECODE_ARGS_BYTES", sizeof(fal_decode_args)) < 0) {
     Py_DECREF(m);
     return nullptr;
   }

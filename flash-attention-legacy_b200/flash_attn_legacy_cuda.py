@@ -121,17 +121,25 @@ _lib.fal_set_fwd_variant.argtypes = [_i]
 __version__ = _lib.fal_version().decode()
 
 
+def _load(name, loader_type, path):
+    loader = loader_type(name, path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader(name, loader))
+    loader.exec_module(module)
+    return module
+
+
 def _load_host():
     """The native host path of short calls (csrc/fal_host.cpp), or None where it was not built for this Python and torch."""
-    path = os.path.join(_HERE, "lib", "_fal_host.so")
+    names = _load("fal_host_file", importlib.machinery.SourceFileLoader, os.path.join(_HERE, "fal_host_file.py"))
+    path = names.host_path(os.path.join(_HERE, "lib"))
     if not os.path.exists(path):
         return None
-    loader = importlib.machinery.ExtensionFileLoader("_fal_host", path)
     try:
-        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fal_host", loader))
-        loader.exec_module(module)
+        module = _load("_fal_host", importlib.machinery.ExtensionFileLoader, path)
     except ImportError:
         return None
+    if (module.FWD_ARGS_BYTES, module.DECODE_ARGS_BYTES) != (_FWD_ARGS.size, _DECODE_ARGS.size):
+        return None  # built with another header than this binding is written for
     address = [ctypes.cast(f, _vp).value for f in (_fwd_run, _decode_run, _lib.fal_decode_workspace_bytes)]
     return module.Calls(*address, _decode_ws, _DECODE_WS_MIN)
 
