@@ -156,10 +156,13 @@ fal_decode_splitk_kernel(const DecodeParams p) {
   // ---- append: the split that holds the new position stores the row (split 0 does when the position lies before
   // `start` and nobody attends to it), and streams it from where it came from: read back through L2 it would have to
   // wait for a load, a store and a fence, at the head of the one CTA that all others then wait for.  us a step on the GPU,
-  // with the statistics and rows of the combine kernel fetched together: 1 entry of 1 999 positions, 32 / 8 heads of 128, 9.1 ->
-  // 7.7 (without a new row 8.2 -> 6.9), 8 of 2 049, 32 / 4 of 64, 8.5 -> 7.0, 16 of 2 000 27.4 -> 26.0.  The choice
-  // of the source stands outside the loop over a slice's loads: in it, it cost every load (3 entries of 8 000, 16 heads
-  // of 64, 30.1 against 20.9). ----
+  // with the statistics and rows of the combine kernel fetched together: 1 entry of 1 999 positions, 32 / 8 heads of 128,
+  // 9.1 -> 7.7 (without a new row 8.2 -> 6.9), 8 of 2 049, 32 / 4 of 64, 8.5 -> 7.0, 16 of 2 000 27.4 -> 26.0.
+  // Only the slice that holds the row chooses between two sources.  With the choice in all of an entry's slices: 1 entry of
+  // 1 999 7.6 -> 7.2, 3 of 8 000, 16 heads of 64, 22.4 -> 20.7, 4 of 3 000 of 256 29.7 -> 25.7, 32 of 1 000, 32 / 32 of 96,
+  // 87 -> 79, 64 of 5 000 220 -> 207, 64 of 1 024 to 32 512 765 -> 685: what the same steps take without a new row.  (It is
+  // not the compare alone: a kernel of its own for steps without a new row, which has one form of the loads, was as slow
+  // again, 207 -> 217, with 167 registers instead of 224.) ----
   const int new_local = can_append ? len_old - start : -1;
   if (can_append) {
     const int store_split = new_local >= 0 ? new_local >> split_shift : 0;
@@ -237,8 +240,8 @@ fal_decode_splitk_kernel(const DecodeParams p) {
           cp_async_16_zfill(sb + L::kSliceBytes + soff, vs + src_ch * 8, ok);
         }
       };
-      if (new_local >= key0) load(std::true_type{});  // (the entry's last slice: the new row is the last one)
-      else load(std::false_type{});
+      if (static_cast<unsigned>(new_local - key0) >= kSliceKeys) load(std::false_type{});
+      else load(std::true_type{});  // (the slice that holds the new row)
     }
     cp_async_commit();  // always commit so that group counting stays uniform
   };
