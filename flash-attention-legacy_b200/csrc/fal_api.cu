@@ -172,33 +172,53 @@ std::atomic<int> g_fwd_variant{FAL_FWD_AUTO};  // fal_set_fwd_variant
 // They overlap as the two tiles of a two-tile CTA do, and each one's prologue and epilogue run under the
 // other's main loop besides, which is what short rows spend their time on; a sequence ends in at most one partial
 // tile instead of two, and under a causal mask the upper tile does not wait for the lower.  The price is that every
-// K / V tile is fetched once per 128 query rows.  us, the better of the others against half-SM CTAs (units: batch x
-// heads of 64):
-//   causal: 256 units x 257 rows 26.0 / 19.2, 64 x 577 15.5 / 12.3, 128 x 1 024 41.1 / 37.3, 32 x 1 300 19.6 / 17.9,
-//     256 x 2 600 441 / 402, 64 x 2 048 65.0 / 59.5, 16 x 3 200 38.0 / 34.9, 128 x 4 000 458 / 444; but 16 x 4 000 49.9 / 56.2;
-//   no mask: 256 x 100 10.0 / 6.4, 256 x 257 29.4 / 24.3, 64 x 768 24.2 / 21.0, 512 x 577 118 / 99, 48 x 1 024 29.6 / 25.8,
-//     640 x 1 024 334 / 306, 640 x 1 300 610 / 553, 64 x 2 048 102.5 / 97.0; but 128 x 400 19.9 / 20.3, 256 x 2 048 460 / 462,
-//     16 x 4 096 95 / 105; with at most two CTAs per SM, where the last two tiles of two-tile CTAs run at once just the
-//     same, 64 x 257 10.0 / 10.6, 32 x 577 13.1 / 14.3, 16 x 1 600 23.6 / 26.5.
-// Packed sequences without a mask end in odd and even tiles: 24 of 500 to 1 500 (16 heads) 228 / 218, 200 of 10 to 300
-// 215 / 174, 8 of 2 048 216 / 223 (these before P had columns of its own).  With one CTA per SM or fewer the alternating
-// warpgroups of the one-tile CTA are faster (16 x 1 024 causal: 10.3 against 12.3), for rows of a single tile the half-SM CTA
-// still is (128 x 100: 6.7 / 6.3).  At head_dim 128, the same shape with single K and V buffers measured 89 against 93 us on
-// 16 x 16 x 577 but 665 against 578 on 4 x 32 x 4 096 causal and 116 against 112 on 2 x 32 x 1 500 (64 KB of K and V per
-// tile and CTA); it is not built.
-constexpr int kHalfSmMaxKeys = 2048;
+// K / V tile is fetched once per 128 query rows.  us, units (batch x heads of 64) x rows, one tile per CTA / two tiles /
+// half-SM CTAs:
+//   one per SM or fewer: the alternating warpgroups of the one-tile CTA are faster (16 x 1 024 causal 10.3 / - / 12.3), but
+//     for rows of a single tile (128 x 100: 6.7 / - / 6.3);
+//   up to two per SM under a mask: 81 x 257 10.8 / 12.9 / 8.0, 54 x 577 12.6 / 13.3 / 10.3, 32 x 1 143 16.0 / 15.7 / 14.2,
+//     22 x 1 640 18.9 / 21.2 / 18.6; long rows 17 x 2 100 21.9 / 26.7 / 22.8, 14 x 2 650 25.2 / 32.3 / 27.3;
+//   more of them under a mask: 100 x 400 17.1 / 15.6 / 13.3, 96 x 1 024 40.8 / 31.6 / 28.8, 48 x 2 600 84.1 / 73.8 / 69.0,
+//     48 x 4 000 175 / 148 / 145; but long rows that are one and a half to two waves of either are balanced best as
+//     two-tile CTAs, heavy ones first: 36 x 1 700 34.8 / 27.9 / 30.1, 32 x 2 048 38.2 / 30.7 / 33.3, 24 x 3 000 52.4 / 44.3 / 49.1,
+//     16 x 4 000 58.0 / 49.5 / 56.0 (an odd number of tiles, the last two-tile CTA half empty, only from 19 on: 27 x 2 100
+//     35.9 / 32.6 / 31.3, 24 x 2 900 49.7 / 44.0 / 46.2); shorter rows are not: 40 x 1 600 34.2 / 30.2 / 29.1;
+//   no mask, all CTAs equal: faster where the last wave leaves SMs to one CTA or saves a wave of half-empty two-tile CTAs
+//     (50 x 1 024 29.6 / 29.5 / 25.8, 96 x 577 30.8 / 22.7 / 23.5 but 109 x 577 31.7 / 30.6 / 23.9, 25 x 2 048
+//     48.1 / 51.2 / 45.5, 252 x 1 024 142 / 108 / 105), slower where it is nearly full, the more so the longer the rows and
+//     the fewer the waves: 96 x 700 of two waves 33.9 / 25.8 / 27.1, 32 x 2 048 62.8 / 51.9 / 56.1, of three 107 x 1 024
+//     58.1 / 45.3 / 46.4, 54 x 2 048 94.3 / 77.7 / 82.8, of five 88 x 2 048 162 / 130 / 136; even at 144 x 400 of two
+//     27.3 / 20.1 / 20.5, 215 x 400 of three 40.2 / 29.6 / 29.4, 176 x 1 024 of five 101 / 76.6 / 75.5.
+//   packed sequences (of, heads), whose last tiles come as they come: causal 24 of 500 to 1 500, 16, 182 / 142 / 128, 8 of 2 048
+//     153 / 122 / 119; no mask 24 of 500 to 1 500 244 / 191 / 183, 12 of 1 400 to 1 900 275 / 229 / 220, 16 of 1 500 to 2 500
+//     427 / 346 / 347, 8 of 2 048 232 / 185 / 190.
+// At head_dim 128, the same shape with single K and V buffers measured 89 against 93 us on 16 x 16 x 577 but 665 against
+// 578 on 4 x 32 x 4 096 causal and 116 against 112 on 2 x 32 x 1 500 (64 KB of K and V per tile and CTA); it is not built.
+constexpr int kHalfSmMaxKeys = 2048;        // a row sees on average; beyond, within 3 % of two tiles or slower
+constexpr int kHalfSmMaxPackedKeys = 1792;  // without a mask
+constexpr int kOneTileRows = 1920;          // from here on one-tile CTAs, up to two half-SM CTAs per SM
+constexpr int kHalfSmKeysPerWave = 384;     // fewer for each wave after the first: a nearly full last wave does not matter
 
 // rows: of every sequence, or 0 for packed sequences of their own lengths; blocks: of 256 and of 128 rows per unit;
 // one_tile: the better of the other two shapes.
 bool half_sm_pays(int rows, int64_t blocks_of_256, int64_t blocks_of_128, int64_t units, int64_t mean_keys, bool masked,
                   bool one_tile, int64_t sms) {
-  if (mean_keys > kHalfSmMaxKeys || 2 * blocks_of_256 * units <= sms) return false;
-  const int64_t ctas = blocks_of_128 * units;
+  const int64_t ctas = blocks_of_128 * units, ctas2 = blocks_of_256 * units;
+  if (mean_keys > kHalfSmMaxKeys || 2 * ctas2 <= sms) return false;
   if (rows > 0 && rows <= 128) return true;
   if (ctas <= sms) return false;
-  if (ctas <= 2 * sms) return masked ? !one_tile : blocks_of_256 * units > sms;
-  if (masked) return true;
-  return rows > 0 || mean_keys <= 1024;
+  if (ctas <= 2 * sms && (masked || rows == 0)) {
+    const bool long_rows = (rows > 0 ? rows : 2 * mean_keys) >= kOneTileRows;
+    return masked ? !one_tile || (ctas2 > sms && !long_rows) : ctas2 > sms;
+  }
+  if (rows == 0) return masked || mean_keys <= kHalfSmMaxPackedKeys;
+  if (masked) {
+    const bool long_rows = blocks_of_128 >= (blocks_of_128 % 2 == 0 ? 14 : 19);
+    return !long_rows || ctas <= 3 * sms || ctas2 > 2 * sms;
+  }
+  const int64_t waves = (ctas + 2 * sms - 1) / (2 * sms);
+  const bool last_wave_doubled = ctas - (waves - 1) * 2 * sms > sms;
+  return !last_wave_doubled || ctas2 > waves * sms || mean_keys < kHalfSmKeysPerWave * (waves - 1);
 }
 
 // triangular: the top-left mask on rows of one length, whose last blocks have twice the average block's keys.

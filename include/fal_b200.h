@@ -98,11 +98,11 @@ FAL_API int fal_fwd(const void* q, const void* k, const void* v, void* o, float*
  *                            two-tile grid would leave SMs without a block or end in a thin wave;
  *   FAL_FWD_HALF_SM          (head_dim 32 and 64) one tile, one softmax warpgroup, two blocks per SM: a block's
  *                            prologue and epilogue run under the other block's main loop.
- * FAL_FWD_AUTO (default) chooses per call (half-SM blocks at head_dim 32 and 64 when there is more than one per
- * SM and the rows see 2 048 keys or fewer on average -- without a mask only where two-tile blocks would leave tiles
- * empty or the rows are short; else one tile when its waves, at 0.6 of a two-tile wave each, finish first; head_dim
- * 256 always runs one tile).  fal_set_fwd_variant forces a variant for
- * every later call in the process: a tuning and test control -- the results agree within rounding.
+ * FAL_FWD_AUTO (default) chooses per call: half-SM blocks at head_dim 32 and 64 where the rows see 2 048 keys or
+ * fewer on average and there is more than one such block per SM, unless the last wave of two-tile blocks is nearly
+ * full; else one tile when its waves, at 0.6 of a two-tile wave each, finish first; head_dim 256 always runs one tile.
+ * fal_set_fwd_variant forces a variant for every later call in the process: a tuning and test control -- the results
+ * agree within rounding.
  * The reference picks tile sizes from a compile-time table per architecture instead
  * (csrc/include/flash_attn_common.h:157-292).
  */
