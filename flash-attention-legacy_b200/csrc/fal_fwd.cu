@@ -72,23 +72,10 @@ constexpr float kNegInf = -INFINITY;
 // Skip the O rescale while the running maximum grows by less than 2^8.
 constexpr float kRescaleThreshold = 8.0f;
 
-// The softmax arithmetic -- scale-and-subtract, the row sums and (for a share of the pairs) the
-// exponential itself -- runs as two-float instructions.  FAL_FWD_EMU_PAIRS of every 4 pairs take the
-// polynomial path on the FMA pipe instead of the special-function unit (0 = none: measured slower
-// with 1, the kernel is bound by dependency latency, not by the special-function unit).
-#ifndef FAL_FWD_EMU_PAIRS
-#define FAL_FWD_EMU_PAIRS 0
-#endif
-template <int K>
-__device__ __forceinline__ uint64_t tile_exp2_pair(int i, uint64_t x) {
-  // pair index within its group of four; i is a multiple of 4 under full unrolling
-  const int q = ((i >> 1) + K) & 3;
-  const bool emu = (FAL_FWD_EMU_PAIRS == 1) ? (q == 0)
-                 : (FAL_FWD_EMU_PAIRS == 2) ? ((q & 1) == 0)
-                 : (FAL_FWD_EMU_PAIRS == 3) ? (q != 3)
-                 : (FAL_FWD_EMU_PAIRS >= 4);
-  return emu ? exp2_pair_fma(x) : exp2_pair_mufu(x);
-}
+// The softmax arithmetic -- scale-and-subtract, the row sums -- runs as two-float instructions, the exponentials on
+// the special-function unit.  (One of every four pairs as a polynomial on the FMA pipe is slower at head_dim 128, whose
+// steps are bound by latency; at 64, where that unit is the bound, 4 x 16 x 2 048 of 64 went from 101.9 to 99.6 us, but with
+// a larger error: not built.)
 
 // Register split after launch (setmaxnreg).  The kernel launches with 168 registers for each of
 // its 384 threads = 64512; the two softmax warpgroups and the third warpgroup must not ask for
@@ -141,8 +128,9 @@ struct FwdSmem {
   static constexpr int kPCol = kOCol + kQTiles * D;
   static_assert(!kSepP || kPCol + kQTiles * 64 <= kTmemCols, "TMEM columns");
   // Keys of P that P V starts on.  What is left then stands between P's end and the next scores: with 96 instead of
-  // 64, us: 4 x 32 / 8 x 4 096 causal 502 -> 495, 16 / 4 x 16 384 852 -> 835, 4 x 16 x 2 048 136.8 -> 135.3.  (At head_dim 256, where a step waits for its loads, and with one tile of 128, where the two warpgroups'
-  // products alternate, the later start costs more: 87 -> 92 us on 2 x 16 x 2 048 of 256.)
+  // 64, us: 4 x 32 / 8 x 4 096 causal 502 -> 495, 16 / 4 x 16 384 852 -> 835, 4 x 16 x 2 048 136.8 -> 135.3.
+  // (At head_dim 256, where a step waits for its loads, and with one tile of 128, where the two warpgroups' products
+  // alternate, the later start costs more: 87 -> 92 us on 2 x 16 x 2 048 of 256.)
   static constexpr int kPFirst = D == 128 && SHAPE == kTwoTiles ? 96 : 64;
   static constexpr int kCtaRows = kQTiles * kTileM;
   static constexpr int kStages = SHAPE == kHalfSm ? 2 : (D == 256) ? 1 : (D == 128) ? 2 : 4;
@@ -547,7 +535,7 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       auto issue_pv = [&](int sb, int ot, int j, int half) {
         const uint32_t v_lo = smem_desc_lo(sbase + L::kVOff + (j % NS) * L::kTileBytes, L::kBoxBytes);
         const uint32_t t_o = L::kAlt ? tmem_base + 384 : tmem_base + L::kOCol + ot * D;
-        const uint32_t t_p = L::kAlt ? tmem_base + 256 + sb * 64 : L::kSepP ? tmem_base + L::kPCol + sb * 64 : tmem_base + sb * kTileN;
+        const uint32_t t_p = tmem_base + (L::kAlt ? 256 + sb * 64 : L::kSepP ? L::kPCol + sb * 64 : sb * kTileN);
 #pragma unroll
         for (int ks = half == 0 ? 0 : L::kPFirst / 16; ks < (half == 0 ? L::kPFirst : kTileN) / 16; ++ks) {
           umma_ts(t_o, t_p + ks * 8,
@@ -647,36 +635,37 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
         if (L::kQTiles == 2) add_pv(1, n_max - 1, n_max - 1 >= ntile[0]);
       } else {
-      // P arrives in two parts, so that PV starts while the softmax warps are still exponentiating the second.  V and the next K are waited for by the first tile that reads them, K under the first part of
-      // PV: what stands between P's arrival and the next scores is one wait and the MMAs.
-      auto step = [&](int w, int j, bool first_v, bool first_k) {
-        const int s = j % NS, s1 = (j + 1) % NS;
-        const bool more = j + 1 < ntile[w];
-        if (first_v) mbar_wait(bar(iVFull + s), (j / NS) & 1, wctx, kBarVFull + s);
-        if (v_fix && j == n_max - 1) mbar_wait(bar(iVFixed), 0, wctx, kBarVFull + s);
-        mbar_wait(bar(iPHalf + w), j & 1, wctx, kBarPReady + w);
-        tc_fence_after_sync();
-        issue_pv(w, w, j, 0);
-        if (NS > 1 && more && first_k) mbar_wait(bar(iKFull + s1), ((j + 1) / NS) & 1, wctx, kBarKFull + s1);
-        mbar_wait(bar(iPReady + w), j & 1, wctx, kBarPReady + w);
-        tc_fence_after_sync();
-        issue_pv(w, w, j, 1);
-        tc_commit(bar(iODone + w));
-        if (w == 1 || j >= ntile[1]) tc_commit(bar(iVEmpty + s));
-        if (more) {
-          if (NS == 1) {  // (one K buffer: the next tile may take longer than the rest of P)
-            mbar_wait(bar(iKFull + s1), ((j + 1) / NS) & 1, wctx, kBarKFull + s1);
-            tc_fence_after_sync();
+        // P arrives in two parts, so that PV starts while the softmax warps are still exponentiating the second.  V and
+        // the next K are waited for by the first tile that reads them, K under the first part of PV: what stands between
+        // P's arrival and the next scores is one wait and the MMAs.
+        auto step = [&](int w, int j, bool first_v, bool first_k) {
+          const int s = j % NS, s1 = (j + 1) % NS;
+          const bool more = j + 1 < ntile[w];
+          if (first_v) mbar_wait(bar(iVFull + s), (j / NS) & 1, wctx, kBarVFull + s);
+          if (v_fix && j == n_max - 1) mbar_wait(bar(iVFixed), 0, wctx, kBarVFull + s);
+          mbar_wait(bar(iPHalf + w), j & 1, wctx, kBarPReady + w);
+          tc_fence_after_sync();
+          issue_pv(w, w, j, 0);
+          if (NS > 1 && more && first_k) mbar_wait(bar(iKFull + s1), ((j + 1) / NS) & 1, wctx, kBarKFull + s1);
+          mbar_wait(bar(iPReady + w), j & 1, wctx, kBarPReady + w);
+          tc_fence_after_sync();
+          issue_pv(w, w, j, 1);
+          tc_commit(bar(iODone + w));
+          if (w == 1 || j >= ntile[1]) tc_commit(bar(iVEmpty + s));
+          if (more) {
+            if (NS == 1) {  // (one K buffer: the next tile may take longer than the rest of P)
+              mbar_wait(bar(iKFull + s1), ((j + 1) / NS) & 1, wctx, kBarKFull + s1);
+              tc_fence_after_sync();
+            }
+            issue_qk(w, w, j + 1);
+            tc_commit(bar(iSReady + w));
+            if (w == 1 || j + 1 >= ntile[1]) tc_commit(bar(iKEmpty + s1));
           }
-          issue_qk(w, w, j + 1);
-          tc_commit(bar(iSReady + w));
-          if (w == 1 || j + 1 >= ntile[1]) tc_commit(bar(iKEmpty + s1));
+        };
+        for (int j = 0; j < n_max; ++j) {
+          if (j < ntile[0]) step(0, j, true, true);
+          if (L::kQTiles == 2 && j < ntile[1]) step(1, j, j >= ntile[0], j + 1 >= ntile[0]);
         }
-      };
-      for (int j = 0; j < n_max; ++j) {
-        if (j < ntile[0]) step(0, j, true, true);
-        if (L::kQTiles == 2 && j < ntile[1]) step(1, j, j >= ntile[0], j + 1 >= ntile[0]);
-      }
       }
       }
     }
@@ -830,8 +819,8 @@ fal_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                                      c2p, moffp);
           const uint64_t x23 = ffma2(pack_f32x2(__uint_as_float(sr[c][i + 2]), __uint_as_float(sr[c][i + 3])),
                                      c2p, moffp);
-          const uint64_t p01 = tile_exp2_pair<0>(i, x01);
-          const uint64_t p23 = tile_exp2_pair<1>(i, x23);
+          const uint64_t p01 = exp2_pair(x01);
+          const uint64_t p23 = exp2_pair(x23);
           sum_a = fadd2(sum_a, p01);
           sum_b = fadd2(sum_b, p23);
           float p0, p1, p2, p3;

@@ -46,9 +46,10 @@ __device__ __forceinline__ void grid_dependency_wait() {
 // True in one lane of a converged warp, the same one every time.  The instructions that one thread issues (tcgen05.mma,
 // commits, TMA) take their descriptors from uniform registers: behind this test the compiler knows that a single lane
 // runs and moves them there directly.  Behind `lane == 0` it does not: each tcgen05.mma then took the issuing thread about
-// 60 cycles, as long as the tensor pipe takes to run it, so that nothing queued up while the thread waited on barriers (cycle counters:
-// four M128 N128 K16 instructions in 230 to 270 cycles, now in 30).  us on the GPU, `lane == 0` -> elected: forward 32 / 8
-// heads x 2 987 of 128 causal 80.8 -> 75.6, 4 x 16 x 2 048 of 64 118.6 -> 112.8; backward 16 x 16 384 of 64 1 811 -> 1 721.
+// 60 cycles, as long as the tensor pipe takes to run it, so that nothing queued up while the thread waited on barriers
+// (cycle counters: four M128 N128 K16 instructions in 230 to 270 cycles, now in 30).  us on the GPU, `lane == 0` ->
+// elected: forward 32 / 8 heads x 2 987 of 128 causal 80.8 -> 75.6, 4 x 16 x 2 048 of 64 118.6 -> 112.8; backward
+// 16 x 16 384 of 64 1 811 -> 1 721.
 __device__ __forceinline__ bool elect_one() {
   uint32_t leader;
   asm volatile(
@@ -385,43 +386,12 @@ __device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-__device__ __forceinline__ uint64_t fsub2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t fadd2_round_down(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rm.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
 
 // 2^x for a pair, on the special-function unit.
-__device__ __forceinline__ uint64_t exp2_pair_mufu(uint64_t x) {
+__device__ __forceinline__ uint64_t exp2_pair(uint64_t x) {
   float a, b;
   unpack_f32x2(x, a, b);
   return pack_f32x2(fast_exp2(a), fast_exp2(b));
-}
-
-// 2^x for a pair on the FMA / ALU pipes instead of the special-function unit: 2^x = 2^floor(x) * 2^frac(x),
-// frac part by a degree-3 polynomial (max relative error 8.6e-5, below fp16 rounding), integer
-// part added into the exponent field.  Valid for x <= 127; x below -126 (masked scores are -inf)
-// is clamped and yields about 1e-38.
-__device__ __forceinline__ uint64_t exp2_pair_fma(uint64_t x) {
-  float a, b;
-  unpack_f32x2(x, a, b);
-  x = pack_f32x2(fmaxf(a, -126.f), fmaxf(b, -126.f));
-  const uint64_t magic = pack_f32x2(12582912.f, 12582912.f);
-  const uint64_t t = fadd2_round_down(x, magic);  // low mantissa bits = floor(x)
-  const uint64_t fr = fsub2(x, fsub2(t, magic));
-  uint64_t pl = ffma2(pack_f32x2(0.07706618f, 0.07706618f), fr, pack_f32x2(0.22764593f, 0.22764593f));
-  pl = ffma2(pl, fr, pack_f32x2(0.69511657f, 0.69511657f));
-  pl = ffma2(pl, fr, pack_f32x2(1.0f, 1.0f));
-  float p0, p1, t0, t1;
-  unpack_f32x2(pl, p0, p1);
-  unpack_f32x2(t, t0, t1);
-  return pack_f32x2(__int_as_float(__float_as_int(p0) + (__float_as_int(t0) << 23)),
-                    __int_as_float(__float_as_int(p1) + (__float_as_int(t1) << 23)));
 }
 
 // Packed fp16 multiply on half2 bit patterns.
