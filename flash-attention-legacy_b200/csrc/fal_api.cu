@@ -189,14 +189,17 @@ std::atomic<int> g_fwd_variant{FAL_FWD_AUTO};  // fal_set_fwd_variant
 //     the fewer the waves: 96 x 700 of two waves 33.9 / 25.8 / 27.1, 32 x 2 048 62.8 / 51.9 / 56.1, of three 107 x 1 024
 //     58.1 / 45.3 / 46.4, 54 x 2 048 94.3 / 77.7 / 82.8, of five 88 x 2 048 162 / 130 / 136; even at 144 x 400 of two
 //     27.3 / 20.1 / 20.5, 215 x 400 of three 40.2 / 29.6 / 29.4, 176 x 1 024 of five 101 / 76.6 / 75.5.
-//   packed sequences (of, heads), whose last tiles come as they come: causal 24 of 500 to 1 500, 16, 182 / 142 / 128, 8 of 2 048
-//     153 / 122 / 119; no mask 24 of 500 to 1 500 244 / 191 / 183, 12 of 1 400 to 1 900 275 / 229 / 220, 16 of 1 500 to 2 500
-//     427 / 346 / 347, 8 of 2 048 232 / 185 / 190.
+//   packed sequences of 16 heads, whose last tiles come as they come: causal 24 of 500 to 1 500 182 / 142 / 128, 8 of 2 048
+//     153 / 122 / 119, of head_dim 32 7 of 80 to 180 10.5 / - / 7.2, but 2 of 1 100 16.6 / - / 18.7; no mask 24 of 500 to
+//     1 500 244 / 191 / 183, 42 of 1 114 to 1 414 - / 467 / 450, 16 of 1 500 to 2 500 427 / 346 / 347, but 4 of 1 401 to
+//     1 696 - / 64.1 / 67.8, 8 of 2 048 232 / 185 / 190.
 // At head_dim 128, the same shape with single K and V buffers measured 89 against 93 us on 16 x 16 x 577 but 665 against
 // 578 on 4 x 32 x 4 096 causal and 116 against 112 on 2 x 32 x 1 500 (64 KB of K and V per tile and CTA); it is not built.
 constexpr int kHalfSmMaxKeys = 2048;        // a row sees on average; beyond, within 3 % of two tiles or slower
-constexpr int kHalfSmMaxPackedKeys = 1792;  // without a mask
+constexpr int kHalfSmMaxPackedKeys = 1024;  // without a mask
+constexpr int kHalfSmManyWavesKeys = 1700;  // the same from eight waves on
 constexpr int kOneTileRows = 1920;          // from here on one-tile CTAs, up to two half-SM CTAs per SM
+constexpr int kOneTilePackedKeys = 320;     // the same for packed sequences, of whose blocks the count is an upper bound
 constexpr int kHalfSmKeysPerWave = 384;     // fewer for each wave after the first: a nearly full last wave does not matter
 
 // rows: of every sequence, or 0 for packed sequences of their own lengths; blocks: of 256 and of 128 rows per unit;
@@ -208,10 +211,10 @@ bool half_sm_pays(int rows, int64_t blocks_of_256, int64_t blocks_of_128, int64_
   if (rows > 0 && rows <= 128) return true;
   if (ctas <= sms) return false;
   if (ctas <= 2 * sms && (masked || rows == 0)) {
-    const bool long_rows = (rows > 0 ? rows : 2 * mean_keys) >= kOneTileRows;
+    const bool long_rows = rows > 0 ? rows >= kOneTileRows : mean_keys >= kOneTilePackedKeys;
     return masked ? !one_tile || (ctas2 > sms && !long_rows) : ctas2 > sms;
   }
-  if (rows == 0) return masked || mean_keys <= kHalfSmMaxPackedKeys;
+  if (rows == 0) return masked || mean_keys <= (ctas > 16 * sms ? kHalfSmManyWavesKeys : kHalfSmMaxPackedKeys);
   if (masked) {
     const bool long_rows = blocks_of_128 >= (blocks_of_128 % 2 == 0 ? 14 : 19);
     return !long_rows || ctas <= 3 * sms || ctas2 > 2 * sms;

@@ -56,7 +56,9 @@ def test_rows_of_one_length(choose, units, rows, mask, best):
 
 
 @pytest.mark.parametrize("lengths,heads,mask,best", [
-    ([992] * 24, 16, NONE, HALF), ([1694] * 12, 16, NONE, HALF), ([2048] * 8, 16, NONE, TWO), ([3500] * 6, 16, NONE, TWO),
+    ([992] * 24, 16, NONE, HALF), ([1694] * 12, 16, NONE, HALF), ([1267] * 42, 16, NONE, HALF), ([1485] * 7, 16, NONE, TWO),
+    ([1743] * 9, 8, NONE, TWO), ([1174] * 6, 8, NONE, TWO), ([1527] * 4, 16, NONE, TWO), ([1083] * 2, 16, CAUSAL, ONE),
+    ([302] * 5, 16, CAUSAL, HALF), ([2048] * 8, 16, NONE, TWO), ([3500] * 6, 16, NONE, TWO),
     ([992] * 24, 16, CAUSAL, HALF), ([2048] * 8, 16, CAUSAL, HALF), ([81] * 10, 16, CAUSAL, HALF),
 ])
 def test_packed(choose, lengths, heads, mask, best):
